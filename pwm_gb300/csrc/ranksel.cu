@@ -18,12 +18,8 @@ namespace pwmgpu {
 
 namespace {
 
-constexpr uint64_t kL1Bits = 2048, kL2Bits = 512, kL1Cover = 32, kL2Cover = 8, kSampleRate = 8192;
+constexpr uint64_t kL1Bits = 2048, kL1Cover = 32, kL2Cover = 8, kSampleRate = 8192;
 constexpr int kRsThreads = 256;
-
-__device__ __forceinline__ uint32_t l2_of(const uint32_t* l12, uint64_t e, uint32_t i) {
-  return (l12[2 * e + 1] >> (10 * i)) & 1023u;
-}
 
 // Phase 1: per L1 block popcounts, l2 fields, and the exclusive prefix of
 // block totals inside each CTA (256 blocks per CTA).  Warp w reads its 32
@@ -248,200 +244,231 @@ __global__ void __launch_bounds__(kRsThreads) rs_finish_kernel(const RankSelectL
 
 // ---------------------------------------------------------------------------
 // Queries (include/queries/query_support.hpp:39-178)
+//
+// A query walks one level after another, each step a few loads whose
+// addresses come from the step before: latency bounds a small batch, scattered
+// sectors a large one.  So a step asks for all it may need at once: a rank
+// loads its block entry and the 512-bit L2 block (64 bytes, 64-byte aligned:
+// levels start at multiples of 128) in one round trip, two 32-byte loads for
+// the words, instead of walking up to 8 words one after the other; a select
+// loads 8 block entries where the occurrence should lie and then one L2 block.
+// A thread a query: pairs and quads of lanes sharing a query's words measured
+// slower (5.0 and 7.2 against 4.2 ms for the large batch below), their
+// exchanges costing more than the counting they save.  The level descriptors
+// come from shared memory.  Measured (GB300): 3 x 10^4 queries on a tree of
+// 10^6 bytes, 8 levels, 139 -> 52 us; 3 x 2^22 on the 2^28 16-bit matrix (16
+// levels) 8.34 -> 4.23 ms (access 1.18, rank 1.32, select 1.73), bound by L1's
+// scattered requests (80 % busy; DRAM 45 % of its peak).  128 threads a block
+// spread a small batch over more SMs than 256 (50.7 against 54.5 us); 48
+// registers a thread (10 blocks an SM) answered the large batch faster than 40
+// (4.23 against 4.48 ms).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t q_rank1(const QueryLevel& L, uint64_t index) {
-  // bin_rank_popcnt::rank1 (bin_rank_popcnt.hpp:98-128); the index of pwm's
-  // extra zeroed L1 entry answers with the level's total instead of 0.
-  const uint64_t nreal = (L.nwords + kL1Cover - 1) / kL1Cover;
-  if (index > L.nwords * 64) index = L.nwords * 64;  // past the level: the padding holds no ones
-  const uint64_t l1 = index / kL1Bits;
-  if (l1 >= nreal) return L.meta[2];
-  uint64_t rem = index - l1 * kL1Bits;
-  uint64_t result = L.l12[2 * l1];
-  const uint64_t l2 = rem / kL2Bits;
-  rem -= l2 * kL2Bits;
-  for (uint32_t i = 0; i < l2; ++i) result += l2_of(L.l12, l1, i);
-  uint64_t off = l1 * kL1Cover + l2 * kL2Cover;
-  while (rem >= 64) { result += __popcll(L.data[off++]); rem -= 64; }
-  if (rem > 0) result += __popcll(L.data[off] >> (64 - rem));
-  return result;
-}
-__device__ __forceinline__ uint64_t q_rank0(const QueryLevel& L, uint64_t index) { return index - q_rank1(L, index); }
+constexpr int kQueryThreads = 128;
+constexpr uint32_t kQueryMaxLevels = 64;
 
-// bin_select_popcnt::select (bin_select_popcnt.hpp:112-117, 166-241), with
-// the scan start at sample (occ-1)/8192 and the block scan and word walk
-// bounded by the real data (pwm reads past its arrays there).
-__device__ uint64_t q_select(const QueryLevel& L, int value, uint64_t occ) {
-  if (occ == 0) return 0;
-  const uint64_t nreal = (L.nwords + kL1Cover - 1) / kL1Cover;
-  const uint64_t ns = L.meta[value ? 1 : 0];
+// A level as the queries read it, in shared memory.
+struct FastLevel {
+  const uint64_t* data;
+  const uint32_t* l12;
+  const uint32_t* s0;
+  const uint32_t* s1;
+  uint32_t nwords;  // rank/select levels hold fewer than 2^32 - 64 bits
+  uint32_t nreal;   // L1 blocks
+  uint32_t total;   // ones
+  uint32_t ns0, ns1;
+  uint32_t zeros;   // matrix
+  uint32_t bits;    // Huffman-shaped
+};
+
+// Four words, or four block entries (ones before the block in the low half,
+// its L2 fields in the high one), by one 32-byte load.  The words go round L1
+// and pull in no more than their 64 bytes of L2 (by default a miss fetched up
+// to 128: 2^22 accesses 1.13 -> 1.00 ms, ranks 2.10 -> 1.25 ms).
+struct Four {
+  uint64_t w[4];
+};
+__device__ __forceinline__ Four load_words(const uint64_t* p) {
+  Four v;
+  asm("ld.global.nc.L1::evict_first.L2::64B.v4.u64 {%0, %1, %2, %3}, [%4];"
+      : "=l"(v.w[0]), "=l"(v.w[1]), "=l"(v.w[2]), "=l"(v.w[3])
+      : "l"(p));
+  return v;
+}
+__device__ __forceinline__ Four load_entries(const uint32_t* p) {
+  Four v;
+  asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(v.w[0]), "=l"(v.w[1]), "=l"(v.w[2]), "=l"(v.w[3]) : "l"(p));
+  return v;
+}
+
+// ~0 << s with s >= 64 giving 0 (PTX clamps the shift amount).
+__device__ __forceinline__ uint64_t high_mask(uint32_t s) {
+  uint64_t r;
+  asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(~0ull), "r"(s));
+  return r;
+}
+
+// Ones of a level before `at` (bin_rank_popcnt::rank1, bin_rank_popcnt.hpp:
+// 98-128).  The index of pwm's extra zeroed L1 entry answers with the level's
+// total instead of 0, an index past the level with the whole level (the
+// padding holds no ones), so that no index reads outside it.  BIT: also bit
+// `at`.
+struct Rank {
+  uint32_t ones, bit;
+};
+template <bool BIT, typename I>
+__device__ __forceinline__ Rank rank_at(const FastLevel& L, I at) {
+  const uint32_t most = L.nwords * 64u - (BIT ? 1u : 0u);
+  const uint32_t index = at > most ? most : uint32_t(at);
+  const uint32_t l1 = index >> 11, l2 = (index >> 9) & 3u;
+  if (l1 >= L.nreal) return Rank{L.total, 0u};
+  const uint2 e = __ldg(reinterpret_cast<const uint2*>(L.l12) + l1);
+  const int nb = int(index & 511u);
+  const uint64_t* block = L.data + size_t(index >> 9) * 8;
+  Rank r{0u, 0u};
+  Four a = {}, b = {};
+  if (BIT || nb > 0) a = load_words(block);
+  if (BIT ? nb >= 256 : nb > 256) b = load_words(block + 4);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    r.ones += __popcll(a.w[k] & high_mask(uint32_t(max(64 * k + 64 - nb, 0))));
+    r.ones += __popcll(b.w[k] & high_mask(uint32_t(max(64 * k + 320 - nb, 0))));
+  }
+  if (BIT) {
+    const int k = nb & 255;
+    const Four& h = nb < 256 ? a : b;
+    const uint64_t w = k < 128 ? (k < 64 ? h.w[0] : h.w[1]) : (k < 192 ? h.w[2] : h.w[3]);
+    r.bit = uint32_t(w >> (63 - (nb & 63))) & 1u;
+  }
+  // whole L2 blocks before it (at most 3)
+  r.ones += e.x + (l2 > 0 ? e.y & 1023u : 0u) + (l2 > 1 ? (e.y >> 10) & 1023u : 0u) + (l2 > 2 ? (e.y >> 20) & 1023u : 0u);
+  return r;
+}
+template <typename I>
+__device__ __forceinline__ uint32_t ones_before(const FastLevel& L, I at) {
+  return rank_at<false>(L, at).ones;
+}
+
+// bin_select_popcnt::select (bin_select_popcnt.hpp:112-117, 166-241), occ > 0:
+// the sample of (occ - 1) / 8192 itself when occ is the one it was taken at,
+// else the first L1 block from the sample's on whose successor's count
+// reaches occ, then its L2 block and word.  The occ-th bit lies at or before
+// the next sample; the block is looked for first where occ's share of the
+// 8192 puts it (a window of 8 entries: found there for all but a few in a
+// thousand selects of the 16-bit matrix, whose gaps between samples reach 300
+// blocks), then between the bounds that leaves, four probes a step.  False
+// past the count.  (pwm walks on past its arrays there.)
+__device__ __forceinline__ bool select_bit(const FastLevel& L, bool value, uint32_t occ, uint32_t* pos) {
+  if (L.nwords == 0) return false;
+  const uint32_t ns = value ? L.ns1 : L.ns0;
   const uint32_t* samples = value ? L.s1 : L.s0;
-  const uint64_t sidx = (occ - 1) / kSampleRate;
-  uint64_t l1;
-  if (sidx < ns) {
-    l1 = samples[sidx];
-    if ((occ - 1) % kSampleRate == 0) return l1;
-    l1 /= kL1Bits;
-  } else {
-    l1 = ns ? samples[ns - 1] / kL1Bits : 0;
+  const uint32_t sidx = (occ - 1) / uint32_t(kSampleRate), share = (occ - 1) % uint32_t(kSampleRate);
+  uint32_t lo = 0, hi = L.nreal - 1, guess = 0;
+  if (ns) {
+    const uint32_t s = __ldg(samples + min(sidx, ns - 1));
+    uint32_t nx = 0;
+    if (sidx + 1 < ns) nx = __ldg(samples + sidx + 1);
+    if (sidx < ns && share == 0) {
+      *pos = s;
+      return true;
+    }
+    guess = lo = min(s >> 11, hi);
+    if (sidx + 1 < ns) {
+      hi = max(lo, min(hi, nx >> 11));
+      guess = lo + uint32_t((uint64_t(hi - lo) * share) >> 13);
+    }
   }
-  if (value == 0) {
-    while (l1 + 1 < nreal && (((l1 + 1) * kL1Bits) - L.l12[2 * (l1 + 1)]) < occ) ++l1;
-    occ -= (l1 * kL1Bits) - L.l12[2 * l1];
-  } else {
-    while (l1 + 1 < nreal && L.l12[2 * (l1 + 1)] < occ) ++l1;
-    occ -= L.l12[2 * l1];
-  }
-  uint32_t l2 = 0;
-  if (value == 0) {
-    while (l2 < 3 && occ > kL2Bits - l2_of(L.l12, l1, l2)) occ -= kL2Bits - l2_of(L.l12, l1, l2++);
-  } else {
-    while (l2 < 3 && occ > l2_of(L.l12, l1, l2)) occ -= l2_of(L.l12, l1, l2++);
-  }
-  const uint64_t last = kL2Cover * l2 + kL1Cover * l1;
-  uint64_t extra = 0;
+  // ones (or zeros) before block e, from its entry's ones
+  auto before = [&](uint32_t e, uint32_t ones) { return value ? ones : e * uint32_t(kL1Bits) - ones; };
+  // the last of blocks lo..hi with fewer than occ before it; lo is one
+  uint32_t base = guess > lo + 2 ? (guess - 2) & ~3u : lo & ~3u;
+  uint32_t l1;
+  uint64_t entry = 0;
   for (;;) {
-    if (last + extra >= L.nwords) return ~0ull;
-    uint64_t w = L.data[last + extra];
-    if (value == 0) w = ~w;
-    const uint64_t pc = __popcll(w);
-    if (pc >= occ) return kL2Bits * l2 + kL1Bits * l1 + extra * 64 + word_select1(w, uint32_t(occ));
-    ++extra;
-    occ -= pc;
-  }
-}
-
-__device__ __forceinline__ bool bit_at(const uint64_t* d, uint64_t i) { return (d[i >> 6] >> (63 - (i & 63))) & 1; }
-
-// ops: the kind of each query (a mixed batch), or null for `op` throughout.
-__global__ void query_kernel(QueryStructure q, int op0, const uint8_t* __restrict__ ops,
-                             const uint64_t* __restrict__ a, const uint64_t* __restrict__ b, uint64_t count,
-                             uint64_t* __restrict__ out) {
-  const uint32_t Lv = q.levels;
-  for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < count; t += uint64_t(gridDim.x) * blockDim.x) {
-    const int op = ops ? int(ops[t]) : op0;
-    uint64_t result = 0;
-    if (op == 0 && a[t] >= q.n) {  // access past the text
-      result = ~0ull;
-    } else if (op == 0) {  // access
-      uint64_t index = a[t], word = 0;
-      if (q.is_tree) {
-        uint64_t start = 0, end = q.n;
-        for (uint32_t level = 0; level < Lv; ++level) {
-          const QueryLevel& L = q.lv[level];
-          const uint64_t left = q_rank0(L, start), right = q_rank0(L, end);
-          word <<= 1;
-          if (bit_at(L.data, start + index)) {
-            word |= 1;
-            index = q_rank1(L, start + index) - (start - left);
-            start = start + right - left;
-          } else {
-            index = q_rank0(L, start + index) - left;
-            end = start + right - left;
-          }
-        }
-      } else {
-        for (uint32_t level = 0; level < Lv; ++level) {
-          const QueryLevel& L = q.lv[level];
-          word <<= 1;
-          if (bit_at(L.data, index)) {
-            word |= 1;
-            index = q_rank1(L, index) + q.zeros[level];
-          } else {
-            index = q_rank0(L, index);
-          }
-        }
-      }
-      result = word;
-    } else if (op == 1) {  // rank(symbol, index)
-      const uint64_t sym = a[t];
-      uint64_t index = b[t];
-      if (index != 0) {
-        if (q.is_tree) {
-          uint64_t start = 0, end = q.n;
-          for (uint32_t level = 0; level < Lv; ++level) {
-            const QueryLevel& L = q.lv[level];
-            const uint64_t left = q_rank0(L, start), right = q_rank0(L, end);
-            if ((sym >> (Lv - level - 1)) & 1) {
-              index = q_rank1(L, start + index) - (start - left);
-              start = start + right - left;
-            } else {
-              index = q_rank0(L, start + index) - left;
-              end = start + right - left;
-            }
-          }
-          result = index;
-        } else {
-          uint64_t offset = 0;
-          for (uint32_t level = 0; level < Lv; ++level) {
-            const QueryLevel& L = q.lv[level];
-            if ((sym >> (Lv - level - 1)) & 1) {
-              index = q.zeros[level] + q_rank1(L, index);
-              offset = q.zeros[level] + q_rank1(L, offset);
-            } else {
-              index = q_rank0(L, index);
-              offset = q_rank0(L, offset);
-            }
-          }
-          result = index - offset;
-        }
-      }
-    } else {  // select(symbol, occ)
-      const uint64_t sym = a[t];
-      uint64_t occ = b[t];
-      if (occ != 0) {
-        uint64_t st[64], le[64];
-        if (q.is_tree) {
-          uint64_t start = 0, end = q.n;
-          for (uint32_t level = 0; level < Lv; ++level) {
-            const QueryLevel& L = q.lv[level];
-            const uint64_t left = q_rank0(L, start), right = q_rank0(L, end);
-            st[level] = start;
-            le[level] = left;
-            if ((sym >> (Lv - level - 1)) & 1) start = start + right - left;
-            else end = start + right - left;
-          }
-          for (int level = int(Lv) - 1; level >= 0; --level) {
-            const QueryLevel& L = q.lv[level];
-            const uint64_t adj = level == 0 ? 0 : 1;
-            if ((sym >> (Lv - level - 1)) & 1) occ = q_select(L, 1, st[level] - le[level] + occ) - st[level] + adj;
-            else occ = q_select(L, 0, le[level] + occ) - st[level] + adj;
-          }
-        } else {
-          uint64_t offset = 0;
-          for (uint32_t level = 0; level < Lv; ++level) {
-            const QueryLevel& L = q.lv[level];
-            if ((sym >> (Lv - level - 1)) & 1) offset = q.zeros[level] + q_rank1(L, offset);
-            else offset = q_rank0(L, offset);
-          }
-          occ += offset;
-          for (int level = int(Lv) - 1; level >= 0; --level) {
-            const QueryLevel& L = q.lv[level];
-            const uint64_t adj = level == 0 ? 0 : 1;
-            if ((sym >> (Lv - level - 1)) & 1) occ = q_select(L, 1, occ - q.zeros[level]) + adj;
-            else occ = q_select(L, 0, occ) + adj;
-          }
-        }
-        result = occ;
+    const Four u = load_entries(L.l12 + 2 * size_t(base));
+    Four v = {};
+    if (base + 4 <= hi) v = load_entries(L.l12 + 2 * size_t(base + 4));
+    // the entries ascend: the last one below occ is the answer, if the window holds it
+    uint32_t n = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+      const uint64_t e = k < 4 ? u.w[k & 3] : v.w[k & 3];
+      if (base + k <= lo || (base + k <= hi && before(base + k, uint32_t(e)) < occ)) {
+        n = k + 1;
+        entry = e;
       }
     }
-    out[t] = result;
+    if (n == 0) {
+      hi = base - 1;
+    } else if (n == 8 && base + 7 < hi) {
+      lo = base + 7;
+    } else {
+      l1 = base + n - 1;
+      break;
+    }
+    while (hi - lo > 4) {
+      const uint64_t span = hi - lo;
+      uint32_t e[4], x[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) e[k] = lo + uint32_t(span * uint32_t(k + 1) / 5);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] = __ldg(L.l12 + 2 * size_t(e[k]));
+#pragma unroll
+      for (int k = 3; k >= 0; --k)
+        if (before(e[k], x[k]) >= occ) hi = max(e[k] - 1, lo);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (e[k] <= hi) lo = e[k];
+    }
+    base = lo & ~3u;
   }
+  occ -= before(l1, uint32_t(entry));
+  // the L2 block: whole blocks skipped by their counts, the fourth has none
+  uint32_t f = uint32_t(entry >> 32);
+  f = value ? f : (512u | 512u << 10 | 512u << 20) - (f & 0x3FFFFFFFu);  // no borrows: a field is at most 512
+  const uint32_t c0 = f & 1023u, c1 = c0 + ((f >> 10) & 1023u), c2 = c1 + ((f >> 20) & 1023u);
+  const uint32_t l2 = (occ > c0 ? 1u : 0u) + (occ > c1 ? 1u : 0u) + (occ > c2 ? 1u : 0u);
+  occ -= occ > c2 ? c2 : occ > c1 ? c1 : occ > c0 ? c0 : 0u;
+  uint32_t word = l1 * 32 + l2 * 8;
+  if (word >= L.nwords) return false;
+  // the word (those past the level, inside its padding, hold no ones; a zero
+  // found there lies past the count)
+  const Four a = load_words(L.data + word), b = load_words(L.data + word + 4);
+  const uint32_t pa0 = value ? __popcll(a.w[0]) : 64u - __popcll(a.w[0]);
+  uint64_t x = a.w[0];
+  uint32_t k = occ, run = pa0;
+#pragma unroll
+  for (int i = 1; i < 8; ++i) {
+    const uint64_t w = i < 4 ? a.w[i & 3] : b.w[i & 3];
+    if (occ > run) {
+      x = w;
+      k = occ - run;
+      word = l1 * 32 + l2 * 8 + i;
+    }
+    run += value ? __popcll(w) : 64u - __popcll(w);
+  }
+  if (occ > run || word >= L.nwords) return false;
+  // the k-th bit of the word, halved from 32 down
+  if (!value) x = ~x;
+  uint32_t at = 64 * word;
+  uint32_t c = uint32_t(x >> 32), n = __popc(c);
+  if (k > n) {
+    k -= n;
+    at += 32;
+    c = uint32_t(x);
+  }
+#pragma unroll
+  for (int h = 16; h; h >>= 1) {
+    n = __popc(c >> (32 - h));
+    if (k > n) {
+      k -= n;
+      c <<= h;
+      at += h;
+    }
+  }
+  *pos = at;
+  return true;
 }
 
-// ---------------------------------------------------------------------------
-// Queries on Huffman-shaped structures (pwm's query_support has none: it
-// prints "NOT YET IMPLEMENTED", include/queries/query_support.hpp:43,55,67).
-//
-// Level l holds bit l of every code longer than l.  In both shapes the codes
-// that end at a level sort behind all codes that go on: the matrix's codes
-// (huff_codes.hpp:204-245) take, length by length, the largest bit-reversed
-// words, and the tree's are negated canonical codes (:246-283), the largest
-// prefixes.  So level l + 1 is a prefix of level l's entries reordered as the
-// plain structures reorder them (the matrix by its stable 0/1 partition, the
-// tree within each node), and the plain position arithmetic holds; a code
-// ends where its position falls past the next level's size.
-// ---------------------------------------------------------------------------
 __device__ uint64_t huff_decode(const HuffQueryTables& h, uint32_t len, uint64_t word) {
   const uint64_t key = (uint64_t(len) << 56) | word;
   uint64_t lo = 0, hi = h.ndec;
@@ -452,150 +479,235 @@ __device__ uint64_t huff_decode(const HuffQueryTables& h, uint32_t len, uint64_t
   return lo < h.ndec && h.dec_key[lo] == key ? h.dec_sym[lo] : ~0ull;
 }
 
-__global__ void huff_query_kernel(QueryStructure q, HuffQueryTables h, int op, const uint64_t* __restrict__ a,
-                                  const uint64_t* __restrict__ b, uint64_t count, uint64_t* __restrict__ out) {
-  const uint32_t Lv = q.levels;
-  for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < count; t += uint64_t(gridDim.x) * blockDim.x) {
-    uint64_t result = ~0ull;
-    if (op == 0) {  // access: read bits until the code ends
-      if (a[t] < q.n) {
-        uint64_t index = a[t], word = 0;
-        if (q.is_tree) {
-          uint64_t start = 0, end = q.n;
-          for (uint32_t level = 0; level < Lv; ++level) {
-            const QueryLevel& L = q.lv[level];
-            const uint64_t left = q_rank0(L, start), right = q_rank0(L, end);
-            const bool one = bit_at(L.data, start + index);
-            word = (word << 1) | (one ? 1u : 0u);
-            if (one) {
-              index = q_rank1(L, start + index) - (start - left);
-              start = start + right - left;
-            } else {
-              index = q_rank0(L, start + index) - left;
-              end = start + right - left;
-            }
-            if (level + 1 == Lv || start + index >= h.level_bits[level + 1]) {
-              result = huff_decode(h, level + 1, word);
-              break;
-            }
-          }
-        } else {
-          for (uint32_t level = 0; level < Lv; ++level) {
-            const QueryLevel& L = q.lv[level];
-            const bool one = bit_at(L.data, index);
-            word = (word << 1) | (one ? 1u : 0u);
-            index = one ? q.zeros[level] + q_rank1(L, index) : q_rank0(L, index);
-            if (level + 1 == Lv || index >= h.level_bits[level + 1]) {
-              result = huff_decode(h, level + 1, word);
-              break;
-            }
-          }
-        }
-      }
-      out[t] = result;
-      continue;
-    }
-    // rank(symbol, index) / select(symbol, occurrence): walk the symbol's code
-    const uint64_t sym = a[t];
-    const uint32_t len = sym < h.nsym ? uint32_t(h.code_len[sym]) : 0u;
-    const uint64_t code = len ? h.code_word[sym] : 0;
-    if (len == 0 || len > Lv) {  // a symbol without a code does not occur
-      out[t] = (op == 1 || b[t] == 0) ? 0 : ~0ull;
-      continue;
-    }
-    auto bit = [&](uint32_t level) { return (code >> (len - 1 - level)) & 1; };
-    if (op == 1) {
-      uint64_t index = b[t] < q.n ? b[t] : q.n;
-      if (q.is_tree) {
-        uint64_t start = 0, end = q.n;
-        for (uint32_t level = 0; level < len && index; ++level) {
-          const QueryLevel& L = q.lv[level];
-          const uint64_t left = q_rank0(L, start), right = q_rank0(L, end);
-          if (bit(level)) {
-            index = q_rank1(L, start + index) - (start - left);
-            start = start + right - left;
-          } else {
-            index = q_rank0(L, start + index) - left;
-            end = start + right - left;
-          }
-        }
-        result = index;
-      } else {
-        uint64_t offset = 0;
-        for (uint32_t level = 0; level < len; ++level) {
-          const QueryLevel& L = q.lv[level];
-          if (bit(level)) {
-            index = q.zeros[level] + q_rank1(L, index);
-            offset = q.zeros[level] + q_rank1(L, offset);
-          } else {
-            index = q_rank0(L, index);
-            offset = q_rank0(L, offset);
-          }
-        }
-        result = index - offset;
-      }
+// access(index): the symbol at a position below n.
+template <bool TREE, bool HUFF>
+__device__ __forceinline__ uint64_t query_access(const QueryStructure& S, const HuffQueryTables& h, const FastLevel* lv,
+                                                 uint32_t index) {
+  const uint32_t Lv = S.levels;
+  uint64_t word = 0;
+  uint32_t start = 0, end = uint32_t(S.n);
+  for (uint32_t level = 0; level < Lv; ++level) {
+    const FastLevel& L = lv[level];
+    const Rank at = rank_at<true>(L, start + index);
+    const bool one = at.bit != 0;
+    word = (word << 1) | at.bit;
+    if constexpr (TREE) {
+      const uint32_t ra = ones_before(L, start), rb = ones_before(L, end);
+      const uint32_t mid = end - rb + ra;  // where the node's zeros end: start + zeros inside it
+      index = one ? at.ones - ra : start + index - at.ones - (start - ra);
+      if (one) start = mid;
+      else end = mid;
     } else {
-      uint64_t occ = b[t];
-      if (occ == 0) {
-        result = 0;  // as the plain structures' select
+      index = one ? L.zeros + at.ones : index - at.ones;
+    }
+    if (HUFF && (level + 1 == Lv || start + index >= lv[level + 1].bits)) return huff_decode(h, level + 1, word);
+  }
+  return word;
+}
+
+// rank(symbol, index): `len` bits of `code`, most significant first.  I =
+// uint32_t: index at most n; uint64_t: any index.
+template <bool TREE, bool HUFF, typename I>
+__device__ __forceinline__ uint64_t query_rank(const QueryStructure& S, const FastLevel* lv, uint64_t code, uint32_t len,
+                                               I index) {
+  I start = 0, end = I(S.n);  // the symbol's node; a matrix uses start alone, its block's first position
+  for (uint32_t level = 0; level < len; ++level) {
+    const FastLevel& L = lv[level];
+    const bool one = (code >> (len - 1 - level)) & 1;
+    if constexpr (TREE) {
+      if (HUFF && index == 0) break;
+      const I at = ones_before(L, I(start + index)), ra = ones_before(L, start), rb = ones_before(L, end);
+      const I mid = end - rb + ra;
+      index = one ? at - ra : start + index - at - (start - ra);
+      if (one) start = mid;
+      else end = mid;
+    } else {
+      const I ra = ones_before(L, start), rb = ones_before(L, index);
+      start = one ? L.zeros + ra : start - ra;
+      index = one ? L.zeros + rb : index - rb;
+    }
+  }
+  return TREE ? index : I(index - start);
+}
+
+// select(symbol, occ), occ > 0; node: words [2 * level] and [2 * level + 1] of
+// this query in shared memory, blockDim.x apart (a tree's node starts and
+// zero counts on the way down).  I = uint32_t: occ at most n; `bad` is set,
+// with no answer, where a step leaves the level (an occurrence past the
+// symbol's last).  uint64_t: any occ, such steps carried through as 64-bit
+// numbers.
+template <bool TREE, bool HUFF, typename I>
+__device__ __forceinline__ uint64_t query_select(const QueryStructure& S, const FastLevel* lv, uint32_t* node,
+                                                 uint64_t code, uint32_t len, I occ, bool* bad) {
+  constexpr bool WIDE = sizeof(I) == 8;
+  const uint32_t n = uint32_t(S.n);
+  uint32_t start = 0, end = n;
+  for (uint32_t level = 0; level < len; ++level) {
+    const FastLevel& L = lv[level];
+    const bool one = (code >> (len - 1 - level)) & 1;
+    const uint32_t ra = ones_before(L, start);
+    if constexpr (TREE) {
+      const uint32_t rb = ones_before(L, end);
+      node[(2 * level) * blockDim.x] = start;
+      node[(2 * level + 1) * blockDim.x] = start - ra;
+      const uint32_t mid = end - rb + ra;
+      if (one) start = mid;
+      else end = mid;
+    } else {
+      if constexpr (HUFF) {
+        const uint32_t rb = ones_before(L, end);
+        end = one ? L.zeros + rb : end - rb;
+      }
+      start = one ? L.zeros + ra : start - ra;
+    }
+  }
+  if (HUFF && occ > I(end - start)) return ~0ull;  // the symbol's node holds its occurrences
+  if constexpr (!TREE) {
+    if (!WIDE && occ > n - start) {
+      *bad = true;
+      return 0;
+    }
+    occ += start;
+  }
+  for (int level = int(len) - 1; level >= 0; --level) {
+    const FastLevel& L = lv[level];
+    const uint32_t adj = level == 0 ? 0 : 1;
+    const bool one = (code >> (len - 1 - uint32_t(level))) & 1;
+    uint32_t off = one ? L.zeros : 0u, st = 0;  // the (occ - off)-th such bit of the level; its position less st
+    if constexpr (TREE) {
+      st = node[(2 * level) * blockDim.x];
+      const uint32_t left = node[(2 * level + 1) * blockDim.x];
+      off = 0u - (one ? st - left : left);
+    }
+    uint32_t pos = 0;
+    if constexpr (WIDE) {
+      const uint64_t o = TREE ? occ + uint32_t(0u - off) : occ - off;
+      uint64_t at = 0;
+      if (o != 0) at = (o >> 32) == 0 && select_bit(L, one, uint32_t(o), &pos) ? uint64_t(pos) : ~0ull;
+      occ = at - st + adj;
+    } else {
+      // a matrix's one lies past the zeros, a tree's bit inside the level
+      const uint32_t o = occ - off;
+      if ((TREE ? (occ > n || o > n) : (one && occ <= off)) || !select_bit(L, one, o, &pos) || (TREE && pos < st)) {
+        *bad = true;
+        return 0;
+      }
+      occ = pos - st + adj;
+    }
+  }
+  return occ;
+}
+
+// Operands past the text or the last occurrence: the 64-bit forms, out of the
+// way of the ordinary ones.
+template <bool TREE, bool HUFF>
+__device__ __noinline__ uint64_t query_outside(const QueryStructure& S, const FastLevel* lv, uint32_t* node, int op,
+                                               uint64_t code, uint32_t len, uint64_t arg) {
+  bool bad = false;
+  return op == 1 ? query_rank<TREE, HUFF, uint64_t>(S, lv, code, len, arg)
+                 : query_select<TREE, HUFF, uint64_t>(S, lv, node, code, len, arg, &bad);
+}
+
+// A batch of queries, a thread each.  OP: 0 access, 1 rank, 2 select; -1: a
+// mixed batch, ops[t] the kind of query t, and blockIdx.y the kind this block
+// answers (a warp whose lanes hold different kinds runs them one after the
+// other; a block a kind runs them side by side).
+//
+// Huffman-shaped structures (pwm's query_support has none: it prints "NOT YET
+// IMPLEMENTED", include/queries/query_support.hpp:43,55,67): level l holds
+// bit l of every code longer than l.  In both shapes the codes that end at a
+// level sort behind all codes that go on: the matrix's codes (huff_codes.hpp:
+// 204-245) take, length by length, the largest bit-reversed words, and the
+// tree's are negated canonical codes (:246-283), the largest prefixes.  So
+// level l + 1 is a prefix of level l's entries reordered as the plain
+// structures reorder them (the matrix by its stable 0/1 partition, the tree
+// within each node), and the plain position arithmetic holds; a code ends
+// where its position falls past the next level's size.
+template <int OP, bool TREE, bool HUFF>
+__global__ void __launch_bounds__(kQueryThreads, 10) query_kernel(QueryStructure S, HuffQueryTables h,
+                                                                 const uint8_t* __restrict__ ops,
+                                                                 const uint64_t* __restrict__ a,
+                                                                 const uint64_t* __restrict__ b, uint64_t count,
+                                                                 uint64_t* __restrict__ out) {
+  __shared__ FastLevel lv[kQueryMaxLevels];
+  extern __shared__ uint32_t nodes[];  // a tree's selects: [2 * levels][threads]
+  for (uint32_t l = threadIdx.x; l < S.levels; l += blockDim.x) {
+    const QueryLevel L = S.lv[l];
+    const uint64_t cap = L.nwords * 64 / kSampleRate + 2;  // entries of a sample array
+    lv[l] = FastLevel{L.data, L.l12, L.s0, L.s1, uint32_t(L.nwords), uint32_t((L.nwords + kL1Cover - 1) / kL1Cover),
+                      uint32_t(L.meta[2]), uint32_t(min(uint64_t(L.meta[0]), cap)),
+                      uint32_t(min(uint64_t(L.meta[1]), cap)), TREE ? 0u : uint32_t(S.zeros[l]),
+                      HUFF ? uint32_t(h.level_bits[l]) : 0u};
+  }
+  __syncthreads();
+  const int op = OP >= 0 ? OP : int(blockIdx.y);
+  uint32_t* node = nodes + threadIdx.x;
+  for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < count; t += uint64_t(gridDim.x) * blockDim.x) {
+    if (OP < 0 && int(ops[t]) != op) continue;
+    uint64_t code = a[t], result = ~0ull;
+    if (op == 0) {
+      if (code < S.n) result = query_access<TREE, HUFF>(S, h, lv, uint32_t(code));
+    } else {
+      uint64_t arg = b[t];
+      uint32_t len = S.levels;
+      bool coded = true;
+      if constexpr (HUFF) {
+        len = code < h.nsym ? uint32_t(h.code_len[code]) : 0u;
+        code = len ? h.code_word[code] : 0;
+        coded = len != 0 && len <= S.levels;
+        if (op == 1) arg = arg < S.n ? arg : S.n;
+      }
+      if (!coded) {
+        result = (op == 1 || arg == 0) ? 0 : ~0ull;  // a symbol without a code does not occur
+      } else if (arg == 0) {
+        result = 0;
       } else {
-        if (q.is_tree) {
-          uint64_t st[64], le[64];
-          uint64_t start = 0, end = q.n;
-          for (uint32_t level = 0; level < len; ++level) {
-            const QueryLevel& L = q.lv[level];
-            const uint64_t left = q_rank0(L, start), right = q_rank0(L, end);
-            st[level] = start;
-            le[level] = left;
-            if (bit(level)) start = start + right - left;
-            else end = start + right - left;
-          }
-          if (occ <= end - start) {  // the symbol's node holds its occurrences
-            for (int level = int(len) - 1; level >= 0; --level) {
-              const QueryLevel& L = q.lv[level];
-              const uint64_t adj = level == 0 ? 0 : 1;
-              if (bit(uint32_t(level))) occ = q_select(L, 1, st[level] - le[level] + occ) - st[level] + adj;
-              else occ = q_select(L, 0, le[level] + occ) - st[level] + adj;
-            }
-            result = occ;
-          }
-        } else {
-          uint64_t offset = 0, end = q.n;
-          for (uint32_t level = 0; level < len; ++level) {
-            const QueryLevel& L = q.lv[level];
-            if (bit(level)) {
-              offset = q.zeros[level] + q_rank1(L, offset);
-              end = q.zeros[level] + q_rank1(L, end);
-            } else {
-              offset = q_rank0(L, offset);
-              end = q_rank0(L, end);
-            }
-          }
-          if (occ <= end - offset) {
-            occ += offset;
-            for (int level = int(len) - 1; level >= 0; --level) {
-              const QueryLevel& L = q.lv[level];
-              const uint64_t adj = level == 0 ? 0 : 1;
-              if (bit(uint32_t(level))) occ = q_select(L, 1, occ - q.zeros[level]) + adj;
-              else occ = q_select(L, 0, occ) + adj;
-            }
-            result = occ;
-          }
-        }
+        bool bad = arg > S.n;
+        if (!bad && op == 1) result = query_rank<TREE, HUFF, uint32_t>(S, lv, code, len, uint32_t(arg));
+        if (!bad && op == 2) result = query_select<TREE, HUFF, uint32_t>(S, lv, node, code, len, uint32_t(arg), &bad);
+        if (bad) result = query_outside<TREE, HUFF>(S, lv, node, op, code, len, arg);
       }
     }
     out[t] = result;
   }
 }
 
+template <bool TREE, bool HUFF>
+void start_queries(const QueryStructure& q, const HuffQueryTables& h, int op, const uint8_t* ops, const uint64_t* a,
+                   const uint64_t* b, uint64_t count, uint64_t* out, cudaStream_t s) {
+  // a tree's selects hold 2 words a level and thread in shared memory: fewer
+  // threads a block for deep trees (at most 64 levels: 32 KB)
+  const bool nodes_used = TREE && (ops || op == 2);
+  unsigned threads = kQueryThreads;
+  while (nodes_used && size_t(2) * q.levels * threads * 4 > 32768) threads /= 2;
+  const size_t nodes = nodes_used ? size_t(2) * q.levels * threads * 4 : 0;
+  const dim3 grid(unsigned(std::min<uint64_t>((count + threads - 1) / threads, 152 * 512)), ops ? 3 : 1);
+  if constexpr (!HUFF) {  // mixed batches: plain structures
+    if (ops) {
+      query_kernel<-1, TREE, HUFF><<<grid, threads, nodes, s>>>(q, h, ops, a, b, count, out);
+      return;
+    }
+  }
+  if (op == 0) query_kernel<0, TREE, HUFF><<<grid, threads, 0, s>>>(q, h, nullptr, a, b, count, out);
+  else if (op == 1) query_kernel<1, TREE, HUFF><<<grid, threads, 0, s>>>(q, h, nullptr, a, b, count, out);
+  else query_kernel<2, TREE, HUFF><<<grid, threads, nodes, s>>>(q, h, nullptr, a, b, count, out);
+}
+
 }  // namespace
+
+void launch_queries(const QueryStructure& q, int op, const uint64_t* a, const uint64_t* b, uint64_t count,
+                    uint64_t* out, cudaStream_t s, uint64_t* launches, const uint8_t* ops) {
+  if (count == 0) return;
+  if (q.is_tree) start_queries<true, false>(q, HuffQueryTables{}, op, ops, a, b, count, out, s);
+  else start_queries<false, false>(q, HuffQueryTables{}, op, ops, a, b, count, out, s);
+  ++*launches;
+}
 
 void launch_huff_queries(const QueryStructure& q, const HuffQueryTables& h, int op, const uint64_t* a,
                          const uint64_t* b, uint64_t count, uint64_t* out, cudaStream_t s, uint64_t* launches) {
   if (count == 0) return;
-  uint64_t blocks = (count + 127) / 128;
-  if (blocks > 65535) blocks = 65535;
-  huff_query_kernel<<<unsigned(blocks), 128, 0, s>>>(q, h, op, a, b, count, out);
+  if (q.is_tree) start_queries<true, true>(q, h, op, nullptr, a, b, count, out, s);
+  else start_queries<false, true>(q, h, op, nullptr, a, b, count, out, s);
   ++*launches;
 }
 
@@ -614,15 +726,6 @@ void launch_rank_select(const RankSelectLevel* host_levels, uint32_t count, Rank
   rs_scan_kernel<<<count, 1024, 0, s>>>(dev_levels, tmp, tmp_words_per_level);
   rs_finish_kernel<<<g1, kRsThreads, 0, s>>>(dev_levels, tmp, tmp_words_per_level);
   *launches += 3;
-}
-
-void launch_queries(const QueryStructure& q, int op, const uint64_t* a, const uint64_t* b, uint64_t count,
-                    uint64_t* out, cudaStream_t s, uint64_t* launches, const uint8_t* ops) {
-  if (count == 0) return;
-  uint64_t blocks = (count + 127) / 128;
-  if (blocks > 65535) blocks = 65535;
-  query_kernel<<<unsigned(blocks), 128, 0, s>>>(q, op, ops, a, b, count, out);
-  ++*launches;
 }
 
 
