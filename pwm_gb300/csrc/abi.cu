@@ -452,6 +452,8 @@ pwmgpu_status pwmgpu_reduce_alphabet(pwmgpu_ctx* ctx, const void* d_text, uint64
     if (!valid_plain_width(word_width)) throw Fail{PWMGPU_ERR_ARG, "word_width must be 1, 2, 4 or 5"};
     *max_char = ~uint64_t(0);  // pwm: no symbol, 0 - 1
     if (size == 0) return PWMGPU_OK;
+    if (word_width != 5 && (reinterpret_cast<uintptr_t>(d_text) % word_width || reinterpret_cast<uintptr_t>(d_out) % word_width))
+      throw Fail{PWMGPU_ERR_ARG, "text and output must be aligned to their symbols"};
     cudaStream_t s = ctx->stream;
     CUDA_TRY(cudaMemsetAsync(ctx->d_status, 0, 4, s));
     uint64_t nsym = word_width == 1 ? 256 : 65536;
@@ -470,30 +472,19 @@ pwmgpu_status pwmgpu_reduce_alphabet(pwmgpu_ctx* ctx, const void* d_text, uint64
       *max_char = reduce_alphabet_hashed(ctx, d_text, size, word_width, d_out);
       return PWMGPU_OK;
     }
-    // symbol counts and first occurrences, then ids in order of first occurrence
-    auto* d_hist = static_cast<unsigned long long*>(ctx->grow("sym_hist", nsym * 8));
-    auto* d_first = static_cast<unsigned long long*>(ctx->grow("sym_first", nsym * 8));
-    CUDA_TRY(cudaMemsetAsync(d_hist, 0, nsym * 8, s));
-    CUDA_TRY(cudaMemsetAsync(d_first, 0xFF, nsym * 8, s));
+    // first positions, their ranks and the renumbered text on the device; the
+    // number of distinct symbols comes back through mapped memory
+    void* scratch = ctx->grow("alphabet", alphabet_scratch_bytes(size, nsym));
+    const uint64_t* distinct = ctx->grow_mapped(8);
     {
-      ProfScope ps(ctx, "symbol_histogram", size * word_width);
-      launch_symbol_histogram(d_text, size, word_width, nsym, d_hist, d_first, ctx->d_status, s, &ctx->launches);
+      ProfScope ps(ctx, "reduce_alphabet", 2 * size * word_width);
+      CUDA_TRY(launch_reduce_alphabet(d_text, size, word_width, nsym, d_out, scratch,
+                                      reinterpret_cast<unsigned long long*>(ctx->mapped_dev), ctx->d_status, s,
+                                      &ctx->launches));
     }
-    std::vector<uint64_t> count(nsym), first(nsym);
-    CUDA_TRY(cudaMemcpyAsync(count.data(), d_hist, nsym * 8, cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaMemcpyAsync(first.data(), d_first, nsym * 8, cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
-    std::vector<uint32_t> present;
-    for (uint64_t c = 0; c < nsym; ++c)
-      if (count[c]) present.push_back(uint32_t(c));
-    std::sort(present.begin(), present.end(), [&](uint32_t a, uint32_t b) { return first[a] < first[b]; });
-    std::vector<uint32_t> map(nsym, 0);
-    for (size_t i = 0; i < present.size(); ++i) map[present[i]] = uint32_t(i);
-    auto* d_map = static_cast<uint32_t*>(ctx->grow("alpha_map", nsym * 4));
-    CUDA_TRY(cudaMemcpyAsync(d_map, map.data(), nsym * 4, cudaMemcpyHostToDevice, s));
-    launch_remap(d_text, size, word_width, d_map, nsym, d_out, ctx->d_status, s, &ctx->launches);
-    check_device_status(ctx);  // also: the map's pageable copy has been read
-    *max_char = present.size() - 1;
+    if (word_width == 4) check_device_status(ctx);  // (every 8- and 16-bit symbol has its entry)
+    else CUDA_TRY(cudaStreamSynchronize(s));
+    *max_char = *distinct - 1;
     return PWMGPU_OK;
   });
 }

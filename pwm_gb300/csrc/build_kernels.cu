@@ -752,28 +752,11 @@ __global__ void huffman_keys_kernel(const T* text, uint64_t n, const uint64_t* c
   }
 }
 
-// First occurrence of every symbol: an atomicMin only where the index is
-// below the value already there, read with a plain (L1-cacheable) load, so
-// that the hot symbols, whose first occurrence the early blocks set, cost
-// neither atomics nor L2 traffic.  A stale cached value is never below the
-// current one (values only decrease), so it costs at most an extra atomic.
 template <typename T>
-__global__ void first_occurrence_kernel(const T* text, uint64_t n, unsigned long long* first) {
-  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
-    unsigned long long* f = &first[uint64_t(text[i])];
-    if (i < *f) atomicMin(f, (unsigned long long)i);
-  }
-}
-
-template <typename T>
-__global__ void symbol_hist_kernel(const T* text, uint64_t n, uint64_t nsym, unsigned long long* hist,
-                                   unsigned long long* first) {
+__global__ void symbol_hist_kernel(const T* text, uint64_t n, uint64_t nsym, unsigned long long* hist) {
   for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
     uint64_t c = uint64_t(text[i]);
-    if (c < nsym) {
-      atomicAdd(&hist[c], 1ull);
-      if (first) atomicMin(&first[c], (unsigned long long)i);
-    }
+    if (c < nsym) atomicAdd(&hist[c], 1ull);
   }
 }
 
@@ -991,26 +974,14 @@ __global__ void alphabet_insert_kernel(const uint8_t* text, uint32_t width, uint
         k = old == kEmptySlot ? v : old;
       }
       if (k == v) {
-        // first positions only decrease, so a stale value costs an extra atomic at most
-        if (i < first[h]) atomicMin(&first[h], (unsigned long long)i);
+        // first positions only move up in the text (their complements up), so a stale value costs an extra atomic
+        if (~i > first[h]) atomicMax(&first[h], ~(unsigned long long)i);
         placed = true;
         break;
       }
       h = (h + 1) & mask;
     }
     if (!placed) atomicOr(status, kErrBounds);
-  }
-}
-
-// The occupied slots, compacted: (slot, symbol, first position) per distinct symbol.
-__global__ void alphabet_collect_kernel(const unsigned long long* keys, const unsigned long long* first, uint64_t cap,
-                                        unsigned long long* count, uint64_t* out) {
-  for (uint64_t h = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; h < cap; h += uint64_t(gridDim.x) * blockDim.x) {
-    if (keys[h] == kEmptySlot) continue;
-    const unsigned long long k = atomicAdd(count, 1ull);
-    out[3 * k] = h;
-    out[3 * k + 1] = keys[h];
-    out[3 * k + 2] = first[h];
   }
 }
 
@@ -1046,16 +1017,10 @@ __global__ void alphabet_remap_kernel(const uint8_t* text, uint32_t width, uint6
   }
 }
 
-__global__ void scatter_ids_kernel(const uint64_t* slots, const uint32_t* ids, uint64_t count, uint32_t* slot_ids) {
-  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += uint64_t(gridDim.x) * blockDim.x)
-    slot_ids[slots[i]] = ids[i];
-}
-
-// Largest symbol of a 32-bit text (warp maxima, one atomic per warp).
 __global__ void max_symbol_kernel(const uint32_t* text, uint64_t n, unsigned int* out) {
   uint32_t m = 0;
-  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
-    m = max(m, text[i]);
+  for_each_symbol_vec<uint32_t>(text, n, uint64_t(blockIdx.x) * blockDim.x + threadIdx.x,
+                                uint64_t(gridDim.x) * blockDim.x, [&](uint64_t c) { m = max(m, uint32_t(c)); });
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, d));
   if ((threadIdx.x & 31) == 0) atomicMax(out, m);
@@ -1254,20 +1219,13 @@ void launch_huffman_keys(const void* text, uint64_t n, uint32_t width, const uin
 }
 
 void launch_symbol_histogram(const void* text, uint64_t n, uint32_t width, uint64_t nsym, unsigned long long* hist,
-                             unsigned long long* first, uint32_t* status, cudaStream_t s, uint64_t* launches) {
+                             uint32_t* status, cudaStream_t s, uint64_t* launches) {
   if (n == 0) return;
-  const int g = grid_for(n, 256);
-  if (width <= 2) {
-    // every value is a bin: the shared-memory leaf histograms of 8 / 16 levels
+  if (width <= 2) {  // every value is a bin: the shared-memory leaf histograms of 8 / 16 levels
     launch_leaf_histogram(text, n, width, 8 * width, hist, status, s, launches);
-    if (first) {
-      if (width == 1) first_occurrence_kernel<<<g, 256, 0, s>>>(static_cast<const uint8_t*>(text), n, first);
-      else first_occurrence_kernel<<<g, 256, 0, s>>>(static_cast<const uint16_t*>(text), n, first);
-      ++*launches;
-    }
     return;
   }
-  symbol_hist_kernel<<<g, 256, 0, s>>>(static_cast<const uint32_t*>(text), n, nsym, hist, first);
+  symbol_hist_kernel<<<grid_for(n, 256), 256, 0, s>>>(static_cast<const uint32_t*>(text), n, nsym, hist);
   ++*launches;
 }
 
@@ -1333,19 +1291,6 @@ void launch_alphabet_insert(const void* text, uint32_t width, uint64_t n, unsign
   ++*launches;
 }
 
-void launch_alphabet_collect(const unsigned long long* keys, const unsigned long long* first, uint64_t cap,
-                             unsigned long long* count, uint64_t* out, cudaStream_t s, uint64_t* launches) {
-  alphabet_collect_kernel<<<grid_for(cap, 256), 256, 0, s>>>(keys, first, cap, count, out);
-  ++*launches;
-}
-
-void launch_scatter_ids(const uint64_t* slots, const uint32_t* ids, uint64_t count, uint32_t* slot_ids, cudaStream_t s,
-                        uint64_t* launches) {
-  if (count == 0) return;
-  scatter_ids_kernel<<<grid_for(count, 256), 256, 0, s>>>(slots, ids, count, slot_ids);
-  ++*launches;
-}
-
 void launch_alphabet_remap(const void* text, uint32_t width, uint64_t n, const unsigned long long* keys,
                            const uint32_t* slot_ids, uint64_t cap, void* out, uint32_t* status, cudaStream_t s,
                            uint64_t* launches) {
@@ -1357,7 +1302,7 @@ void launch_alphabet_remap(const void* text, uint32_t width, uint64_t n, const u
 
 void launch_max_symbol(const uint32_t* text, uint64_t n, unsigned int* out, cudaStream_t s, uint64_t* launches) {
   if (n == 0) return;
-  max_symbol_kernel<<<grid_for(n, 256), 256, 0, s>>>(text, n, out);
+  max_symbol_kernel<<<grid_for((n + 3) / 4, 256), 256, 0, s>>>(text, n, out);
   ++*launches;
 }
 

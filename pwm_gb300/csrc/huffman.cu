@@ -18,20 +18,24 @@ HuffCodes huffman_codes_device(pwmgpu_ctx* ctx, const void* d_text, uint64_t n, 
     // bound the alphabet by the largest symbol (one histogram bin per value)
     throw Fail{PWMGPU_ERR_ARG, "Huffman codes for 32-bit texts: pass a code table"};
   }
-  auto* d_hist = static_cast<unsigned long long*>(ctx->grow("sym_hist", nsym * 8));
-  auto* d_first = static_cast<unsigned long long*>(ctx->grow("sym_first", nsym * 8));
-  CUDA_TRY(cudaMemsetAsync(d_hist, 0, nsym * 8, s));
-  CUDA_TRY(cudaMemsetAsync(d_first, 0xFF, nsym * 8, s));
+  // counts, ~first positions and the scratch of the latter, zeroed together
+  const uint64_t seen_bytes = 65536 / 8 + 8;
+  auto* d_hist = static_cast<unsigned long long*>(ctx->grow("sym_first", nsym * 16 + seen_bytes));
+  auto* d_first = d_hist + nsym;
+  CUDA_TRY(cudaMemsetAsync(d_hist, 0, nsym * 16 + seen_bytes, s));
   CUDA_TRY(cudaMemsetAsync(ctx->d_status, 0, 4, s));
   {
     ProfScope ps(ctx, "symbol_histogram", n * width);
-    launch_symbol_histogram(d_text, n, width, nsym, d_hist, width == 1 ? nullptr : d_first, ctx->d_status, s,
-                            &ctx->launches);
+    launch_symbol_histogram(d_text, n, width, nsym, d_hist, ctx->d_status, s, &ctx->launches);
+    if (width > 1)
+      launch_first_positions(d_text, n, width, nsym, d_first, reinterpret_cast<uint32_t*>(d_first + nsym), s,
+                             &ctx->launches);
   }
   std::vector<uint64_t> count(nsym), first(nsym);
   CUDA_TRY(cudaMemcpyAsync(count.data(), d_hist, nsym * 8, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaMemcpyAsync(first.data(), d_first, nsym * 8, cudaMemcpyDeviceToHost, s));
+  if (width > 1) CUDA_TRY(cudaMemcpyAsync(first.data(), d_first, nsym * 8, cudaMemcpyDeviceToHost, s));
   CUDA_TRY(cudaStreamSynchronize(s));
+  for (auto& f : first) f = ~f;
   uint64_t max_symbol = 0;
   for (uint64_t c = 0; c < nsym; ++c)
     if (count[c]) max_symbol = c;
@@ -56,7 +60,7 @@ void build_huffman(pwmgpu_ctx* ctx, const void* d_text, uint64_t n, uint32_t wid
   CUDA_TRY(cudaMemsetAsync(d_hist, 0, bins * 8, s));
   {
     ProfScope ps(ctx, "symbol_histogram", n * width);
-    launch_symbol_histogram(d_text, n, width, nsym, d_hist, nullptr, ctx->d_status, s, &ctx->launches);
+    launch_symbol_histogram(d_text, n, width, nsym, d_hist, ctx->d_status, s, &ctx->launches);
   }
   std::vector<uint64_t> count(nsym);
   CUDA_TRY(cudaMemcpyAsync(count.data(), d_hist, nsym * 8, cudaMemcpyDeviceToHost, s));

@@ -40,21 +40,36 @@ void launch_readback(const unsigned long long* src, uint64_t n, const uint32_t* 
                      cudaStream_t s, uint64_t* launches);
 // Alphabet reduction of 32- or 40-bit symbols (width 4 or 5) through a hash
 // table of `cap` (a power of two, at least twice the text) slots: keys set to
-// all ones and first positions to all ones by the caller; insert, collect the
-// occupied slots as (slot, symbol, first) triples (count zeroed by the
-// caller), scatter the ids the host assigns to their slots, remap.
+// all ones, first (the complements of first positions) to zero by the caller;
+// insert, rank the slots, remap.
 void launch_alphabet_insert(const void* text, uint32_t width, uint64_t n, unsigned long long* keys,
                             unsigned long long* first, uint64_t cap, uint32_t* status, cudaStream_t s,
                             uint64_t* launches);
-void launch_alphabet_collect(const unsigned long long* keys, const unsigned long long* first, uint64_t cap,
-                             unsigned long long* count, uint64_t* out, cudaStream_t s, uint64_t* launches);
-void launch_scatter_ids(const uint64_t* slots, const uint32_t* ids, uint64_t count, uint32_t* slot_ids, cudaStream_t s,
-                        uint64_t* launches);
+// ids[h]: the rank of slot h's first position among all (positions below n);
+// *distinct (device view of mapped host memory): the occupied slots.
+// scratch: alphabet_rank_scratch_bytes(n) bytes.
+uint64_t alphabet_rank_scratch_bytes(uint64_t n);
+cudaError_t launch_rank_slots(const unsigned long long* first, uint64_t cap, uint64_t n, void* scratch, uint32_t* ids,
+                              unsigned long long* distinct, cudaStream_t s, uint64_t* launches);
 void launch_alphabet_remap(const void* text, uint32_t width, uint64_t n, const unsigned long long* keys,
                            const uint32_t* slot_ids, uint64_t cap, void* out, uint32_t* status, cudaStream_t s,
                            uint64_t* launches);
-// Largest symbol of a 32-bit text into *out (zeroed by the caller).
+// Largest symbol of a 32-bit text (4-byte aligned) into *out (zeroed by the caller).
 void launch_max_symbol(const uint32_t* text, uint64_t n, unsigned int* out, cudaStream_t s, uint64_t* launches);
+// Alphabet reduction of 8-, 16- and 32-bit symbols below nsym (256, 65536, up
+// to 2^24): `out` (in place allowed; both aligned to the symbol) the text
+// renumbered in order of first occurrence, *distinct (device view of mapped
+// host memory) the number of distinct symbols.  scratch:
+// alphabet_scratch_bytes(n, nsym) bytes.
+uint64_t alphabet_scratch_bytes(uint64_t n, uint64_t nsym);
+cudaError_t launch_reduce_alphabet(const void* text, uint64_t n, uint32_t width, uint64_t nsym, void* out,
+                                   void* scratch, unsigned long long* distinct, uint32_t* status, cudaStream_t s,
+                                   uint64_t* launches);
+// ~(the first position) of every symbol below nsym into first[0..nsym), which
+// is zeroed by the caller (0: the symbol does not occur).  seen: scratch of
+// max(65536, nsym rounded up to 256) / 8 + 4 bytes, zeroed.
+void launch_first_positions(const void* text, uint64_t n, uint32_t width, uint64_t nsym, unsigned long long* first,
+                            uint32_t* seen, cudaStream_t s, uint64_t* launches);
 // out[i] = map[text[i]] (same width; in place allowed).
 void launch_remap(const void* text, uint64_t n, uint32_t width, const uint32_t* map, uint64_t nmap, void* out,
                   uint32_t* status, cudaStream_t s, uint64_t* launches);
@@ -185,12 +200,10 @@ void launch_huffman_keys(const void* text, uint64_t n, uint32_t width, const uin
                          const uint64_t* code_word, uint64_t ncodes, uint32_t levels, uint32_t key_bytes, void* keys,
                          uint32_t* status, cudaStream_t s, uint64_t* launches);
 // Histogram of the symbols (u64 counts; 8- and 16-bit texts: all 2^8 / 2^16
-// values, so hist needs that many entries; 32-bit texts: symbols below nsym)
-// and, with `first` (filled with UINT64_MAX), the first position of every
-// symbol.  hist must be zeroed.
+// values, so hist needs that many entries; 32-bit texts: symbols below nsym).
+// hist must be zeroed.
 void launch_symbol_histogram(const void* text, uint64_t n, uint32_t width, uint64_t nsym,
-                             unsigned long long* hist, unsigned long long* first, uint32_t* status, cudaStream_t s,
-                             uint64_t* launches);
+                             unsigned long long* hist, uint32_t* status, cudaStream_t s, uint64_t* launches);
 
 // ---- rank / select --------------------------------------------------------------
 struct RankSelectLevel {

