@@ -107,47 +107,45 @@ void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint
 }
 
 // Rank/select blocks of every level of the given structures (asynchronous),
-// all levels in one launch sequence.  share_level0: a plain matrix and tree,
-// whose level 0 is the same bit vector: the tree's blocks of level 0 are a
-// copy of the matrix's.  The kernels write every entry that is read (l0 is
-// cleared by the scan kernel), so nothing is zeroed first.
+// all levels in one launch.  share_level0: a plain matrix and tree, whose
+// level 0 is the same bit vector: counted once, written to both.
 //
-// Levels [lo, hi) only, on `stream` (default: the context's) with scratch
-// buffers named after `tag` (so that two groups can run at once); only the
+// Levels [lo, hi) only, on `stream` (default: the context's) with a scratch
+// buffer named after `tag` (so that two groups can run at once); only the
 // context's stream is profiled.
 void build_rank_select(pwmgpu_ctx* ctx, Structure* wm, Structure* wt, bool share_level0, uint32_t lo, uint32_t hi,
                        cudaStream_t stream, const char* tag) {
-  std::vector<RankSelectLevel> lv;
-  auto add = [&](const Structure* st, uint32_t from) {
-    for (uint32_t l = std::max(lo, from); l < std::min(hi, st->levels); ++l) lv.push_back(st->rs_levels[l]);
+  uint64_t max_words = 0, bytes = 0;
+  auto take = [&](const Structure* st, uint32_t from, uint32_t* first) -> uint32_t {
+    if (!st || !st->rs) return 0;
+    *first = std::max(lo, from);
+    const uint32_t end = std::min(hi, st->levels);
+    for (uint32_t l = *first; l < end; ++l) {
+      const uint64_t w = st->rs_levels[l].nwords;
+      max_words = std::max(max_words, w);
+      bytes += w * 8 + (w / 32 + 1) * 8;
+    }
+    return end > *first ? end - *first : 0;
   };
-  if (wm && wm->rs) add(wm, 0);
-  const bool copy0 = share_level0 && lo == 0 && hi > 0 && wm && wm->rs && wm->levels && wt && wt->rs && wt->levels;
-  if (wt && wt->rs) add(wt, copy0 ? 1 : 0);
-  if (lv.empty() && !copy0) return;
+  RankSelectArgs a{};
+  a.twin = share_level0 && lo == 0 && hi > 0 && wm && wm->rs && wm->levels && wt && wt->rs && wt->levels;
+  a.nfirst = take(wm, 0, &a.first_lo);
+  a.nsecond = take(wt, a.twin ? 1 : 0, &a.second_lo);
+  if (a.nfirst + a.nsecond == 0) return;
+  a.first = a.nfirst ? wm->d_rs_levels : nullptr;
+  a.second = wt && wt->rs ? wt->d_rs_levels : nullptr;
   cudaStream_t s = stream ? stream : ctx->stream;
-  const std::string t(tag);
-  if (!lv.empty()) {
-    auto* d_lv = static_cast<RankSelectLevel*>(ctx->grow("rs_levels" + t, lv.size() * sizeof(RankSelectLevel)));
-    CUDA_TRY(cudaMemcpyAsync(d_lv, lv.data(), lv.size() * sizeof(RankSelectLevel), cudaMemcpyHostToDevice, s));
-    uint64_t max_real = 0, bytes = 0;
-    for (auto& r : lv) {
-      max_real = std::max<uint64_t>(max_real, (r.nwords + 31) / 32);
-      bytes += r.nwords * 8 + (r.nwords / 32 + 1) * 8;
-    }
-    const uint64_t stride = max_real + (max_real + 255) / 256 + 1;
-    uint32_t* tmp = static_cast<uint32_t*>(ctx->grow("rs_tmp" + t, std::max<uint64_t>(stride * lv.size() * 4, 256)));
-    if (s == ctx->stream) {
-      ProfScope ps(ctx, "rank_select", bytes);
-      launch_rank_select(lv.data(), uint32_t(lv.size()), d_lv, tmp, stride, s, &ctx->launches);
-    } else {
-      launch_rank_select(lv.data(), uint32_t(lv.size()), d_lv, tmp, stride, s, &ctx->launches);
-    }
-  }
-  if (copy0) {  // l0, l12, samples and meta of level 0 lie in this order in both structures
-    const RankSelectLevel &a = wm->rs_levels[0], &b = wt->rs_levels[0];
-    const size_t n = size_t(reinterpret_cast<const char*>(a.meta + 3) - reinterpret_cast<const char*>(a.l0));
-    CUDA_TRY(cudaMemcpyAsync(b.l0, a.l0, n, cudaMemcpyDeviceToDevice, s));
+  a.stride = rank_select_state_words(max_words);
+  const uint64_t state_bytes = a.stride * (a.nfirst + a.nsecond) * 8;
+  a.state = static_cast<unsigned long long*>(ctx->grow("rs_state" + std::string(tag), state_bytes));
+  a.status = ctx->d_status;
+  a.spin_limit = kSpinLimit;
+  CUDA_TRY(cudaMemsetAsync(a.state, 0, state_bytes, s));
+  if (s == ctx->stream) {
+    ProfScope ps(ctx, "rank_select", bytes);
+    launch_rank_select(a, max_words, s, &ctx->launches);
+  } else {
+    launch_rank_select(a, max_words, s, &ctx->launches);
   }
 }
 

@@ -215,10 +215,24 @@ struct RankSelectLevel {
   uint32_t* s1;
   unsigned long long* meta;  // [0] ns0, [1] ns1, [2] total ones
 };
-// Builds pwm's rank/select blocks for `count` levels.  tmp must hold
-// max(ceil(nwords/32)) + 1 u32 per level plus per-CTA totals (see .cu).
-void launch_rank_select(const RankSelectLevel* host_levels, uint32_t count, RankSelectLevel* dev_levels,
-                        uint32_t* tmp, uint64_t tmp_words_per_level, cudaStream_t s, uint64_t* launches);
+// Rank/select of levels first[first_lo..+nfirst) and second[second_lo..
+// +nsecond) (device arrays; first == nullptr: the one level `one`).  twin:
+// level first[0]'s outputs go to second[0]'s arrays too (a plain matrix and
+// tree share level 0).  state: zeroed, `stride` =
+// rank_select_state_words(words of the longest level) words a level.
+struct RankSelectArgs {
+  const RankSelectLevel* first;
+  const RankSelectLevel* second;
+  RankSelectLevel one;
+  uint32_t first_lo, nfirst, second_lo, nsecond;
+  uint32_t twin;
+  uint32_t spin_limit;
+  uint64_t stride;
+  unsigned long long* state;
+  uint32_t* status;
+};
+uint64_t rank_select_state_words(uint64_t max_words);
+void launch_rank_select(const RankSelectArgs& a, uint64_t max_words, cudaStream_t s, uint64_t* launches);
 
 struct QueryLevel {
   const uint64_t* data;

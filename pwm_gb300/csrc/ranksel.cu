@@ -19,29 +19,125 @@ namespace pwmgpu {
 namespace {
 
 constexpr uint64_t kL1Bits = 2048, kL1Cover = 32, kL2Cover = 8, kSampleRate = 8192;
-constexpr int kRsThreads = 256;
+constexpr int kRsThreads = 512;
 
-// Phase 1: per L1 block popcounts, l2 fields, and the exclusive prefix of
-// block totals inside each CTA (256 blocks per CTA).  Warp w reads its 32
-// blocks (8 KB) with coalesced 16-byte loads: in step i, lanes 0-15 read
-// block 2i and lanes 16-31 block 2i+1, four lanes per 512-bit L2 block; the
-// counts are then gathered so that lane b holds block b's.
-__global__ void __launch_bounds__(kRsThreads) rs_blocks_kernel(const RankSelectLevel* lv, uint32_t* tmp,
-                                                              uint64_t tmp_stride) {
-  const RankSelectLevel L = lv[blockIdx.y];
-  const uint64_t nreal = (L.nwords + kL1Cover - 1) / kL1Cover;
-  const uint64_t first = uint64_t(blockIdx.x) * kRsThreads;
-  if (first >= nreal) return;
-  uint32_t* intra = tmp + blockIdx.y * tmp_stride;
-  uint32_t* cta_tot = intra + nreal;
-  __shared__ uint32_t tot[kRsThreads];
+// Select-sample position inside L1 block b: the `rem`-th one (value 1) or
+// zero (value 0) counted from the block's first word, found by one thread.
+// pwm walks the L2 blocks and then the words of the block
+// (bin_select_popcnt.hpp:55-99); skipping whole L2 blocks by their counts
+// first does not change which word and rank it ends on, so this gives the
+// same position.  Only words of the level count (the last block may be
+// short).  rem == 0 is pwm's word_select1(first word, 0).  Returns false when
+// the block ends before the rem-th bit (pwm then takes no sample).
+__device__ __forceinline__ bool thread_block_select(const uint64_t* data, uint64_t nwords, uint32_t fields,
+                                                    uint64_t b, int value, uint32_t rem, uint64_t* pos) {
+  const uint64_t w0 = b * kL1Cover;
+  if (rem == 0) {
+    const uint64_t first = value ? data[w0] : ~data[w0];
+    *pos = word_select1(first, 0) + 64 * w0;
+    return true;
+  }
+  // skip whole L2 blocks (8 words) by their counts; the fourth has no field
+  uint32_t sub = 0;
+  for (; sub < 3; ++sub) {
+    const uint64_t ws = w0 + kL2Cover * sub;
+    const uint64_t left = ws >= nwords ? 0 : nwords - ws;
+    const uint32_t words = uint32_t(left < kL2Cover ? left : kL2Cover);
+    const uint32_t ones = (fields >> (10 * sub)) & 1023u;
+    const uint32_t cnt = value ? ones : 64u * words - ones;
+    if (rem <= cnt) break;
+    rem -= cnt;
+  }
+  const uint64_t ws = w0 + kL2Cover * sub;
+  if (ws + kL2Cover <= nwords && (reinterpret_cast<uintptr_t>(data) & 15) == 0) {
+    // a whole L2 block: its words at once, the one that holds the bit by their counts
+    const uint4* v = reinterpret_cast<const uint4*>(data + ws);
+    uint64_t w[kL2Cover];
+#pragma unroll
+    for (uint32_t k = 0; k < kL2Cover / 2; ++k) {
+      const uint4 x = v[k];
+      w[2 * k] = uint64_t(x.y) << 32 | x.x;
+      w[2 * k + 1] = uint64_t(x.w) << 32 | x.z;
+    }
+    uint32_t run = 0, at = kL2Cover, left = 0;
+    uint64_t word = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kL2Cover; ++k) {
+      const uint64_t y = value ? w[k] : ~w[k];
+      const uint32_t pc = uint32_t(__popcll(y));
+      if (rem > run && rem <= run + pc) {
+        at = k;
+        left = rem - run;
+        word = y;
+      }
+      run += pc;
+    }
+    if (at < kL2Cover) {
+      *pos = word_select1(word, left) + 64 * (ws + at);
+      return true;
+    }
+    return false;
+  }
+  for (uint32_t k = 0; k < kL2Cover; ++k) {
+    if (ws + k >= nwords) return false;
+    const uint64_t w = value ? data[ws + k] : ~data[ws + k];
+    const uint32_t pc = uint32_t(__popcll(w));
+    if (pc >= rem) {
+      *pos = word_select1(w, rem) + 64 * (ws + k);
+      return true;
+    }
+    rem -= pc;
+  }
+  return false;
+}
+
+// One pass over the words: a CTA counts 512 L1 blocks (128 KB of a level),
+// learns the ones before them by a decoupled look-back over the level's CTAs
+// and writes the finished entries and the select samples that fall into its
+// blocks, whose words are still in L2.  (Three kernels before: block counts
+// into scratch, a scan of the CTA totals, and the entries and samples from
+// the scratch and a second look at the words.  Both structures of 10^6 bytes,
+// 8 levels: 12 us of kernels and two more launches -> 7 us; 8 levels of 2^30
+// bits 261 -> 254 us, 171 of them the reading and counting, the rest waits on
+// predecessors and samples.)  CTAs take their place in
+// the level by ticket, so a CTA waits only for CTAs that already run; the wait
+// is bounded (kErrTimeout, a zero prefix).  Consecutive CTAs belong to
+// different levels: with the resident CTAs all in one level, prefixes reached
+// them too slowly (8 levels of 2^30 bits 388 against 273 us, both with 256
+// threads; 512 threads 254).  Looking back over 64 to 256 CTAs a step changed
+// nothing: the wait is for the slowest loads.
+//
+// Counting: warp w reads its 32 blocks (8 KB) with coalesced 16-byte loads: in
+// step i, lanes 0-15 read block 2i and lanes 16-31 block 2i+1, four lanes per
+// 512-bit L2 block; the counts are then gathered so that lane b holds block
+// b's.
+__global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSelectArgs a) {
+  const uint32_t y = blockIdx.x;
+  RankSelectLevel L, twin{};
+  bool twinned = false;
+  if (y < a.nfirst) {
+    L = a.first ? a.first[a.first_lo + y] : a.one;
+    twinned = a.twin && a.first_lo + y == 0;  // level 0 of a plain tree is the matrix's
+    if (twinned) twin = a.second[0];
+  } else {
+    L = a.second[a.second_lo + y - a.nfirst];
+  }
+  const uint64_t nreal = (L.nwords + kL1Cover - 1) / kL1Cover, n12 = L.nwords / kL1Cover + 1;
+  const uint64_t ctas = nreal ? (nreal + kRsThreads - 1) / kRsThreads : 1;
+  if (blockIdx.y >= ctas) return;
+  unsigned long long* state = a.state + uint64_t(y) * a.stride;  // a ticket, then a word a CTA
+  __shared__ uint32_t s_cta;
+  if (threadIdx.x == 0) s_cta = uint32_t(atomicAdd(state, 1ull));
+  __syncthreads();
+  const uint32_t cta = s_cta;
+  const uint64_t first = uint64_t(cta) * kRsThreads;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t l2[4] = {0, 0, 0, 0};
   {
     const uint64_t wb = first + 32 * uint64_t(warp);  // first block of this warp
     const uint64_t ww = wb * kL1Cover;                 // first word of this warp
     // 16-byte loads when the warp's words are all in the level and aligned
     const bool full = ww + 32 * kL1Cover <= L.nwords && (reinterpret_cast<uintptr_t>(L.data) & 15) == 0;
-    uint32_t l2[4] = {0, 0, 0, 0};
     auto gather = [&](int i, uint32_t c) {
       c += __shfl_xor_sync(0xFFFFFFFFu, c, 1);
       c += __shfl_xor_sync(0xFFFFFFFFu, c, 2);
@@ -57,7 +153,7 @@ __global__ void __launch_bounds__(kRsThreads) rs_blocks_kernel(const RankSelectL
       uint32_t c[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const uint4 v = __ldcs(reinterpret_cast<const uint4*>(L.data + ww + 2 * uint64_t(i * 32 + lane)));
+        const uint4 v = *reinterpret_cast<const uint4*>(L.data + ww + 2 * uint64_t(i * 32 + lane));
         c[i] = __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
       }
 #pragma unroll
@@ -68,177 +164,111 @@ __global__ void __launch_bounds__(kRsThreads) rs_blocks_kernel(const RankSelectL
         gather(i, (w < L.nwords ? __popcll(L.data[w]) : 0) + (w + 1 < L.nwords ? __popcll(L.data[w + 1]) : 0));
       }
     }
-    const uint64_t blk = wb + lane;
-    if (blk < nreal) L.l12[2 * blk + 1] = (l2[0] & 1023u) | ((l2[1] & 1023u) << 10) | ((l2[2] & 1023u) << 20);
-    tot[threadIdx.x] = blk < nreal ? l2[0] + l2[1] + l2[2] + l2[3] : 0u;
   }
-  // exclusive scan of the 256 block totals (u32, wrapping)
-  uint32_t v = tot[threadIdx.x];
+  // exclusive scan of the block totals (past the level: 0)
+  const uint32_t v = l2[0] + l2[1] + l2[2] + l2[3];
   uint32_t x = v;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-    if (lane >= d) x += y;
+    const uint32_t s = __shfl_up_sync(0xFFFFFFFFu, x, d);
+    if (lane >= d) x += s;
   }
   __shared__ uint32_t wsum[kRsThreads / 32];
+  __shared__ unsigned long long s_before;
   if (lane == 31) wsum[warp] = x;
   __syncthreads();
+  uint32_t before_warp = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < kRsThreads / 32; ++w) {
+    before_warp += w < warp ? wsum[w] : 0u;
+    total += wsum[w];
+  }
+  // publish, then look back 32 CTAs a step
   if (warp == 0) {
-    uint32_t s = lane < kRsThreads / 32 ? wsum[lane] : 0;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      uint32_t y = __shfl_up_sync(0xFFFFFFFFu, s, d);
-      if (lane >= d) s += y;
-    }
-    if (lane < kRsThreads / 32) wsum[lane] = s;  // inclusive
-  }
-  __syncthreads();
-  const uint32_t warp_excl = warp ? wsum[warp - 1] : 0u;
-  const uint64_t blk = first + threadIdx.x;
-  if (blk < nreal) intra[blk] = warp_excl + x - v;
-  if (threadIdx.x == kRsThreads - 1) cta_tot[blockIdx.x] = warp_excl + x;
-}
-
-// Phase 2: one CTA per level scans the CTA totals (exclusive, u32 wrap) and
-// the exact u64 total of ones.
-__global__ void __launch_bounds__(1024) rs_scan_kernel(const RankSelectLevel* lv, uint32_t* tmp,
-                                                       uint64_t tmp_stride) {
-  const RankSelectLevel L = lv[blockIdx.x];
-  const uint64_t nreal = (L.nwords + kL1Cover - 1) / kL1Cover;
-  const uint64_t ncta = (nreal + kRsThreads - 1) / kRsThreads;
-  uint32_t* cta_tot = tmp + blockIdx.x * tmp_stride + nreal;
-  // l0: all zero below 2^32-1 bits per level (the only sizes built); the
-  // sample counts stay 0 for levels too short to examine a block
-  // (rs_finish_kernel writes them otherwise)
-  for (uint64_t i = threadIdx.x; i < L.nwords / (4294967295ull / 64) + 1; i += blockDim.x) L.l0[i] = 0;
-  if (threadIdx.x == 0) {
-    L.meta[0] = 0;
-    L.meta[1] = 0;
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __shared__ unsigned long long wsum[32];
-  __shared__ unsigned long long carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (uint64_t base = 0; base < ncta; base += 1024) {
-    const uint64_t i = base + threadIdx.x;
-    const unsigned long long v = i < ncta ? cta_tot[i] : 0ull;
-    unsigned long long x = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-      if (lane >= d) x += y;
-    }
-    if (lane == 31) wsum[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-      unsigned long long s = wsum[lane];
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, s, d);
-        if (lane >= d) s += y;
+    unsigned long long before = 0;
+    if (lane == 0) st_volatile(state + 1 + cta, (cta == 0 ? kFlagPrefix : kFlagAggregate) | total);
+    for (int64_t at = int64_t(cta) - 1; at >= 0; at -= 32) {
+      const int64_t k = at - lane;
+      uint64_t w = kFlagPrefix;  // before the level: nothing
+      if (k >= 0) {
+        w = ld_volatile(state + 1 + k);
+        for (uint32_t spins = 0; (w >> 62) == 0; ++spins) {
+          if (spins >= a.spin_limit) {
+            atomicOr(a.status, kErrTimeout);
+            w = kFlagPrefix;
+            break;
+          }
+          __nanosleep(32);
+          w = ld_volatile(state + 1 + k);
+        }
       }
-      wsum[lane] = s;
+      const uint32_t done = __ballot_sync(0xFFFFFFFFu, (w >> 62) == 2);
+      const int stop = done ? __ffs(done) - 1 : 31;  // the nearest CTA with everything before it
+      unsigned long long c = lane <= stop ? (w & kCountMask) : 0ull;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, d);
+      before += c;
+      if (done) break;
     }
-    __syncthreads();
-    const unsigned long long excl = carry + (warp ? wsum[warp - 1] : 0ull) + x - v;
-    if (i < ncta) cta_tot[i] = uint32_t(excl);  // now the CTA's exclusive offset
-    __syncthreads();
-    if (threadIdx.x == 1023) carry = excl + v;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) L.meta[2] = carry;  // total ones of the level
-}
-
-__device__ __forceinline__ uint32_t l1_value(const uint32_t* intra, const uint32_t* cta_off, uint64_t nreal,
-                                             uint64_t e) {
-  // pwm's l1 value of entry e; the extra entry past the real blocks is 0.
-  return e < nreal ? cta_off[e / kRsThreads] + intra[e] : 0u;
-}
-
-// Select-sample position inside L1 block b: the `rem`-th one (value 1) or
-// zero (value 0) counted from the block's first word, found by one thread.
-// pwm walks the L2 blocks and then the words of the block
-// (bin_select_popcnt.hpp:55-99); skipping whole L2 blocks by their counts
-// first does not change which word and rank it ends on, so this gives the
-// same position.  Only words of the level count (the last block may be
-// short).  rem == 0 is pwm's word_select1(first word, 0).  Returns false when
-// the block ends before the rem-th bit (pwm then takes no sample).
-__device__ __forceinline__ bool thread_block_select(const uint64_t* data, uint64_t nwords, const uint32_t* l12,
-                                                    uint64_t b, int value, uint32_t rem, uint64_t* pos) {
-  const uint64_t w0 = b * kL1Cover;
-  if (rem == 0) {
-    const uint64_t first = value ? data[w0] : ~data[w0];
-    *pos = word_select1(first, 0) + 64 * w0;
-    return true;
-  }
-  // skip whole L2 blocks (8 words) by their counts; the fourth has no field
-  const uint32_t fields = l12[2 * b + 1];
-  uint32_t sub = 0;
-  for (; sub < 3; ++sub) {
-    const uint64_t ws = w0 + kL2Cover * sub;
-    const uint64_t left = ws >= nwords ? 0 : nwords - ws;
-    const uint32_t words = uint32_t(left < kL2Cover ? left : kL2Cover);
-    const uint32_t ones = (fields >> (10 * sub)) & 1023u;
-    const uint32_t cnt = value ? ones : 64u * words - ones;
-    if (rem <= cnt) break;
-    rem -= cnt;
-  }
-  const uint64_t ws = w0 + kL2Cover * sub;
-  for (uint32_t k = 0; k < kL2Cover; ++k) {
-    if (ws + k >= nwords) return false;
-    const uint64_t w = value ? data[ws + k] : ~data[ws + k];
-    const uint32_t pc = uint32_t(__popcll(w));
-    if (pc >= rem) {
-      *pos = word_select1(w, rem) + 64 * (ws + k);
-      return true;
+    if (lane == 0) {
+      if (cta) st_volatile(state + 1 + cta, kFlagPrefix | (before + total));
+      s_before = before;
     }
-    rem -= pc;
   }
-  return false;
-}
-
-// Phase 3: l1 values and the select samples, one thread per L1 block (the
-// searches of a warp's blocks are independent, so their loads overlap).
-__global__ void __launch_bounds__(kRsThreads) rs_finish_kernel(const RankSelectLevel* lv, const uint32_t* tmp,
-                                                              uint64_t tmp_stride) {
-  const RankSelectLevel L = lv[blockIdx.y];
-  const uint64_t nreal = (L.nwords + kL1Cover - 1) / kL1Cover;
-  const uint64_t n12 = L.nwords / kL1Cover + 1;
-  const uint32_t* intra = tmp + blockIdx.y * tmp_stride;
-  const uint32_t* cta_off = intra + nreal;
-  const uint64_t b = uint64_t(blockIdx.x) * kRsThreads + threadIdx.x;
+  __syncthreads();
+  const uint64_t level_before = s_before;
+  auto finish = [&](const RankSelectLevel& R) {  // the outputs of one structure
+    if (cta == 0) {
+      // all zero below 2^32-1 bits per level (the only sizes built)
+      for (uint64_t i = threadIdx.x; i < L.nwords / (4294967295ull / 64) + 1; i += kRsThreads) R.l0[i] = 0;
+      if (threadIdx.x == 0) {
+        if (n12 < 2) R.meta[0] = R.meta[1] = 0;  // too short for pwm to examine a block
+        if (n12 > nreal) R.l12[2 * nreal] = R.l12[2 * nreal + 1] = 0;
+      }
+    }
+    if (threadIdx.x == 0 && cta + 1 == ctas) R.meta[2] = level_before + total;  // ones of the level
+  };
+  finish(L);
+  if (twinned) finish(twin);
+  const uint64_t b = first + threadIdx.x;
   if (b >= nreal) return;
-  const uint64_t ones_before = l1_value(intra, cta_off, nreal, b);
-  L.l12[2 * b] = uint32_t(ones_before);
-  if (b == 0 && n12 > nreal) { L.l12[2 * nreal] = 0; L.l12[2 * nreal + 1] = 0; }
+  const uint64_t ones_before = level_before + before_warp + x - v, ones_through = ones_before + v;
+  const uint32_t fields = (l2[0] & 1023u) | ((l2[1] & 1023u) << 10) | ((l2[2] & 1023u) << 20);
+  auto entry = [&](const RankSelectLevel& R) {
+    R.l12[2 * b] = uint32_t(ones_before);
+    R.l12[2 * b + 1] = fields;
+  };
+  entry(L);
+  if (twinned) entry(twin);
   if (b + 1 >= n12) return;  // pwm examines blocks 0 .. n12-2
-  const uint64_t ones_through = l1_value(intra, cta_off, nreal, b + 1);
   // sample s is taken in the first block whose running count exceeds
-  // 1 + 8192 s (bin_select_popcnt.hpp:55-99)
+  // 1 + 8192 s (bin_select_popcnt.hpp:55-99); pwm's count before the entry
+  // that follows the last real block is 0
+  const uint64_t through = b + 1 < nreal ? ones_through : 0;
   const uint64_t s1 = ones_before == 0 ? 0 : (ones_before - 1 + kSampleRate - 1) / kSampleRate;
   const uint64_t next1 = 1 + kSampleRate * s1;
-  const bool need1 = ones_through > next1;
   const uint64_t f_prev = b * kL1Bits - ones_before;
-  const uint64_t f_here = (b + 1) * kL1Bits - ones_through;
+  const uint64_t f_here = (b + 1) * kL1Bits - through;
   const uint64_t s0 = f_prev == 0 ? 0 : (f_prev - 1 + kSampleRate - 1) / kSampleRate;
   const uint64_t next0 = 1 + kSampleRate * s0;
-  const bool need0 = f_here > next0;
-  bool got1 = false, got0 = false;
   uint64_t pos;
-  if (need1 && thread_block_select(L.data, L.nwords, L.l12, b, 1, uint32_t(next1 - ones_before), &pos)) {
-    L.s1[s1] = uint32_t(pos);
-    got1 = true;
-  }
-  if (need0 && thread_block_select(L.data, L.nwords, L.l12, b, 0, uint32_t(next0 - f_prev), &pos)) {
-    L.s0[s0] = uint32_t(pos);
-    got0 = true;
-  }
+  auto sample = [&](int value, uint64_t s, uint64_t rem) -> uint32_t {
+    if (!thread_block_select(L.data, L.nwords, fields, b, value, uint32_t(rem), &pos)) return 0;
+    (value ? L.s1 : L.s0)[s] = uint32_t(pos);
+    if (twinned) (value ? twin.s1 : twin.s0)[s] = uint32_t(pos);
+    return 1;
+  };
+  const uint32_t got1 = through > next1 ? sample(1, s1, next1 - ones_before) : 0u;
+  const uint32_t got0 = f_here > next0 ? sample(0, s0, next0 - f_prev) : 0u;
   // samples are taken in block order, so the count is fixed by the last
   // block pwm examines (n12 - 2): the samples before it plus its own
   if (b == n12 - 2) {
-    L.meta[1] = s1 + (got1 ? 1 : 0);
-    L.meta[0] = s0 + (got0 ? 1 : 0);
+    L.meta[1] = s1 + got1;
+    L.meta[0] = s0 + got0;
+    if (twinned) {
+      twin.meta[1] = s1 + got1;
+      twin.meta[0] = s0 + got0;
+    }
   }
 }
 
@@ -711,23 +741,18 @@ void launch_huff_queries(const QueryStructure& q, const HuffQueryTables& h, int 
   ++*launches;
 }
 
-void launch_rank_select(const RankSelectLevel* host_levels, uint32_t count, RankSelectLevel* dev_levels,
-                        uint32_t* tmp, uint64_t tmp_words_per_level, cudaStream_t s, uint64_t* launches) {
-  if (count == 0) return;
-  uint64_t max_real = 0;
-  for (uint32_t i = 0; i < count; ++i) {
-    uint64_t nreal = (host_levels[i].nwords + kL1Cover - 1) / kL1Cover;
-    if (nreal > max_real) max_real = nreal;
-  }
-  if (max_real == 0) return;
-  const uint64_t ctas = (max_real + kRsThreads - 1) / kRsThreads;
-  dim3 g1(unsigned(ctas), count);
-  rs_blocks_kernel<<<g1, kRsThreads, 0, s>>>(dev_levels, tmp, tmp_words_per_level);
-  rs_scan_kernel<<<count, 1024, 0, s>>>(dev_levels, tmp, tmp_words_per_level);
-  rs_finish_kernel<<<g1, kRsThreads, 0, s>>>(dev_levels, tmp, tmp_words_per_level);
-  *launches += 3;
+uint64_t rank_select_state_words(uint64_t max_words) {
+  const uint64_t nreal = (max_words + kL1Cover - 1) / kL1Cover;
+  return 1 + std::max<uint64_t>(1, (nreal + kRsThreads - 1) / kRsThreads);
 }
 
+void launch_rank_select(const RankSelectArgs& a, uint64_t max_words, cudaStream_t s, uint64_t* launches) {
+  const uint32_t levels = a.nfirst + a.nsecond;
+  if (levels == 0) return;
+  const dim3 grid(levels, unsigned(rank_select_state_words(max_words) - 1));  // at most 8192 CTAs a level (2^32 bits)
+  rank_select_kernel<<<grid, kRsThreads, 0, s>>>(a);
+  ++*launches;
+}
 
 // ===========================================================================
 // Allocation-free rank/select build (pwmgpu_rank_select_build_noalloc).
@@ -735,42 +760,34 @@ void launch_rank_select(const RankSelectLevel* host_levels, uint32_t count, Rank
 // For callers that must not allocate device memory while they run:
 // allocator-less plugins that receive every buffer from their host framework,
 // and latency-critical serving loops that cannot afford an allocator's
-// implicit synchronisation.  The per-L1-block prefix counts the build needs
-// live in a fixed, file-scope device array instead of context scratch, and
-// the level descriptor the kernels read lives in a file-scope device slot.
-// Both are resident on every GPU that loads this library until the process
-// exits.  Every call shares them: calls that overlap on the GPU (different
-// streams, or different host threads on one device) race and must be
-// serialised by the caller.
+// implicit synchronisation.  The look-back state of the build lives in a
+// fixed, file-scope device array instead of context scratch, resident on every
+// GPU that loads this library until the process exits; the level descriptor
+// travels as a kernel parameter.  Every call shares the array: calls that
+// overlap on the GPU (different streams, or different host threads on one
+// device) race and must be serialised by the caller.
 // ===========================================================================
 namespace {
 
-// 4 MiB: prefix counts for up to kNoAllocMaxL1Blocks L1 blocks plus their
-// per-CTA totals.
+// 4 MiB: a status word, then the look-back state.  The level limit is the
+// entry point's published one.
 constexpr uint64_t kNoAllocScratchWords = uint64_t(1) << 20;
 constexpr uint64_t kNoAllocMaxL1Blocks = (uint64_t(1) << 20) - (uint64_t(1) << 12);
 
 static __device__ __align__(256) uint32_t g_noalloc_rs_scratch[kNoAllocScratchWords];
-static __device__ __align__(256) RankSelectLevel g_noalloc_rs_level[1];
-
-// Stores the level descriptor into its file-scope slot in stream order: the
-// values travel as a kernel parameter, so no host buffer has to outlive the
-// call.
-__global__ void noalloc_set_level_kernel(RankSelectLevel level) { g_noalloc_rs_level[0] = level; }
 
 struct NoAllocSymbols {
   bool ready = false;
   uint32_t* scratch = nullptr;
-  RankSelectLevel* level = nullptr;
 };
 
 }  // namespace
 
-// Device addresses of the file-scope arrays for the current device, looked
+// Device address of the file-scope array for the current device, looked
 // up once per device (the first call on a device does it) and kept for the
 // life of the process: after a cudaDeviceReset the module may load at other
 // addresses, so the entry point must not be used across a device reset.
-cudaError_t noalloc_rank_select_symbols(uint32_t** scratch, RankSelectLevel** level) {
+cudaError_t noalloc_rank_select_symbols(uint32_t** scratch) {
   static std::mutex mu;
   static NoAllocSymbols per_device[64];
   int dev = 0;
@@ -784,27 +801,22 @@ cudaError_t noalloc_rank_select_symbols(uint32_t** scratch, RankSelectLevel** le
     e = cudaGetSymbolAddress(&p, g_noalloc_rs_scratch);
     if (e != cudaSuccess) return e;
     s.scratch = static_cast<uint32_t*>(p);
-    e = cudaGetSymbolAddress(&p, g_noalloc_rs_level);
-    if (e != cudaSuccess) return e;
-    s.level = static_cast<RankSelectLevel*>(p);
     s.ready = true;
   }
   *scratch = s.scratch;
-  *level = s.level;
   return cudaSuccess;
 }
 
 uint64_t noalloc_rank_select_max_words() { return kNoAllocMaxL1Blocks * kL1Cover; }
 
 // Enqueues the build of one level's blocks on `stream` using only the
-// file-scope arrays; outputs that must start at zero (l0, counts) are cleared
+// file-scope array; outputs that must start at zero (l0, counts) are cleared
 // here.  Returns cudaErrorInvalidValue for levels above the limit.
 cudaError_t noalloc_rank_select_build(const uint64_t* words, uint64_t nwords, uint64_t* l0, uint32_t* l12,
                                       uint32_t* s0, uint32_t* s1, unsigned long long* counts, cudaStream_t stream) {
   if (nwords > noalloc_rank_select_max_words()) return cudaErrorInvalidValue;
   uint32_t* scratch = nullptr;
-  RankSelectLevel* dev_level = nullptr;
-  cudaError_t e = noalloc_rank_select_symbols(&scratch, &dev_level);
+  cudaError_t e = noalloc_rank_select_symbols(&scratch);
   if (e != cudaSuccess) return e;
   const uint64_t n0 = nwords / (4294967295ull / 64) + 1;
   e = cudaMemsetAsync(l0, 0, n0 * 8, stream);
@@ -816,12 +828,17 @@ cudaError_t noalloc_rank_select_build(const uint64_t* words, uint64_t nwords, ui
     e = cudaMemsetAsync(l12, 0, 2 * sizeof(uint32_t), stream);
     return e;
   }
-  RankSelectLevel host{words, nwords, l0, l12, s0, s1, counts};
-  noalloc_set_level_kernel<<<1, 1, 0, stream>>>(host);
-  const uint64_t nreal = (nwords + kL1Cover - 1) / kL1Cover;
-  const uint64_t stride = nreal + (nreal + kRsThreads - 1) / kRsThreads + 1;
+  RankSelectArgs a{};
+  a.one = RankSelectLevel{words, nwords, l0, l12, s0, s1, counts};
+  a.nfirst = 1;
+  a.stride = rank_select_state_words(nwords);
+  a.status = scratch;
+  a.state = reinterpret_cast<unsigned long long*>(scratch + 2);
+  a.spin_limit = kSpinLimit;
+  e = cudaMemsetAsync(scratch, 0, 8 + a.stride * 8, stream);
+  if (e != cudaSuccess) return e;
   uint64_t launches = 0;
-  launch_rank_select(&host, 1, dev_level, scratch, stride, stream, &launches);
+  launch_rank_select(a, nwords, stream, &launches);
   return cudaGetLastError();
 }
 
