@@ -41,8 +41,8 @@ pwmgpu_status pwmgpu_ctx_create(int device, void* cuda_stream, pwmgpu_ctx** out)
       CUDA_TRY(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
       ctx->own_stream = true;
     }
-    CUDA_TRY(cudaMalloc(&ctx->d_status, 64));
-    CUDA_TRY(cudaMemset(ctx->d_status, 0, 64));
+    CUDA_TRY(cudaMalloc(&ctx->d_status, kStatusBytes));
+    CUDA_TRY(cudaMemset(ctx->d_status, 0, kStatusBytes));
     // a kernel of this library must be loadable on this device
     cudaFuncAttributes attr;
     cudaError_t e = cudaFuncGetAttributes(&attr, reinterpret_cast<const void*>(&pwmgpu_ctx_create));

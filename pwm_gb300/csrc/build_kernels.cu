@@ -245,7 +245,9 @@ __global__ void __launch_bounds__(kTileHistThreads) tile_hist_kernel(const T* te
 //    runs in natural prefix order, runs of S_K; tree entries 0 without a
 //    tree.  A key_j run is a contiguous range of bins (those with the same
 //    j-bit prefix), so its count is a difference of the bins' prefix sums,
-//    and the tree's starts are those prefix sums themselves.
+//    and the tree's starts are those prefix sums themselves.  For a text
+//    built in one pass it also writes the rest that follows from the
+//    histogram (TileOnePass), so that the host plans nothing.
 template <int W>
 __device__ __forceinline__ unsigned long long block_exclusive_scan(unsigned long long v, unsigned long long* wsum,
                                                                    unsigned long long* total) {
@@ -275,7 +277,7 @@ __device__ __forceinline__ unsigned long long block_exclusive_scan(unsigned long
 __global__ void __launch_bounds__(1024) tile_block_scan_kernel(unsigned long long* blocksum, uint32_t nblocks,
                                                                uint32_t NB, const unsigned long long* hist,
                                                                uint32_t levels, uint32_t K, uint32_t out,
-                                                               uint32_t tree, uint64_t* table) {
+                                                               uint32_t tree, uint64_t* table, TileOnePass one) {
   __shared__ unsigned long long wsum[32];
   const uint32_t tid = threadIdx.x;
   if (blockIdx.x < NB) {
@@ -317,7 +319,25 @@ __global__ void __launch_bounds__(1024) tile_block_scan_kernel(unsigned long lon
   const unsigned long long ex = block_exclusive_scan<32>(cnt, wsum, &total);
   if (tid < bins) P[tid] = ex;
   if (tid == 0) P[bins] = total;
+  if (one.d_seg && tid == 0) {
+    *one.d_seg = one.seg;
+    *one.d_text = one.text;
+    if (one.host) one.host[levels] = *one.status;
+  }
   __syncthreads();
+  if (one.d_seg && tid >= 512 && tid < 512 + 32 * levels) {
+    // zeros of level l: the symbols whose bit of that level is 0, its bins in runs of 2^(levels - 1 - l)
+    const uint32_t l = (tid >> 5) - 16, lane = tid & 31, run = levels - 1 - l;
+    unsigned long long z = 0;
+    for (uint32_t p = lane; p < (1u << l); p += 32) z += P[(2 * p + 1) << run] - P[(2 * p) << run];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) z += __shfl_xor_sync(0xFFFFFFFFu, z, d);
+    if (lane == 0) {
+      one.d_zeros[l] = z;
+      one.host[l] = z;
+    }
+    return;
+  }
   // warp j: level j (j < K: matrix and tree starts; j == K: runs of S_K)
   const uint32_t warp = tid >> 5, lane = tid & 31;
   if (warp > K || (warp == K && !out)) return;
@@ -346,8 +366,9 @@ __global__ void __launch_bounds__(1024) tile_block_scan_kernel(unsigned long lon
     const uint32_t x = 8 * lane + q;
     if (x < R) {
       if (j < K) {
+        const unsigned long long nat = P[reverse_low_bits(x, j) << sh];
         table[tile_wm_entry(int(j), int(x))] = run;
-        table[tile_wt_entry(int(K), int(j), int(x))] = tree ? P[reverse_low_bits(x, j) << sh] : 0ull;
+        table[tile_wt_entry(int(K), int(j), int(x))] = tree ? nat : 0ull;
       } else {
         table[tile_out_entry(int(K), int(x))] = run;
       }
@@ -1068,12 +1089,11 @@ uint32_t tile_hist_blocks(uint64_t n, uint32_t tile_keys) {
 }
 
 void launch_tile_histogram_blocks(const void* text, uint64_t n, uint32_t width, uint32_t levels, uint32_t D,
-                                  uint32_t tile_keys, uint32_t block0, uint32_t nblk, unsigned long long* hist,
-                                  uint32_t* tilecnt, uint32_t* relpre, unsigned long long* blocksum,
+                                  uint32_t tile_keys, uint32_t per, uint32_t block0, uint32_t nblk,
+                                  unsigned long long* hist, uint32_t* tilecnt, uint32_t* relpre, unsigned long long* blocksum,
                                   uint64_t* level0_a, uint64_t* level0_b, uint32_t* status, cudaStream_t s,
                                   uint64_t* launches) {
   if (n == 0 || nblk == 0) return;
-  const uint32_t per = tile_hist_tiles_per_block();
 #define PWMGPU_TH(T, B8)                                                                                       \
   tile_hist_kernel<T, B8><<<nblk, kTileHistThreads, 0, s>>>(static_cast<const T*>(text), n, levels, D, tile_keys, \
                                                             per, block0, hist, tilecnt, relpre, blocksum,       \
@@ -1088,10 +1108,11 @@ void launch_tile_histogram_blocks(const void* text, uint64_t n, uint32_t width, 
 
 void launch_tile_block_scan(unsigned long long* blocksum, uint32_t nblocks, uint32_t D, const unsigned long long* hist,
                             uint32_t levels, uint32_t K, bool out, bool tree, uint64_t* table, cudaStream_t s,
-                            uint64_t* launches) {
+                            uint64_t* launches, const TileOnePass* one) {
   if (nblocks == 0) return;
   tile_block_scan_kernel<<<(1u << D) + (table ? 1u : 0u), 1024, 0, s>>>(blocksum, nblocks, 1u << D, hist, levels, K,
-                                                                        out ? 1u : 0u, tree ? 1u : 0u, table);
+                                                                        out ? 1u : 0u, tree ? 1u : 0u, table,
+                                                                        one ? *one : TileOnePass{});
   ++*launches;
 }
 

@@ -111,10 +111,11 @@ void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint
 // level 0 is the same bit vector: counted once, written to both.
 //
 // Levels [lo, hi) only, on `stream` (default: the context's) with a scratch
-// buffer named after `tag` (so that two groups can run at once); only the
+// buffer named after `tag` (so that two groups can run at once), or the
+// caller's zeroed words (rank_select_state_words for every level); only the
 // context's stream is profiled.
 void build_rank_select(pwmgpu_ctx* ctx, Structure* wm, Structure* wt, bool share_level0, uint32_t lo, uint32_t hi,
-                       cudaStream_t stream, const char* tag) {
+                       cudaStream_t stream, const char* tag, unsigned long long* zeroed_state) {
   uint64_t max_words = 0, bytes = 0;
   auto take = [&](const Structure* st, uint32_t from, uint32_t* first) -> uint32_t {
     if (!st || !st->rs) return 0;
@@ -137,10 +138,13 @@ void build_rank_select(pwmgpu_ctx* ctx, Structure* wm, Structure* wt, bool share
   cudaStream_t s = stream ? stream : ctx->stream;
   a.stride = rank_select_state_words(max_words);
   const uint64_t state_bytes = a.stride * (a.nfirst + a.nsecond) * 8;
-  a.state = static_cast<unsigned long long*>(ctx->grow("rs_state" + std::string(tag), state_bytes));
   a.status = ctx->d_status;
   a.spin_limit = kSpinLimit;
-  CUDA_TRY(cudaMemsetAsync(a.state, 0, state_bytes, s));
+  a.state = zeroed_state;
+  if (!a.state) {
+    a.state = static_cast<unsigned long long*>(ctx->grow("rs_state" + std::string(tag), state_bytes));
+    CUDA_TRY(cudaMemsetAsync(a.state, 0, state_bytes, s));
+  }
   if (s == ctx->stream) {
     ProfScope ps(ctx, "rank_select", bytes);
     launch_rank_select(a, max_words, s, &ctx->launches);

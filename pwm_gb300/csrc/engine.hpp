@@ -37,6 +37,7 @@ constexpr uint32_t kSinglePassMaxLevels = 7;  // one tile pass for texts of at m
 constexpr uint32_t kMaxStreamChunks = 16;  // chunks of a pass whose finished words stream to pinned outputs
 constexpr uint64_t kAlphabetMaxSymbol = uint64_t(1) << 24;  // 32-bit alphabet reduction: one bin per value below
 constexpr uint64_t kAlphabetHashMaxSymbols = uint64_t(1) << 30;  // wider symbols: through a hash table
+constexpr uint64_t kStatusBytes = 16384;  // a context's status word and the words zeroed with it
 constexpr uint64_t kStagePiece = uint64_t(16) << 20;  // bytes of one pinned staging piece
 constexpr unsigned kStagePieces = 4;                  // pieces in the staging ring
 constexpr unsigned kStageAutoThreads = 8;             // host copy threads by default (at most)
@@ -77,6 +78,7 @@ struct pwmgpu_ctx {
   bool own_stream = false;
   std::string err;
   uint64_t launches = 0;
+  // the status word; behind it the words a one-pass build zeroes with it (kStatusBytes in all)
   uint32_t* d_status = nullptr;
   std::map<std::string, DevBuf> scratch;
   int pass_levels = kDefaultPassLevels;
@@ -400,7 +402,8 @@ void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint
 // copy of the matrix's.  Levels [lo, hi) only, on `stream` (default: the
 // context's) with scratch buffers named after `tag`.
 void build_rank_select(pwmgpu_ctx* ctx, Structure* wm, Structure* wt = nullptr, bool share_level0 = false,
-                       uint32_t lo = 0, uint32_t hi = ~0u, cudaStream_t stream = nullptr, const char* tag = "");
+                       uint32_t lo = 0, uint32_t hi = ~0u, cudaStream_t stream = nullptr, const char* tag = "",
+                       unsigned long long* zeroed_state = nullptr);
 uint32_t read_status(pwmgpu_ctx* ctx);
 void throw_status(uint32_t st);
 void check_device_status(pwmgpu_ctx* ctx);

@@ -74,17 +74,31 @@ void launch_first_positions(const void* text, uint64_t n, uint32_t width, uint64
 void launch_remap(const void* text, uint64_t n, uint32_t width, const uint32_t* map, uint64_t nmap, void* out,
                   uint32_t* status, cudaStream_t s, uint64_t* launches);
 uint32_t tile_hist_blocks(uint64_t n, uint32_t tile_keys);
+// per: the tiles of a block (tile_hist_tiles_per_block(), or fewer).
 void launch_tile_histogram_blocks(const void* text, uint64_t n, uint32_t width, uint32_t levels, uint32_t D,
-                                  uint32_t tile_keys, uint32_t block0, uint32_t nblk, unsigned long long* hist,
+                                  uint32_t tile_keys, uint32_t per, uint32_t block0, uint32_t nblk,
+                                  unsigned long long* hist,
                                   uint32_t* tilecnt, uint32_t* relpre, unsigned long long* blocksum,
                                   uint64_t* level0_a, uint64_t* level0_b, uint32_t* status, cudaStream_t s,
                                   uint64_t* launches);
 // With `table` set, the same launch also writes the start table
 // (tile_table_size(K) entries) of the first tile pass of the text (levels <=
-// 8, one segment) from its leaf histogram.
+// 8, one segment) from its leaf histogram.  With `one` set (a text whose only
+// pass this is, K == levels; d_seg set) it writes everything else the build needs from
+// the histogram: the pass's descriptors, the zero bits of every level for the
+// device and, with the status word, for the host.
+struct TileOnePass {
+  TileSeg seg;              // written to *d_seg, text to *d_text
+  TileText text;
+  TileSeg* d_seg;
+  TileText* d_text;
+  uint64_t* d_zeros;        // zeros of every level
+  uint64_t* host;           // mapped: the same, then the status word
+  const uint32_t* status;
+};
 void launch_tile_block_scan(unsigned long long* blocksum, uint32_t nblocks, uint32_t D, const unsigned long long* hist,
                             uint32_t levels, uint32_t K, bool out, bool tree, uint64_t* table, cudaStream_t s,
-                            uint64_t* launches);
+                            uint64_t* launches, const TileOnePass* one = nullptr);
 // The start table of the first tile pass of a text of any level count (one
 // segment: the whole text) from the natural prefix counts of its levels 0..K
 // (`flat`: level m at offset 2^m - 1, as launch_fold_levels writes them), so
@@ -141,6 +155,9 @@ void launch_split_pass_batched(uint32_t key_bytes, int K, const SplitArgs* args,
 // ---- segmented tile passes (plain keys, matrix and tree together) ------------
 // Keys of one tile for a key width.
 uint32_t tile_pass_elems(uint32_t key_bytes);
+// The same of the half-size tiles of a one-pass text of 1-byte keys
+// (TileArgs::half_tiles).
+uint32_t tile_pass_half_elems();
 // One pass of K levels over a.tiles tiles; `out`: the pass writes S_{l+K}.
 // Digit counts of the passes of a matrix-only build (pass_digits_kernel):
 // pass p covers levels level[p]..level[p]+K[p]-1, its natural digit is

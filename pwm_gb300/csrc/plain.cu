@@ -210,6 +210,120 @@ void validate_plain(uint64_t n, uint32_t width, uint32_t levels, bool allow40) {
   if (n >= (uint64_t(1) << 62)) throw Fail{PWMGPU_ERR_ARG, "size too large"};
 }
 
+namespace {
+
+// A text of at most 8 levels whose levels all come from one tile pass: every
+// table follows from the leaf histogram on the device (launch_tile_block_scan
+// with TileOnePass), so the host enqueues the whole build (one memset, the
+// histogram, the tables, the pass, rank/select) and then waits for the zeros
+// and the status word.
+//
+// Measured (GB300), both structures with rank/select and 3 x 10^4 queries:
+// 10^6 bytes, 8 levels 189 -> 94 us a build, 4099 bytes 160 -> 81; 2^26
+// DNA-like bytes, 2 levels, without queries 102 -> 86.
+//
+// Short texts take half-size tiles and histogram blocks of one tile, so that
+// more SMs work: both structures of 2^20 bytes take 36 us at 8 levels against
+// 46 with whole tiles (3 levels 19 and 22), 2^21 bytes 41 and 46, 2^22 57 and
+// 52.
+constexpr uint64_t kHalfTileMax = uint64_t(1) << 21;  // symbols
+// 8 levels of bytes in one pass: its tiles cost more than two 4-level passes
+// (127 runs at the deepest level), but a text saves the second pass, the
+// host's plan of it and the regroup.  One pass against two: both structures
+// 36 and 86 us at 2^20 bytes, 131 and 160 at 2^24, 236 and 233 at 2^25, 432
+// and 388 at 2^26; the matrix alone 207 and 235 at 2^25, 368 and 361 at 2^26.
+constexpr uint64_t kOnePass8Tree = uint64_t(30) << 20;    // symbols, with a tree
+constexpr uint64_t kOnePass8Matrix = uint64_t(60) << 20;  // a matrix alone
+
+void build_one_pass(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text) {
+  cudaStream_t s = ctx->stream;
+  const uint32_t L = wx->levels, w = wx->width;
+  const uint64_t n = wx->n;
+  const bool tree = wx->wt.present;
+  const bool half = w == 1 && n <= kHalfTileMax;
+  const uint32_t T = half ? tile_pass_half_elems() : tile_pass_elems(w);
+  const uint32_t tiles = uint32_t((n + T - 1) / T);
+  const uint32_t per = tiles <= 2 * 152 ? 1u : std::min(tile_hist_tiles_per_block(), tiles / 152);
+  const uint32_t nblocks = (tiles + per - 1) / per, D = L - 1;
+  const uint64_t NB = uint64_t(1) << D;
+  // zeroed with the status word: the histogram, the pass's tile counter and,
+  // where it fits, the look-back state of rank/select
+  auto* words = reinterpret_cast<unsigned char*>(ctx->d_status);
+  auto* d_hist = reinterpret_cast<unsigned long long*>(words + 64);
+  auto* counter = reinterpret_cast<uint32_t*>(words + 64 + 2048);
+  constexpr uint64_t kState = 64 + 2048 + 64;
+  Structure* rs_wm = wx->wm.rs && !wx->wm_internal ? &wx->wm : nullptr;
+  Structure* rs_wt = tree && wx->wt.rs ? &wx->wt : nullptr;
+  const uint64_t rs_bytes =
+      (rs_wm || rs_wt) ? 8 * rank_select_state_words(words_for(n)) * L * ((rs_wm ? 1 : 0) + (rs_wt ? 1 : 0)) : 0;
+  const bool rs_fits = kState + rs_bytes <= kStatusBytes;
+  CUDA_TRY(cudaMemsetAsync(words, 0, kState + (rs_fits ? rs_bytes : 0), s));
+  // the tables: counts and prefixes of every tile, the block prefixes, the start table and descriptors
+  const uint64_t counts = uint64_t(tiles) * NB * 8, pre = (counts + 255) & ~uint64_t(255);
+  const uint64_t desc = (pre + nblocks * NB * 8 + 255) & ~uint64_t(255);
+  auto* base = static_cast<unsigned char*>(ctx->grow("tile_first", desc + 256 + size_t(tile_table_size(int(L))) * 8));
+  auto* tilecnt = reinterpret_cast<uint32_t*>(base);
+  auto* relpre = tilecnt + uint64_t(tiles) * NB;
+  auto* blockpre = reinterpret_cast<unsigned long long*>(base + pre);
+  auto* table = reinterpret_cast<uint64_t*>(base + desc + 256);
+  uint64_t* h = ctx->grow_mapped((L + 1) * 8);
+  uint64_t* l0[2] = {wx->wm.d_words, tree ? wx->wt.d_words : nullptr};
+  {
+    ProfScope ps(ctx, "leaf_histogram", n * w + (l0[1] ? 2 : 1) * words_for(n) * 8);
+    launch_tile_histogram_blocks(d_text, n, w, L, D, T, per, 0, nblocks, d_hist, tilecnt, relpre, blockpre, l0[0], l0[1],
+                                 ctx->d_status, s, &ctx->launches);
+  }
+  TileOnePass one{};
+  one.seg = TileSeg{0, n, 0, 0, 0};
+  one.text.wm = wx->wm.d_words;
+  one.text.wt = tree ? wx->wt.d_words : nullptr;
+  one.text.stride = wx->wm.offs[1] - wx->wm.offs[0];
+  one.text.nbits = n;
+  one.text.shift = L - 1;
+  one.d_seg = reinterpret_cast<TileSeg*>(base + desc);
+  one.d_text = reinterpret_cast<TileText*>(base + desc + 128);
+  one.d_zeros = wx->wm.d_zeros;
+  one.host = ctx->mapped_dev;
+  one.status = ctx->d_status;
+  launch_tile_block_scan(blockpre, nblocks, D, d_hist, L, L, false, tree, table, s, &ctx->launches, &one);
+  CUDA_TRY(cudaEventRecord(ctx->hist_event(), s));
+  TileArgs a{};
+  a.in = d_text;
+  a.segs = one.d_seg;
+  a.texts = one.d_text;
+  a.tables = table;
+  a.tile_counter = counter;
+  a.status = ctx->d_status;
+  a.nsegs = 1;
+  a.tiles = tiles;
+  a.launch_tiles = tiles;
+  a.blockpre = blockpre;
+  a.relpre = relpre;
+  a.tilecnt = tilecnt;
+  a.tiles_per_block = per;
+  a.first_level_written = 1u;
+  a.clear_edges = 1u;
+  a.half_tiles = half ? 1u : 0u;
+  a.spin_limit = ctx->spin_limit;
+  const uint64_t structs = one.text.wt ? 2 : 1;
+  {
+    ProfScope ps(ctx, "split_pass", structs * (L * (n * w + words_for(n) * 8) - words_for(n) * 8));
+    launch_tile_pass(w, w, int(L), false, a, s, &ctx->launches);
+  }
+  build_rank_select(ctx, rs_wm, rs_wt, true, 0, ~0u, nullptr, "",
+                    rs_fits ? reinterpret_cast<unsigned long long*>(words + kState) : nullptr);
+  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(cudaEventSynchronize(ctx->hist_event()));
+  const uint32_t status = uint32_t(h[L]);
+  if (status) {
+    CUDA_TRY(cudaStreamSynchronize(s));  // the pass may still read the text
+    throw_status(status);
+  }
+  wx->wm.zeros.assign(h, h + L);
+}
+
+}  // namespace
+
 // Plain build of a wx from a device text (with `io`: from a host text, into
 // host arrays; d_text is then the device copy to fill).
 void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostIO* io) {
@@ -242,6 +356,20 @@ void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostI
     }
   } drain{ctx, pinned_in || stream_out};
   if (io && io->text && !pinned_in) host_to_device(ctx, const_cast<void*>(d_text), io->text, n * wx->width, s);
+  // (the withheld-tile hook is about look-backs, which one pass has none of)
+  const bool short_piece = pinned_in && n * wx->width <= ctx->upload_piece;  // nothing to overlap
+  if (ctx->engine == PWMGPU_ENGINE_TILE && ctx->tile_levels == 0 && L >= 2 && !wx->keep_hist && !stream_out &&
+      (!pinned_in || short_piece) && !ctx->withhold_first_tile &&
+      (L <= kSinglePassMaxLevels ||
+       (L == 8 && wx->width == 1 && n <= (wx->wt.present ? kOnePass8Tree : kOnePass8Matrix)))) {
+    if (pinned_in) CUDA_TRY(cudaMemcpyAsync(const_cast<void*>(d_text), io->text, n * wx->width, cudaMemcpyHostToDevice, s));
+    build_one_pass(ctx, wx, d_text);
+    for (int st = 0; st < 2; ++st) {
+      const Structure& S = st ? wx->wt : wx->wm;
+      if (host_out[st] && S.present) device_to_host(ctx, host_out[st], S.d_words, S.total_words * 8, s);
+    }
+    return;
+  }
   CUDA_TRY(cudaMemsetAsync(ctx->d_status, 0, 4, s));
   const uint64_t bins = uint64_t(1) << L;
   // Tile engine: level 0 is written in whole words (by the histogram kernel,
@@ -353,7 +481,7 @@ void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostI
                                  cudaMemcpyHostToDevice, ctx->up));
         CUDA_TRY(cudaStreamWaitEvent(s, ctx->mark(ctx->up), 0));
       }
-      launch_tile_histogram_blocks(d_text, n, wx->width, L, D0, T, b0, nb, d_hist,
+      launch_tile_histogram_blocks(d_text, n, wx->width, L, D0, T, per, b0, nb, d_hist,
                                    const_cast<uint32_t*>(first.tilecnt), const_cast<uint32_t*>(first.relpre),
                                    const_cast<unsigned long long*>(first.blockpre), l0[0], l0[1], ctx->d_status, s,
                                    &ctx->launches);

@@ -42,9 +42,9 @@ uint32_t tile_key_bytes(uint32_t bits) { return bits <= 8 ? 1u : (bits <= 16 ? 2
 void launch_tile_pass(uint32_t key_bytes, uint32_t out_bytes, int K, bool out, const TileArgs& a, cudaStream_t s,
                       uint64_t* launches) {
   if (a.launch_tiles == 0) return;
-  if (K > kTileMaxLevels) {
+  if (K > kTileMaxLevels || a.half_tiles) {
     // only as the last pass of a text whose prefixes the histogram gives
-    if (out || !a.blockpre || K > kTileGivenMaxLevels) return;
+    if (out || !a.blockpre || K > kTileGivenMaxLevels || (a.half_tiles && (key_bytes != 1 || K < 2))) return;
     launch_tile_pass_deep(key_bytes, K, a, s);
   } else if (key_bytes == 1) launch_key<uint8_t>(K, out, out_bytes, a, s);
   else if (key_bytes == 2) launch_key<uint16_t>(K, out, out_bytes, a, s);

@@ -100,6 +100,7 @@ struct TileArgs {
   // tile's index in its segment / tiles_per_block.
   uint32_t text_blocks;
   uint32_t first_level_written;  // level l is already written (by the histogram kernel)
+  uint32_t half_tiles;           // one-pass texts of 1-byte keys: tiles of half as many keys
   uint32_t clear_edges;          // the levels were not zeroed: shared words are cleared before they are set
   // Optional: words [0, zero_words) at zero_a (and zero_b) are zeroed, tile g
   // taking words [g * zero_per_tile, (g + 1) * zero_per_tile): the levels of

@@ -10,10 +10,10 @@ constexpr int kTileThreads = 256;
 constexpr int kTileVectors = 4;  // 16-byte vectors per thread: 64 bytes of keys
 
 // PLANES: the bit-plane form of a pass without S_{l+K} over 1-byte keys.
-template <typename KeyT, int K, bool OUT, typename KeyO = KeyT, bool PLANES = false>
+template <typename KeyT, int K, bool OUT, typename KeyO = KeyT, bool PLANES = false, int V = kTileVectors>
 void launch_tile_one(const TileArgs& a, cudaStream_t s) {
-  using C = TileCfg<KeyT, K, OUT, kTileThreads, kTileVectors>;
-  auto kern = tile_pass_kernel<KeyT, K, OUT, kTileThreads, kTileVectors, KeyO, PLANES>;
+  using C = TileCfg<KeyT, K, OUT, kTileThreads, V>;
+  auto kern = tile_pass_kernel<KeyT, K, OUT, kTileThreads, V, KeyO, PLANES>;
   constexpr size_t smem = PLANES ? C::plane_smem_bytes() : C::smem_bytes();
   static bool configured = false;  // attribute set once per instantiation
   if (!configured) {
@@ -23,7 +23,8 @@ void launch_tile_one(const TileArgs& a, cudaStream_t s) {
   kern<<<a.launch_tiles, kTileThreads, smem, s>>>(a);
 }
 
-// Last passes of 5..8 levels with given prefixes (tile_deep.cu).
+// Last passes of 5..8 levels with given prefixes (tile_deep.cu); with
+// TileArgs::half_tiles, of 2..8 levels over 1-byte keys.
 void launch_tile_pass_deep(uint32_t key_bytes, int K, const TileArgs& a, cudaStream_t s);
 
 }  // namespace pwmgpu
