@@ -524,23 +524,43 @@ pwmgpu_status pwmgpu_wx_build_huffman(pwmgpu_ctx* ctx, const void* d_text, uint6
     wx->flags = shape_flags;
     wx->huffman = true;
     uint32_t L = 0;
+    SymbolCounts counts;
     if (code_len) {
       if (!code_word || num_codes == 0) throw Fail{PWMGPU_ERR_ARG, "code table incomplete"};
       wx->code_len.assign(code_len, code_len + num_codes);
       wx->code_word.assign(code_word, code_word + num_codes);
     } else {
       uint64_t max_symbol = 0;
-      HuffCodes h = huffman_codes_device(ctx, d_text, size, word_width, tree, &max_symbol);
-      wx->code_len = h.len;
-      wx->code_word = h.word;
+      HuffCodes h = huffman_codes_device(ctx, d_text, size, word_width, tree, &max_symbol, &counts);
+      wx->code_len = std::move(h.len);
+      wx->code_word = std::move(h.word);
       L = h.levels;
     }
     for (uint64_t c = 0; c < wx->code_len.size(); ++c) {
       if (wx->code_len[c] > 56) throw Fail{PWMGPU_ERR_ARG, "codes longer than 56 bits"};
       if (wx->code_len[c]) wx->code_word[c] &= (uint64_t(1) << wx->code_len[c]) - 1;
     }
+    // device tables for queries: codes per symbol, codes sorted by (length,
+    // word), level sizes; made and copied while the passes run
+    const uint64_t nsym = wx->code_len.size();
+    std::vector<std::pair<uint64_t, uint64_t>> dec;
+    auto query_tables = [&]() {
+      const Structure& S = tree ? wx->wt : wx->wm;
+      for (uint64_t c = 0; c < nsym; ++c)
+        if (wx->code_len[c]) dec.emplace_back((wx->code_len[c] << 56) | wx->code_word[c], c);
+      std::sort(dec.begin(), dec.end());
+      std::vector<uint64_t> blob;
+      blob.reserve(2 * nsym + 2 * dec.size() + S.levels);
+      blob.insert(blob.end(), wx->code_len.begin(), wx->code_len.end());
+      blob.insert(blob.end(), wx->code_word.begin(), wx->code_word.end());
+      for (const auto& d : dec) blob.push_back(d.first);
+      for (const auto& d : dec) blob.push_back(d.second);
+      blob.insert(blob.end(), S.bits.begin(), S.bits.end());
+      CUDA_TRY(cudaMalloc(&wx->d_huff, std::max<size_t>(blob.size(), 1) * 8));
+      CUDA_TRY(cudaMemcpy(wx->d_huff, blob.data(), blob.size() * 8, cudaMemcpyHostToDevice));
+    };
     build_huffman(ctx, d_text, size, word_width, tree, wx->code_len, wx->code_word, L, wx->wm,
-                  tree ? &wx->wt : nullptr, rs);
+                  tree ? &wx->wt : nullptr, rs, counts.device ? &counts : nullptr, query_tables);
     const Structure& S = tree ? wx->wt : wx->wm;
     wx->levels = S.levels;
     if (tree) {  // the matrix was only the tree's source
@@ -548,25 +568,9 @@ pwmgpu_status pwmgpu_wx_build_huffman(pwmgpu_ctx* ctx, const void* d_text, uint6
       wx->wm.present = false;
       wx->wm_internal = true;
     }
-    // device tables for queries: codes per symbol, codes sorted by (length, word), level sizes
-    const uint64_t nsym = wx->code_len.size();
-    std::vector<std::pair<uint64_t, uint64_t>> dec;
-    for (uint64_t c = 0; c < nsym; ++c)
-      if (wx->code_len[c]) dec.emplace_back((wx->code_len[c] << 56) | wx->code_word[c], c);
-    std::sort(dec.begin(), dec.end());
-    std::vector<uint64_t> blob;
-    blob.reserve(2 * nsym + 2 * dec.size() + S.levels);
-    blob.insert(blob.end(), wx->code_len.begin(), wx->code_len.end());
-    blob.insert(blob.end(), wx->code_word.begin(), wx->code_word.end());
-    for (const auto& d : dec) blob.push_back(d.first);
-    for (const auto& d : dec) blob.push_back(d.second);
-    blob.insert(blob.end(), S.bits.begin(), S.bits.end());
-    CUDA_TRY(cudaMalloc(&wx->d_huff, std::max<size_t>(blob.size(), 1) * 8));
-    CUDA_TRY(cudaMemcpyAsync(wx->d_huff, blob.data(), blob.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
     const uint64_t* d = wx->d_huff;
     wx->hq = HuffQueryTables{d, d + nsym, nsym, d + 2 * nsym, d + 2 * nsym + dec.size(), dec.size(),
                              d + 2 * nsym + 2 * dec.size()};
-    CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // the pageable table copy has been read
     *out = wx.release();
     return PWMGPU_OK;
   });
@@ -663,19 +667,21 @@ pwmgpu_status pwmgpu_compute_huffman(pwmgpu_ctx* ctx, const void* text, uint64_t
     host_to_device(ctx, d_text, text, size * word_width, ctx->stream);
     std::vector<uint64_t> len, word;
     uint32_t L = levels;
+    SymbolCounts counts;
     if (code_len) {
       if (!code_word || num_codes == 0) throw Fail{PWMGPU_ERR_ARG, "code table incomplete"};
       len.assign(code_len, code_len + num_codes);
       word.assign(code_word, code_word + num_codes);
     } else {
       uint64_t max_symbol = 0;
-      HuffCodes h = huffman_codes_device(ctx, d_text, size, word_width, is_tree != 0, &max_symbol);
-      len = h.len;
-      word = h.word;
+      HuffCodes h = huffman_codes_device(ctx, d_text, size, word_width, is_tree != 0, &max_symbol, &counts);
+      len = std::move(h.len);
+      word = std::move(h.word);
       L = h.levels;
     }
     Structure wm, wt;
-    build_huffman(ctx, d_text, size, word_width, is_tree != 0, len, word, L, wm, is_tree ? &wt : nullptr, false);
+    build_huffman(ctx, d_text, size, word_width, is_tree != 0, len, word, L, wm, is_tree ? &wt : nullptr, false,
+                  counts.device ? &counts : nullptr);
     const Structure& s = is_tree ? wt : wm;
     if (level_sizes)
       for (uint32_t l = 0; l < L; ++l)

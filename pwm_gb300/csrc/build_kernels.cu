@@ -752,27 +752,6 @@ __global__ void __launch_bounds__(kSegThreads) regroup_seg_write_kernel(const ui
   }
 }
 
-// ---------------------------------------------------------------------------
-// Huffman code keys
-// ---------------------------------------------------------------------------
-// Key of symbol c with code (word, len), L the longest code: the code
-// followed by a stop bit, ((word << 1) | 1) << (L - len), in L + 1 <= 8 *
-// sizeof(K) bits (split.cuh HuffKeys).
-template <typename T, typename K>
-__global__ void huffman_keys_kernel(const T* text, uint64_t n, const uint64_t* code_len, const uint64_t* code_word,
-                                    uint64_t ncodes, uint32_t L, K* keys, uint32_t* status) {
-  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
-    uint64_t c = uint64_t(text[i]);
-    uint64_t len = c < ncodes ? code_len[c] : 0;
-    if (len == 0 || len > L) {
-      atomicOr(status, kErrSymbol);
-      keys[i] = K(0);
-      continue;
-    }
-    keys[i] = K(((uint64_t(code_word[c]) << 1) | 1u) << (L - len));
-  }
-}
-
 template <typename T>
 __global__ void symbol_hist_kernel(const T* text, uint64_t n, uint64_t nsym, unsigned long long* hist) {
   for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x) {
@@ -1207,36 +1186,6 @@ bool launch_regroup_segs(const uint64_t* flat, const uint32_t* levels, uint32_t 
   regroup_seg_write_kernel<<<unsigned(blocks), kSegThreads, 0, s>>>(flat, p, scratch, out);
   *launches += 3;
   return true;
-}
-
-template <typename T, typename K>
-void launch_hk(const void* text, uint64_t n, const uint64_t* code_len, const uint64_t* code_word, uint64_t ncodes,
-               uint32_t L, void* keys, uint32_t* status, cudaStream_t s) {
-  huffman_keys_kernel<T, K><<<grid_for(n, 256), 256, 0, s>>>(static_cast<const T*>(text), n, code_len, code_word,
-                                                             ncodes, L, static_cast<K*>(keys), status);
-}
-
-template <typename T>
-void launch_hk_width(uint32_t key_bytes, const void* text, uint64_t n, const uint64_t* code_len,
-                     const uint64_t* code_word, uint64_t ncodes, uint32_t L, void* keys, uint32_t* status,
-                     cudaStream_t s) {
-  switch (key_bytes) {
-    case 1: launch_hk<T, uint8_t>(text, n, code_len, code_word, ncodes, L, keys, status, s); break;
-    case 2: launch_hk<T, uint16_t>(text, n, code_len, code_word, ncodes, L, keys, status, s); break;
-    case 4: launch_hk<T, uint32_t>(text, n, code_len, code_word, ncodes, L, keys, status, s); break;
-    default: launch_hk<T, uint64_t>(text, n, code_len, code_word, ncodes, L, keys, status, s); break;
-  }
-}
-
-void launch_huffman_keys(const void* text, uint64_t n, uint32_t width, const uint64_t* code_len,
-                         const uint64_t* code_word, uint64_t ncodes, uint32_t levels, uint32_t key_bytes, void* keys,
-                         uint32_t* status, cudaStream_t s, uint64_t* launches) {
-  if (n == 0) return;
-  if (width == 1) launch_hk_width<uint8_t>(key_bytes, text, n, code_len, code_word, ncodes, levels, keys, status, s);
-  else if (width == 2)
-    launch_hk_width<uint16_t>(key_bytes, text, n, code_len, code_word, ncodes, levels, keys, status, s);
-  else launch_hk_width<uint32_t>(key_bytes, text, n, code_len, code_word, ncodes, levels, keys, status, s);
-  ++*launches;
 }
 
 void launch_symbol_histogram(const void* text, uint64_t n, uint32_t width, uint64_t nsym, unsigned long long* hist,

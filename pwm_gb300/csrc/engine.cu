@@ -89,8 +89,10 @@ void alloc_rank_select(Structure& s) {
   s.rs = true;
 }
 
+// stream: where the structure is built (its words are zeroed there, so that
+// the first build comes after).
 void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint64_t n, bool tree, bool huff,
-                     bool rank_select, cudaStream_t alloc_stream) {
+                     bool rank_select, cudaStream_t stream, cudaStream_t alloc_stream) {
   s.release();
   s.alloc_stream = alloc_stream;
   s.present = true;
@@ -100,8 +102,7 @@ void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint
   s.set_layout(level_bits);
   dev_alloc(&s.d_words, std::max<uint64_t>(s.total_words, 16) * 8, alloc_stream);
   // padding bits and words are never written by a build: zero from here on
-  if (alloc_stream) CUDA_TRY(cudaMemsetAsync(s.d_words, 0, std::max<uint64_t>(s.total_words, 16) * 8, alloc_stream));
-  else CUDA_TRY(cudaMemset(s.d_words, 0, std::max<uint64_t>(s.total_words, 16) * 8));
+  CUDA_TRY(cudaMemsetAsync(s.d_words, 0, std::max<uint64_t>(s.total_words, 16) * 8, stream));
   dev_alloc(&s.d_zeros, std::max<uint32_t>(s.levels, 1) * 8, alloc_stream);
   if (rank_select) alloc_rank_select(s);
 }
@@ -173,9 +174,10 @@ void check_device_status(pwmgpu_ctx* ctx) { throw_status(read_status(ctx)); }
 // ---------------------------------------------------------------------------
 // keys: the level-0 sequence (text or Huffman keys) of `key_bytes` per
 // element.  Builds the matrix levels into `wm` and, if wanted, the tree
-// levels into `wt`.
+// levels into `wt`.  fresh: the structures were just allocated (their words
+// are zero).
 void run_passes(pwmgpu_ctx* ctx, const void* keys, uint32_t key_bytes, uint32_t text_bytes, bool huff, uint32_t L,
-                const std::vector<PassPlan>& plan, const LevelTables& tabs, Structure& wm, Structure* wt) {
+                const std::vector<PassPlan>& plan, const LevelTables& tabs, Structure& wm, Structure* wt, bool fresh) {
   cudaStream_t s = ctx->stream;
   // Device copies of the per-pass run starts.
   size_t start_words = 0;
@@ -188,7 +190,7 @@ void run_passes(pwmgpu_ctx* ctx, const void* keys, uint32_t key_bytes, uint32_t 
 
   // Inner levels of a pass are written with OR at run edges: zero them.
   for (const auto& p : plan)
-    for (int j = 1; j < p.K; ++j) {
+    for (int j = 1; j < p.K && !fresh; ++j) {
       const uint32_t m = p.level + uint32_t(j);
       CUDA_TRY(cudaMemsetAsync(wm.d_words + wm.offs[m], 0, words_for(wm.bits[m]) * 8, s));
     }

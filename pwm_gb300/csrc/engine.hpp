@@ -395,7 +395,7 @@ void dev_alloc(P** p, size_t bytes, cudaStream_t stream) {
 // ---- structures and rank/select storage (engine.cu) ------------------------
 void alloc_rank_select(Structure& s);
 void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint64_t n, bool tree, bool huff,
-                     bool rank_select, cudaStream_t alloc_stream = nullptr);
+                     bool rank_select, cudaStream_t stream, cudaStream_t alloc_stream = nullptr);
 // Rank/select blocks of every level of the given structures (asynchronous),
 // all levels in one launch sequence.  share_level0: a plain matrix and tree,
 // whose level 0 is the same bit vector: the tree's blocks of level 0 are a
@@ -410,7 +410,8 @@ void check_device_status(pwmgpu_ctx* ctx);
 // The warp-pass matrix passes and the tree regroup, shared by plain and
 // Huffman builds (engine.cu).
 void run_passes(pwmgpu_ctx* ctx, const void* keys, uint32_t key_bytes, uint32_t text_bytes, bool huff, uint32_t L,
-                const std::vector<PassPlan>& plan, const LevelTables& tabs, Structure& wm, Structure* wt);
+                const std::vector<PassPlan>& plan, const LevelTables& tabs, Structure& wm, Structure* wt,
+                bool fresh = false);
 
 // ---- plain builds (plain.cu) -------------------------------------------------
 void validate_plain(uint64_t n, uint32_t width, uint32_t levels, bool allow40 = false);
@@ -444,12 +445,17 @@ void release_staging(pwmgpu_ctx* ctx);
 // ---- Huffman-shaped builds (huffman.cu) ------------------------------------------
 // Symbol histogram + first occurrences of a device text on the GPU, then the
 // code table on the host.
+struct SymbolCounts {  // of a text: one per symbol value
+  std::vector<uint64_t> host;
+  unsigned long long* device = nullptr;  // the context's scratch
+};
 HuffCodes huffman_codes_device(pwmgpu_ctx* ctx, const void* d_text, uint64_t n, uint32_t width, bool is_tree,
-                               uint64_t* max_symbol_out);
+                               uint64_t* max_symbol_out, SymbolCounts* counts = nullptr);
 // Huffman build of one structure (matrix, or tree through the matrix).
 void build_huffman(pwmgpu_ctx* ctx, const void* d_text, uint64_t n, uint32_t width, bool is_tree,
                    const std::vector<uint64_t>& code_len, const std::vector<uint64_t>& code_word, uint32_t levels,
-                   Structure& wm, Structure* wt, bool rank_select);
+                   Structure& wm, Structure* wt, bool rank_select, const SymbolCounts* known = nullptr,
+                   const std::function<void()>& while_running = {});
 
 // ---- shards, semi-external builds, alphabet reduction (shards.cu) -----------------
 std::unique_ptr<pwmgpu_wx> make_wx(pwmgpu_ctx* ctx, uint64_t size, uint32_t word_width, uint32_t levels,

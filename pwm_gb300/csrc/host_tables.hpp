@@ -426,6 +426,39 @@ inline std::vector<MergeRun> plan_merge_level(const std::vector<PrefixCounts>& c
   return runs;
 }
 
+// Run starts of a pass of K levels from the counts of its key_j values (level
+// j's 2^j at 2^j - 2).
+inline std::vector<uint64_t> huff_pass_starts(const uint64_t* cnt, int K) {
+  std::vector<uint64_t> st(size_t((2 << K) - 2), 0);
+  for (int j = 1; j <= K; ++j) {
+    uint64_t r = 0;
+    for (int v = 0; v < (1 << j); ++v) {
+      st[size_t((1 << j) - 2 + v)] = r;
+      r += cnt[size_t((1 << j) - 2 + v)];
+    }
+  }
+  return st;
+}
+
+// Tables of a Huffman-shaped matrix from the counts the device sums
+// (launch_huff_counts with passes of kmax levels).
+inline LevelTables build_tables_counts(const uint64_t* counts, uint32_t L, const std::vector<PassPlan>& plan,
+                                       int kmax) {
+  LevelTables t;
+  t.level_bits.assign(L, 0);
+  uint64_t run = 0;
+  for (uint32_t m = L; m-- > 0;) {
+    run += counts[m];
+    t.level_bits[m] = run;
+  }
+  t.zeros.assign(counts + L, counts + 2 * L);
+  for (size_t pi = 0; pi < plan.size(); ++pi)
+    t.starts.push_back(huff_pass_starts(counts + 2 * L + pi * size_t((2 << kmax) - 2), plan[pi].K));
+  t.seg_tree.resize(L);
+  t.seg_matrix.resize(L);
+  return t;
+}
+
 // Tables of a Huffman-shaped text from its weighted codes.  want_tree: also
 // the segments.
 inline LevelTables build_tables(const std::vector<WeightedCode>& codes, uint32_t L, const std::vector<PassPlan>& plan,
@@ -465,20 +498,7 @@ inline LevelTables build_tables(const std::vector<WeightedCode>& codes, uint32_t
     t.level_bits[m] = run;
   }
   t.starts.resize(plan.size());
-  for (size_t pi = 0; pi < plan.size(); ++pi) {
-    const auto& p = plan[pi];
-    const int C = (2 << p.K) - 2;
-    const std::vector<uint64_t>& cnt = cnts[pi];
-    std::vector<uint64_t> st(size_t(C), 0);
-    for (int j = 1; j <= p.K; ++j) {
-      uint64_t r = 0;
-      for (int v = 0; v < (1 << j); ++v) {
-        st[size_t((1 << j) - 2 + v)] = r;
-        r += cnt[size_t((1 << j) - 2 + v)];
-      }
-    }
-    t.starts[pi] = std::move(st);
-  }
+  for (size_t pi = 0; pi < plan.size(); ++pi) t.starts[pi] = huff_pass_starts(cnts[pi].data(), plan[pi].K);
   if (want_tree) {
     t.seg_tree.resize(L);
     t.seg_matrix.resize(L);

@@ -216,6 +216,16 @@ bool launch_regroup_segs(const uint64_t* flat, const uint32_t* levels, uint32_t 
 void launch_huffman_keys(const void* text, uint64_t n, uint32_t width, const uint64_t* code_len,
                          const uint64_t* code_word, uint64_t ncodes, uint32_t levels, uint32_t key_bytes, void* keys,
                          uint32_t* status, cudaStream_t s, uint64_t* launches);
+// Counts of a code table over a text with symbol counts hist, codes at most L
+// long (those of symbols that occur), passes of K levels: at m the symbols
+// whose code is m + 1 long, at L + m the zeros of level m, then (2 << K) - 2
+// words a pass, its key_j counts.  out: huff_count_words(L, K) zeroed words.
+__host__ __device__ constexpr uint32_t huff_count_words(uint32_t L, uint32_t K) {
+  return 2 * L + (L + K - 1) / K * ((2u << K) - 2);
+}
+void launch_huff_counts(const unsigned long long* hist, const uint64_t* code_len, const uint64_t* code_word,
+                        uint64_t ncodes, uint32_t L, uint32_t K, unsigned long long* out, cudaStream_t s,
+                        uint64_t* launches);
 // Histogram of the symbols (u64 counts; 8- and 16-bit texts: all 2^8 / 2^16
 // values, so hist needs that many entries; 32-bit texts: symbols below nsym).
 // hist must be zeroed.

@@ -20,9 +20,9 @@ std::unique_ptr<pwmgpu_wx> make_wx(pwmgpu_ctx* ctx, uint64_t size, uint32_t word
   const bool rs = shape_flags & PWMGPU_RANK_SELECT;
   std::vector<uint64_t> bits(levels, size);
   cudaStream_t as = ctx->async_alloc ? ctx->stream : nullptr;
-  alloc_structure(wx->wm, bits, size, false, false, rs && (shape_flags & PWMGPU_MATRIX), as);
+  alloc_structure(wx->wm, bits, size, false, false, rs && (shape_flags & PWMGPU_MATRIX), ctx->stream, as);
   wx->wm_internal = !(shape_flags & PWMGPU_MATRIX);
-  if (shape_flags & PWMGPU_TREE) alloc_structure(wx->wt, bits, size, true, false, rs, as);
+  if (shape_flags & PWMGPU_TREE) alloc_structure(wx->wt, bits, size, true, false, rs, ctx->stream, as);
   return wx;
 }
 
