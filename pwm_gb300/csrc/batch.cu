@@ -3,6 +3,7 @@
 // that a single build derives on the host computed on the device instead, so
 // that a whole batch is one CUDA graph without host round trips.
 #include "kernels.cuh"
+#include "plane_count.cuh"
 
 namespace pwmgpu {
 
@@ -12,6 +13,44 @@ constexpr int kBatchThreads = 256;
 
 __device__ __forceinline__ uint32_t rev_bits_dev(uint32_t v, uint32_t bits) {
   return bits == 0 ? 0u : (__brev(v) >> (32 - bits));
+}
+
+// Counts of one chunk (whole first-pass tiles) of an 8-bit text of L = 2..4
+// levels by planes (plane_count.cuh): the finest runs of every tile, their
+// prefixes in the chunk and totals, and the text's histogram.
+template <int L>
+__device__ __forceinline__ void batch_hist_planes(const uint8_t* text, const BatchChunk& c, uint32_t ntiles,
+                                                  uint32_t* smem, unsigned long long* hist, uint32_t* tilecnt,
+                                                  uint32_t* relpre, unsigned long long* blocksum, uint32_t* status) {
+  constexpr int WARPS = kBatchThreads / 32;
+  constexpr uint32_t NB = 1u << (L - 1);  // D = L - 1: every text of up to 4 levels takes one pass
+  auto* pairs = reinterpret_cast<uint32_t (*)[WARPS][8]>(smem);  // [2]
+  const uint32_t tid = threadIdx.x, T = 1u << c.log2T;
+  const int nv = int(T / (16 * kBatchThreads));  // 1, 2 or 4 vectors a thread
+  uint32_t rel = 0, mine = 0, seen = 0;
+  for (uint32_t k = 0; k < ntiles; ++k) {
+    const uint64_t start = uint64_t(k) << c.log2T;
+    const uint32_t len = uint32_t(c.len - start < T ? c.len - start : T);
+    count_tile_planes<L, kBatchThreads, 4>(text + start, len, nv, seen, pairs[k & 1], [](int, uint32_t, const uint4&) {});
+    __syncthreads();
+    const uint32_t (*pr)[8] = pairs[k & 1];
+    if (tid < NB) {
+      const uint32_t q = __brev(tid) >> (32 - (L - 1));
+      uint32_t x = 0;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) x += (pr[w][q] & 0xFFFFu) + (pr[w][q] >> 16);
+      tilecnt[c.cnt_off + k * NB + tid] = x;
+      relpre[c.cnt_off + k * NB + tid] = rel;
+      rel += x;
+    } else if (tid >= 32 && tid < 32 + (1u << L)) {
+      const uint32_t s = tid - 32;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) mine += (pr[w][s >> 1] >> (16 * (s & 1))) & 0xFFFFu;
+    }
+  }
+  if (seen & ~(((1u << L) - 1u) * 0x01010101u)) atomicOr(status, kErrSymbol);
+  if (tid < NB) blocksum[c.blk_off + tid] = rel;
+  if (tid >= 32 && tid < 32 + (1u << L) && mine) atomicAdd(&hist[tid - 32], (unsigned long long)mine);
 }
 
 // Leaf histogram of one chunk of one text (2^L <= 4096 bins in shared
@@ -42,11 +81,22 @@ __global__ void __launch_bounds__(kBatchThreads) batch_hist_kernel(const T* __re
   const uint32_t mine = threadIdx.x % copies, lane = threadIdx.x & 31;
   const uint32_t D = c.D, dsh = t.levels - c.D;  // the digit: symbol bits [L-D, L)
   const uint32_t ntiles = D ? uint32_t((c.len + (uint64_t(1) << c.log2T) - 1) >> c.log2T) : 0u;
-  // Up to 16 bins: one counter per (tile, bin, lane) serves both the text's
-  // histogram and the tiles' finest-run counts (each a sum over bins), one
-  // shared atomic per symbol; else a text histogram (per-thread copies) and
-  // the tiles' digit counters.
+  // Up to 16 bins: counts per (tile, bin) serve both the text's histogram and
+  // the tiles' finest-run counts (each a sum over bins), of 8-bit texts by
+  // planes, of wider ones a counter per (tile, bin, lane) and one shared atomic
+  // per symbol; else a text histogram (per-thread copies) and the tiles' digit
+  // counters.
   const bool by_tile = D && bins <= 16;
+  if constexpr (sizeof(T) == 1) {
+    if (by_tile) {
+      switch (t.levels) {
+        case 2: batch_hist_planes<2>(texts + t.offset + c.start, c, ntiles, hsm, hist + t.hist_off, tilecnt, relpre, blocksum, status); break;
+        case 3: batch_hist_planes<3>(texts + t.offset + c.start, c, ntiles, hsm, hist + t.hist_off, tilecnt, relpre, blocksum, status); break;
+        default: batch_hist_planes<4>(texts + t.offset + c.start, c, ntiles, hsm, hist + t.hist_off, tilecnt, relpre, blocksum, status); break;
+      }
+      return;
+    }
+  }
   if (!by_tile)
     for (uint32_t i = threadIdx.x; i < bins * copies; i += kBatchThreads) h[i] = 0;
   for (uint32_t i = threadIdx.x; i < ntiles * 16 * 32; i += kBatchThreads) tc[i] = 0;

@@ -3,6 +3,7 @@
 
 #include "gen.hpp"
 #include "kernels.cuh"
+#include "plane_count.cuh"
 
 namespace pwmgpu {
 
@@ -233,6 +234,62 @@ __global__ void __launch_bounds__(kTileHistThreads) tile_hist_kernel(const T* te
   if (seen >> levels) atomicOr(status, kErrSymbol);
   if (tid < int(NB)) blocksum[uint64_t(block) * NB + tid] = rel;
   if (tid < int(bins) && prev) atomicAdd(&hist[tid], (unsigned long long)prev);
+}
+
+// The same for 8-bit texts of 2 to 4 levels, counted by planes
+// (plane_count.cuh): 2^26 symbols of 2 levels 34 -> 20 us, where an atomic a
+// symbol bounded it.  Per tile one barrier: the warps' sums lie in one of two
+// buffers, so the threads that add them up (one a run, one a symbol value) read
+// one while the next tile fills the other.
+template <int L>
+__global__ void __launch_bounds__(kTileHistThreads) tile_hist_planes_kernel(
+    const uint8_t* text, uint64_t n, uint32_t tile_keys, uint32_t tiles_per_block, uint32_t block0,
+    unsigned long long* hist, uint32_t* tilecnt, uint32_t* relpre, unsigned long long* blocksum, uint64_t* level0_a,
+    uint64_t* level0_b, uint32_t* status) {
+  constexpr int WARPS = kTileHistThreads / 32, HV = 4;
+  constexpr uint32_t NB = 1u << (L - 1);  // runs of the first L - 1 bits
+  __shared__ uint32_t pairs[2][WARPS][8];
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  const uint32_t block = block0 + blockIdx.x;
+  const uint64_t first_tile = uint64_t(block) * tiles_per_block;
+  const int nv = int(tile_keys / (16 * kTileHistThreads));  // 2 or 4 vectors a thread
+  uint32_t rel = 0, mine = 0, seen = 0;  // run tid so far; symbol value tid - 32 so far
+  for (uint32_t k = 0; k < tiles_per_block; ++k) {
+    const uint64_t tile = first_tile + k, start = tile * tile_keys;
+    if (start >= n) break;
+    const uint32_t len = uint32_t(n - start < tile_keys ? n - start : tile_keys);
+    count_tile_planes<L, kTileHistThreads, HV>(
+        text + start, len, nv, seen, pairs[k & 1], [&](int, uint32_t i, const uint4& v) {
+          if (!level0_a) return;
+          // level 0: the top bits in order, 64 symbols from 4 lanes
+          uint32_t x = vector_bits<uint8_t>(v, L - 1) << (16 * (1 - (lane & 1)));
+          x |= __shfl_down_sync(0xFFFFFFFFu, x, 1);
+          const uint32_t lo = __shfl_down_sync(0xFFFFFFFFu, x, 2);
+          if ((lane & 3) == 0 && 16 * i < len) {
+            const uint64_t word = (uint64_t(x) << 32) | lo;
+            level0_a[(start >> 6) + (i >> 2)] = word;
+            if (level0_b) level0_b[(start >> 6) + (i >> 2)] = word;
+          }
+        });
+    __syncthreads();
+    const uint32_t (*pr)[8] = pairs[k & 1];
+    if (tid < NB) {  // run tid: the two symbol values whose top bits, reversed, are tid
+      const uint32_t q = reverse_low_bits(tid, L - 1);
+      uint32_t c = 0;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) c += (pr[w][q] & 0xFFFFu) + (pr[w][q] >> 16);
+      tilecnt[tile * NB + tid] = c;
+      relpre[tile * NB + tid] = rel;
+      rel += c;
+    } else if (tid >= 32 && tid < 32 + (1u << L)) {
+      const uint32_t s = tid - 32;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) mine += (pr[w][s >> 1] >> (16 * (s & 1))) & 0xFFFFu;
+    }
+  }
+  if (seen & ~(((1u << L) - 1u) * 0x01010101u)) atomicOr(status, kErrSymbol);
+  if (tid < NB) blocksum[uint64_t(block) * NB + tid] = rel;
+  if (tid >= 32 && tid < 32 + (1u << L) && mine) atomicAdd(&hist[tid - 32], (unsigned long long)mine);
 }
 
 // After the tile histogram, one launch of NB + 1 CTAs of 1024 threads:
@@ -1077,11 +1134,21 @@ void launch_tile_histogram_blocks(const void* text, uint64_t n, uint32_t width, 
   tile_hist_kernel<T, B8><<<nblk, kTileHistThreads, 0, s>>>(static_cast<const T*>(text), n, levels, D, tile_keys, \
                                                             per, block0, hist, tilecnt, relpre, blocksum,       \
                                                             level0_a, level0_b, status)
-  if (width == 1 && levels == 8) PWMGPU_TH(uint8_t, true);
+#define PWMGPU_THP(L)                                                                                              \
+  tile_hist_planes_kernel<L><<<nblk, kTileHistThreads, 0, s>>>(static_cast<const uint8_t*>(text), n, tile_keys, per, \
+                                                               block0, hist, tilecnt, relpre, blocksum, level0_a,    \
+                                                               level0_b, status)
+  const bool planes = width == 1 && D + 1 == levels &&
+                      (tile_keys == 32 * kTileHistThreads || tile_keys == 64 * kTileHistThreads);
+  if (planes && levels == 2) PWMGPU_THP(2);
+  else if (planes && levels == 3) PWMGPU_THP(3);
+  else if (planes && levels == 4) PWMGPU_THP(4);
+  else if (width == 1 && levels == 8) PWMGPU_TH(uint8_t, true);
   else if (width == 1) PWMGPU_TH(uint8_t, false);
   else if (width == 2) PWMGPU_TH(uint16_t, false);
   else PWMGPU_TH(uint32_t, false);
 #undef PWMGPU_TH
+#undef PWMGPU_THP
   ++*launches;
 }
 

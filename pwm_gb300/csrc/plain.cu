@@ -243,7 +243,10 @@ void build_one_pass(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text) {
   const bool half = w == 1 && n <= kHalfTileMax;
   const uint32_t T = half ? tile_pass_half_elems() : tile_pass_elems(w);
   const uint32_t tiles = uint32_t((n + T - 1) / T);
-  const uint32_t per = tiles <= 2 * 152 ? 1u : std::min(tile_hist_tiles_per_block(), tiles / 152);
+  // tiles of a histogram block: one while there are few; then, counted by planes (nothing to set up or sum at a
+  // block's end), blocks for every SM several times over, else longer ones
+  const uint32_t per =
+      tiles <= 2 * 152 ? 1u : std::min(tile_hist_tiles_per_block(), std::max(1u, tiles / (w == 1 && L <= 4 ? 152 * 6 : 152)));
   const uint32_t nblocks = (tiles + per - 1) / per, D = L - 1;
   const uint64_t NB = uint64_t(1) << D;
   // zeroed with the status word: the histogram, the pass's tile counter and,
