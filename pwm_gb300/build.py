@@ -14,7 +14,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libpwmgpu.so")
 OBJ = os.path.join(HERE, "_build")
 SOURCES = ["abi.cu", "engine.cu", "plain.cu", "huffman.cu", "shards.cu", "batch_host.cu", "build_kernels.cu", "split.cu",
-           "tile.cu", "tile_deep.cu", "tile_batch.cu", "ranksel.cu", "batch.cu", "serve.cu", "merge.cu", "staging.cu",
+           "tile.cu", "tile_deep.cu", "tile_wide.cu", "tile_batch.cu", "ranksel.cu", "batch.cu", "serve.cu", "merge.cu", "staging.cu",
            "alphabet.cu", "huff_kernels.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC",

@@ -95,8 +95,8 @@ __global__ void __launch_bounds__(kTileHistThreads) tile_hist_kernel(const T* te
   constexpr int BINS = 256;
   // One counter per (bin, lane) shared by the block's warps: lane k counts
   // into column k, so the 32 lanes of an atomic never meet on an address or
-  // a bank, however skewed the text (at most 8 warps x 64 symbols x 16
-  // tiles = 8192 per counter).
+  // a bank, however skewed the text (at most 8 warps x 128 symbols x 16
+  // tiles = 16384 per counter).
   __shared__ __align__(16) uint32_t h[BINS * 32];
   __shared__ uint32_t s_tc[BINS / 2];  // runs of the first D <= 7 bits
   const int tid = threadIdx.x;
@@ -123,33 +123,37 @@ __global__ void __launch_bounds__(kTileHistThreads) tile_hist_kernel(const T* te
     atomicAdd(&mine[(c & binmask) * 32], 1u);  // an out-of-range symbol fails the build below
   };
   constexpr int PER = 16 / sizeof(T);
-  // whole aligned tiles of HV 16-byte vectors per thread, loaded one tile
-  // ahead so that the loads overlap the counting of the previous tile
+  // whole aligned units (a tile, or half of a double one) of HV 16-byte
+  // vectors per thread, loaded one unit ahead so that the loads overlap the
+  // counting of the previous one
   constexpr int HV = 4;
-  const uint32_t tile_vecs = uint32_t(tile_keys * sizeof(T) / 16);
-  const bool vec = tile_keys * sizeof(T) % (16 * kTileHistThreads) == 0 && tile_vecs <= HV * kTileHistThreads &&
+  const uint32_t tile_units = tile_keys * sizeof(T) > 16 * HV * kTileHistThreads ? 2 : 1;
+  const uint32_t unit_keys = tile_keys / tile_units, units = tiles_per_block * tile_units;
+  const uint32_t unit_vecs = uint32_t(unit_keys * sizeof(T) / 16);
+  const bool vec = unit_keys * sizeof(T) % (16 * kTileHistThreads) == 0 && unit_vecs <= HV * kTileHistThreads &&
                    (reinterpret_cast<uintptr_t>(text) % 16) == 0;
-  const int nv = int(tile_vecs / kTileHistThreads);  // vectors per thread (1..HV)
-  auto full_tile = [&](uint64_t tile) { return vec && (tile + 1) * tile_keys <= n; };
+  const int nv = int(unit_vecs / kTileHistThreads);  // vectors per thread (1..HV)
+  auto full_unit = [&](uint64_t start) { return vec && start + unit_keys <= n; };
+  const uint64_t block_start = first_tile * tile_keys;
   uint4 ahead[HV];
-  if (full_tile(first_tile)) {
-    const uint4* p = reinterpret_cast<const uint4*>(text + first_tile * tile_keys);
+  if (full_unit(block_start)) {
+    const uint4* p = reinterpret_cast<const uint4*>(text + block_start);
 #pragma unroll
     for (int v = 0; v < HV; ++v)
       if (v < nv) ahead[v] = __ldcs(p + tid + v * kTileHistThreads);
   }
-  for (uint32_t k = 0; k < tiles_per_block; ++k) {
-    const uint64_t tile = first_tile + k;
-    const uint64_t start = tile * tile_keys;
+  for (uint32_t k = 0; k < units; ++k) {
+    const uint64_t start = block_start + uint64_t(k) * unit_keys;
     if (start >= n) break;
-    const uint64_t len = n - start < tile_keys ? n - start : tile_keys;
+    const uint64_t tile = first_tile + k / tile_units;
+    const uint64_t len = n - start < unit_keys ? n - start : unit_keys;
     const T* p = text + start;
-    if (full_tile(tile)) {
+    if (full_unit(start)) {
       uint4 cur[HV];
 #pragma unroll
       for (int v = 0; v < HV; ++v) cur[v] = ahead[v];
-      if (k + 1 < tiles_per_block && full_tile(tile + 1)) {
-        const uint4* q = reinterpret_cast<const uint4*>(text + (tile + 1) * tile_keys);
+      if (k + 1 < units && full_unit(start + unit_keys)) {
+        const uint4* q = reinterpret_cast<const uint4*>(text + start + unit_keys);
 #pragma unroll
         for (int v = 0; v < HV; ++v)
           if (v < nv) ahead[v] = __ldcs(q + tid + v * kTileHistThreads);
@@ -204,6 +208,7 @@ __global__ void __launch_bounds__(kTileHistThreads) tile_hist_kernel(const T* te
         }
       }
     }
+    if (k % tile_units + 1 < tile_units && start + unit_keys < n) continue;  // the tile goes on
     __syncthreads();
     if (tid < int(bins)) {
       // row of 32 counters, its 16-byte pieces read in a rotated order so
@@ -246,13 +251,13 @@ __global__ void __launch_bounds__(kTileHistThreads) tile_hist_planes_kernel(
     const uint8_t* text, uint64_t n, uint32_t tile_keys, uint32_t tiles_per_block, uint32_t block0,
     unsigned long long* hist, uint32_t* tilecnt, uint32_t* relpre, unsigned long long* blocksum, uint64_t* level0_a,
     uint64_t* level0_b, uint32_t* status) {
-  constexpr int WARPS = kTileHistThreads / 32, HV = 4;
+  constexpr int WARPS = kTileHistThreads / 32, HV = 8;
   constexpr uint32_t NB = 1u << (L - 1);  // runs of the first L - 1 bits
   __shared__ uint32_t pairs[2][WARPS][8];
   const uint32_t tid = threadIdx.x, lane = tid & 31;
   const uint32_t block = block0 + blockIdx.x;
   const uint64_t first_tile = uint64_t(block) * tiles_per_block;
-  const int nv = int(tile_keys / (16 * kTileHistThreads));  // 2 or 4 vectors a thread
+  const int nv = int(tile_keys / (16 * kTileHistThreads));  // 2, 4 or 8 vectors a thread
   uint32_t rel = 0, mine = 0, seen = 0;  // run tid so far; symbol value tid - 32 so far
   for (uint32_t k = 0; k < tiles_per_block; ++k) {
     const uint64_t tile = first_tile + k, start = tile * tile_keys;
@@ -1139,7 +1144,8 @@ void launch_tile_histogram_blocks(const void* text, uint64_t n, uint32_t width, 
                                                                block0, hist, tilecnt, relpre, blocksum, level0_a,    \
                                                                level0_b, status)
   const bool planes = width == 1 && D + 1 == levels &&
-                      (tile_keys == 32 * kTileHistThreads || tile_keys == 64 * kTileHistThreads);
+                      (tile_keys == 32 * kTileHistThreads || tile_keys == 64 * kTileHistThreads ||
+                       tile_keys == 128 * kTileHistThreads);
   if (planes && levels == 2) PWMGPU_THP(2);
   else if (planes && levels == 3) PWMGPU_THP(3);
   else if (planes && levels == 4) PWMGPU_THP(4);

@@ -236,6 +236,7 @@ struct TilePassHost {
   int K = 0;
   bool out = false;
   bool segmented = false;
+  uint32_t vectors = 0;  // 16-byte vectors a thread of its tiles (0: the usual; tile_keys follows it)
   uint32_t tiles = 0;
   std::vector<TileSegHost> segs;
   std::vector<uint64_t> table;  // per segment: tile_table_size(K) entries

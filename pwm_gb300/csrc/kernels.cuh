@@ -153,11 +153,9 @@ void launch_split_pass_batched(uint32_t key_bytes, int K, const SplitArgs* args,
                                uint64_t* launches);
 
 // ---- segmented tile passes (plain keys, matrix and tree together) ------------
-// Keys of one tile for a key width.
-uint32_t tile_pass_elems(uint32_t key_bytes);
-// The same of the half-size tiles of a one-pass text of 1-byte keys
-// (TileArgs::half_tiles).
-uint32_t tile_pass_half_elems();
+// Keys of one tile for a key width and the vectors a thread of
+// TileArgs::tile_vectors (0: the usual).
+uint32_t tile_pass_elems(uint32_t key_bytes, uint32_t vectors = 0);
 // One pass of K levels over a.tiles tiles; `out`: the pass writes S_{l+K}.
 // Digit counts of the passes of a matrix-only build (pass_digits_kernel):
 // pass p covers levels level[p]..level[p]+K[p]-1, its natural digit is

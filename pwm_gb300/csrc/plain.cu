@@ -29,6 +29,18 @@ uint32_t tile_pass_key_bytes(uint32_t width, uint32_t L, uint32_t l) {
   return l == 0 ? width : std::min(width, tile_key_bytes(L - l));
 }
 
+// 16-byte vectors a thread of the tiles of the pass from level l (0: the
+// usual): double tiles where the text fills the SMs with them.  Passes that
+// write the next sequence from 1024 tiles on (3 CTAs an SM: 456 at once);
+// last passes over 1-byte keys from 512 (5 an SM): at 4 levels in one pass 51
+// us either way at 2^24 symbols, 75 against 85 at 2^25.
+uint32_t pass_vectors(uint32_t width, uint32_t L, int kmax, uint32_t l, uint64_t n) {
+  const uint32_t K = std::min<uint32_t>(uint32_t(kmax), L - l), kb = tile_pass_key_bytes(width, L, l);
+  const uint32_t V = 8;
+  if (l + K < L) return K == uint32_t(kTileMaxLevels) && n >= 1024 * uint64_t(tile_pass_elems(kb, V)) ? V : 0u;
+  return kb == 1 && K <= uint32_t(kTileMaxLevels) && n >= 512 * uint64_t(tile_pass_elems(kb, V)) ? V : 0u;
+}
+
 // Device descriptors of passes [from, to): per pass its segments, its level
 // descriptor and its start tables, at offsets of one uploaded blob.
 struct TileBlob {
@@ -130,6 +142,7 @@ const void* enqueue_tile_pass(pwmgpu_ctx* ctx, const std::vector<TilePassHost>& 
     a.first_level_written = first->level0_written ? 1u : 0u;
   }
   if (pi == 0 && first) a.clear_edges = 1u;  // the histogram kernel did not zero the first pass's levels
+  a.tile_vectors = p.vectors;
   a.spin_limit = ctx->spin_limit;
   std::vector<uint32_t> b = bounds.size() >= 2 ? bounds : std::vector<uint32_t>{0, p.tiles};
   if (ctx->withhold_first_tile && !given && p.tiles >= 2 && bounds.size() < 2) b = {1, p.tiles};  // tile 0 never publishes
@@ -227,6 +240,10 @@ namespace {
 // 46 with whole tiles (3 levels 19 and 22), 2^21 bytes 41 and 46, 2^22 57 and
 // 52.
 constexpr uint64_t kHalfTileMax = uint64_t(1) << 21;  // symbols
+// Long ones take double tiles (tile_wide.cu): 3 levels of 2^24 bytes 53 us
+// against 59, 2^28 312 and 358; 5 levels of 2^24 73 and 71, 2^25 116 and 123,
+// 2^28 694 and 735; 8 levels are no faster with them.
+constexpr uint64_t kDoubleTileMin = uint64_t(1) << 24;  // symbols, up to 4 levels; twice as many up to 7
 // 8 levels of bytes in one pass: its tiles cost more than two 4-level passes
 // (127 runs at the deepest level), but a text saves the second pass, the
 // host's plan of it and the regroup.  One pass against two: both structures
@@ -240,8 +257,8 @@ void build_one_pass(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text) {
   const uint32_t L = wx->levels, w = wx->width;
   const uint64_t n = wx->n;
   const bool tree = wx->wt.present;
-  const bool half = w == 1 && n <= kHalfTileMax;
-  const uint32_t T = half ? tile_pass_half_elems() : tile_pass_elems(w);
+  const uint32_t vectors = w != 1 ? 0u : n <= kHalfTileMax ? 2u : L <= 7 && n >= (L <= 4 ? kDoubleTileMin : 2 * kDoubleTileMin) ? 8u : 0u;
+  const uint32_t T = tile_pass_elems(w, vectors);
   const uint32_t tiles = uint32_t((n + T - 1) / T);
   // tiles of a histogram block: one while there are few; then, counted by planes (nothing to set up or sum at a
   // block's end), blocks for every SM several times over, else longer ones
@@ -306,7 +323,7 @@ void build_one_pass(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text) {
   a.tiles_per_block = per;
   a.first_level_written = 1u;
   a.clear_edges = 1u;
-  a.half_tiles = half ? 1u : 0u;
+  a.tile_vectors = vectors;
   a.spin_limit = ctx->spin_limit;
   const uint64_t structs = one.text.wt ? 2 : 1;
   {
@@ -454,7 +471,7 @@ void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostI
                              ctx->down));
   };
   if (tile_hist) {
-    const uint32_t T = tile_pass_elems(wx->width);
+    const uint32_t T = tile_pass_elems(wx->width, pass_vectors(wx->width, L, kmax, 0, n));
     const uint64_t tiles = (n + T - 1) / T;
     const uint32_t per = tile_hist_tiles_per_block();
     const uint32_t nblocks = tile_hist_blocks(n, T);
@@ -564,7 +581,8 @@ void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostI
       early[i].out = shape[i].has_out;
     }
     TilePassHost& p0 = early[0];
-    const uint32_t T = tile_pass_elems(wx->width);
+    p0.vectors = pass_vectors(wx->width, L, kmax, 0, n);
+    const uint32_t T = tile_pass_elems(wx->width, p0.vectors);
     p0.segmented = want_tree;
     p0.tiles = uint32_t((n + T - 1) / T);
     p0.segs.push_back({0, n, 0, 0, 0});
@@ -611,7 +629,8 @@ void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostI
       early[i].out = shape[i].has_out;
     }
     TilePassHost& p0 = early[0];
-    const uint32_t T = tile_pass_elems(wx->width);
+    p0.vectors = pass_vectors(wx->width, L, kmax, 0, n);
+    const uint32_t T = tile_pass_elems(wx->width, p0.vectors);
     p0.segmented = want_tree;
     p0.tiles = uint32_t((n + T - 1) / T);
     p0.segs.push_back({0, n, 0, 0, 0});
@@ -624,7 +643,8 @@ void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostI
     // the look-back state sized for every later pass now (a later pass has at
     // most 2^16 segments, each adding at most one partial tile), so that no
     // later pass reallocates it, which would wait for this one
-    ctx->grow("lookback", (uint64_t(p0.tiles) + 65536 + 16) * (uint64_t(1) << kTileMaxLevels) * 8 + 64);
+    const uint64_t most = n / tile_pass_elems(wx->width) + 1;  // no pass has smaller tiles
+    ctx->grow("lookback", (most + 65536 + 16) * (uint64_t(1) << kTileMaxLevels) * 8 + 64);
     next_in = enqueue_tile_pass(ctx, early, 0, d_b0, b0, d_text, wx->width, n, wx->wm, want_tree ? &wx->wt : nullptr,
                                 nullptr);
     from = 1;
@@ -642,7 +662,7 @@ void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostI
   uint64_t* d_segs = nullptr;  // the regroup's segments (device)
   PrefixCounts cnt;  // natural-prefix counts per level
   const uint32_t w = wx->width;
-  auto tile_keys = [&](uint32_t l) { return tile_pass_elems(tile_pass_key_bytes(w, L, l)); };
+  auto tile_keys = [&](uint32_t l) { return tile_pass_elems(tile_pass_key_bytes(w, L, l), pass_vectors(w, L, kmax, l, n)); };
   if (digit_plan) {
     tile_passes = plan_matrix_passes(h_digits, n, L, kmax, tile_keys);
     tabs.level_bits.assign(L, n);
@@ -665,6 +685,7 @@ void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostI
     plan = plan_passes(L, ctx->pass_levels);
     tabs = build_tables_plain(std::vector<uint64_t>(h_hist, h_hist + bins), L, plan, want_tree);
   }
+  for (auto& p : tile_passes) p.vectors = pass_vectors(w, L, kmax, p.level, n);
   wx->wm.zeros = tabs.zeros;
   CUDA_TRY(cudaMemcpyAsync(wx->wm.d_zeros, wx->wm.zeros.data(), L * 8, cudaMemcpyHostToDevice, s));
   // Streaming the structures back: after each pass its levels of the

@@ -100,7 +100,7 @@ struct TileArgs {
   // tile's index in its segment / tiles_per_block.
   uint32_t text_blocks;
   uint32_t first_level_written;  // level l is already written (by the histogram kernel)
-  uint32_t half_tiles;           // one-pass texts of 1-byte keys: tiles of half as many keys
+  uint32_t tile_vectors;         // 16-byte vectors a thread of the tiles (0: the usual kTileVectors)
   uint32_t clear_edges;          // the levels were not zeroed: shared words are cleared before they are set
   // Optional: words [0, zero_words) at zero_a (and zero_b) are zeroed, tile g
   // taking words [g * zero_per_tile, (g + 1) * zero_per_tile): the levels of
@@ -1384,13 +1384,18 @@ __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in)
 }
 
 // A launch of one pass: each CTA takes the next tile from the launch's tile
-// counter.  CTAs per SM (registers a thread): the bit-plane form 6 (40), 4
-// (64) for 5-8 levels; the key form over 1-byte keys 5 (48), over wider keys
-// 4 (64; at 48 they spill more and measured slower), 3 for 5-8 levels.
+// counter.  Threads per SM (registers a thread): the bit-plane form 1536 (40),
+// with double tiles 1280 (48), 1024 (64) for 5-8 levels; the key form over
+// 1-byte keys 1280 (48), over wider keys 1024 (64; at 48 they spill more and
+// measured slower), 768 (80) with double tiles and for 5-8 levels.
+template <typename KeyT, int K, int V, bool PLANES>
+constexpr int tile_threads_per_sm() {
+  if (PLANES) return K > kTileMaxLevels ? (V > 4 ? 768 : 1024) : (V > 4 ? 1280 : 1536);
+  return K > kTileMaxLevels || V > 4 ? 768 : (sizeof(KeyT) == 1 ? 1280 : 1024);
+}
 template <typename KeyT, int K, bool OUT, int THREADS, int V, typename KeyO = KeyT, bool PLANES = false>
-__global__ void __launch_bounds__(THREADS, (K > kTileMaxLevels ? (PLANES ? 1024 : 768)
-                                                                 : (PLANES ? 1536 : (sizeof(KeyT) == 1 ? 1280 : 1024))) /
-                                               THREADS) tile_pass_kernel(TileArgs a) {
+__global__ void __launch_bounds__(THREADS, tile_threads_per_sm<KeyT, K, V, PLANES>() / THREADS)
+    tile_pass_kernel(TileArgs a) {
   __shared__ uint32_t s_g;
   if (threadIdx.x == 0) s_g = a.tile_base + atomicAdd(a.tile_counter, 1u);
   __syncthreads();

@@ -19,25 +19,27 @@ void launch_deep_key(int K, const TileArgs& a, cudaStream_t s) {
   }
 }
 
-// Half-size tiles: a short text fills twice as many SMs.
-void launch_half(int K, const TileArgs& a, cudaStream_t s) {
+// Tiles of V vectors a thread: half-size ones for short texts, which fill
+// twice as many SMs; double ones for long texts (tile_wide.cu says why).
+template <int V>
+void launch_sized(int K, const TileArgs& a, cudaStream_t s) {
   switch (K) {
-    case 2: launch_tile_one<uint8_t, 2, false, uint8_t, true, kTileVectors / 2>(a, s); break;
-    case 3: launch_tile_one<uint8_t, 3, false, uint8_t, true, kTileVectors / 2>(a, s); break;
-    case 4: launch_tile_one<uint8_t, 4, false, uint8_t, true, kTileVectors / 2>(a, s); break;
-    case 5: launch_tile_one<uint8_t, 5, false, uint8_t, true, kTileVectors / 2>(a, s); break;
-    case 6: launch_tile_one<uint8_t, 6, false, uint8_t, true, kTileVectors / 2>(a, s); break;
-    case 7: launch_tile_one<uint8_t, 7, false, uint8_t, true, kTileVectors / 2>(a, s); break;
-    default: launch_tile_one<uint8_t, 8, false, uint8_t, true, kTileVectors / 2>(a, s); break;
+    case 1: launch_tile_one<uint8_t, 1, false, uint8_t, true, V>(a, s); return;
+    case 2: launch_tile_one<uint8_t, 2, false, uint8_t, true, V>(a, s); return;
+    case 3: launch_tile_one<uint8_t, 3, false, uint8_t, true, V>(a, s); return;
+    case 4: launch_tile_one<uint8_t, 4, false, uint8_t, true, V>(a, s); return;
+    case 5: launch_tile_one<uint8_t, 5, false, uint8_t, true, V>(a, s); break;
+    case 6: launch_tile_one<uint8_t, 6, false, uint8_t, true, V>(a, s); break;
+    case 7: launch_tile_one<uint8_t, 7, false, uint8_t, true, V>(a, s); break;
+    default: launch_tile_one<uint8_t, 8, false, uint8_t, true, V>(a, s); break;
   }
 }
 
 }  // namespace
 
-uint32_t tile_pass_half_elems() { return uint32_t(kTileThreads * (kTileVectors / 2) * 16); }
-
 void launch_tile_pass_deep(uint32_t key_bytes, int K, const TileArgs& a, cudaStream_t s) {
-  if (a.half_tiles) launch_half(K, a, s);
+  if (a.tile_vectors == kTileVectors / 2) launch_sized<kTileVectors / 2>(K, a, s);
+  else if (a.tile_vectors) launch_sized<kTileVectors * 2>(K, a, s);
   else if (key_bytes == 1) launch_deep_key<uint8_t>(K, a, s);
   else if (key_bytes == 2) launch_deep_key<uint16_t>(K, a, s);
   else launch_deep_key<uint32_t>(K, a, s);

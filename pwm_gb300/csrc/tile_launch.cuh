@@ -24,7 +24,11 @@ void launch_tile_one(const TileArgs& a, cudaStream_t s) {
 }
 
 // Last passes of 5..8 levels with given prefixes (tile_deep.cu); with
-// TileArgs::half_tiles, of 2..8 levels over 1-byte keys.
+// TileArgs::tile_vectors, last passes over 1-byte keys (half: 2..8 levels,
+// double: 1..8).
 void launch_tile_pass_deep(uint32_t key_bytes, int K, const TileArgs& a, cudaStream_t s);
+// Passes of kTileMaxLevels levels that write S_{l+K}, double tiles
+// (tile_wide.cu).
+void launch_tile_pass_wide(uint32_t key_bytes, uint32_t out_bytes, const TileArgs& a, cudaStream_t s);
 
 }  // namespace pwmgpu

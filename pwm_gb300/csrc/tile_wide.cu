@@ -1,0 +1,33 @@
+// Tile passes of 4 levels that write S_{l+K}, in tiles of twice the usual keys.
+//
+// Half of a tile's instructions do not grow with its keys: finding its
+// segment, the barriers and scans of every split, the set-up of each of its 44
+// runs.  With 8 vectors a thread (32768 keys of 8 bits, 16384 of 16, 8192 of
+// 32; 80 registers, 3 CTAs an SM) they serve twice as many, and the runs are
+// twice as long.  Measured (GB300), whole builds: 2^30 bytes, both structures
+// of 8 levels, 5.55 -> 5.00 ms; 2^28 16-bit symbols, 16 levels, 4.79 -> 4.40;
+// 2^26 32-bit symbols, the matrix of 20 levels, 1.87 -> 1.64 (with 4 CTAs an SM
+// at 64 registers 16-bit 4.55, 32-bit 1.72).  Texts too short to fill the SMs
+// with such tiles keep the usual ones.
+#include "kernels.cuh"
+#include "tile_launch.cuh"
+
+namespace pwmgpu {
+
+namespace {
+template <typename KeyT, typename KeyO>
+void launch(const TileArgs& a, cudaStream_t s) {
+  launch_tile_one<KeyT, kTileMaxLevels, true, KeyO, false, 2 * kTileVectors>(a, s);
+}
+}  // namespace
+
+void launch_tile_pass_wide(uint32_t key_bytes, uint32_t out_bytes, const TileArgs& a, cudaStream_t s) {
+  if (key_bytes == 1) launch<uint8_t, uint8_t>(a, s);
+  else if (key_bytes == 2 && out_bytes == 1) launch<uint16_t, uint8_t>(a, s);
+  else if (key_bytes == 2) launch<uint16_t, uint16_t>(a, s);
+  else if (out_bytes == 1) launch<uint32_t, uint8_t>(a, s);
+  else if (out_bytes == 2) launch<uint32_t, uint16_t>(a, s);
+  else launch<uint32_t, uint32_t>(a, s);
+}
+
+}  // namespace pwmgpu
