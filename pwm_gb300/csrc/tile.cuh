@@ -161,7 +161,7 @@ struct TileCfg {
   // the bit-plane form (tile_pass_body with PLANES): two sets of K planes, a
   // zero count per plane word, the 256-entry compress table, then the deep
   // records
-  static constexpr size_t plane_area() { return size_t(2) * K * SBW * 4 + size_t(T / 32) * 4 + 256 * 4; }
+  static constexpr size_t plane_area() { return size_t(2) * K * SBW * 4 + size_t(T / 32) * 4 + 256 * 8; }
   static constexpr size_t plane_smem_bytes() { return plane_area() + deep_bytes(); }
 };
 
@@ -600,11 +600,15 @@ __device__ __forceinline__ void bulk_load_tile(void* dst, const void* src, uint3
 // together; the move masks of a byte depend on its mask byte only and come
 // from a 256-entry table, so a mask word costs four table reads and a byte
 // transpose, once per word and polarity, for every plane that moves.
+// Both the moves (as multiply-adds) and the making of the planes (as
+// transposes of 32 keys) are counted in instructions: they bound the kernel.
+// The last pass of 2^28 keys, 4 levels of both structures, 419 -> 374 us,
+// of 2^25 67 -> 58; 2^26 symbols of 2 levels 67 -> 62 us the whole build.
 
-// Table entry of mask byte b: the move masks of compress toward bit 7 inside
-// the byte (Hacker's Delight 7-4 with every shift mirrored: round i moves the
-// selected bits whose remaining distance has bit i set) in bytes 0-2, the
-// number of selected bits in byte 3.
+// The move masks of mask byte b: compress toward bit 7 inside the byte
+// (Hacker's Delight 7-4 with every shift mirrored: round i moves the selected
+// bits whose remaining distance has bit i set) in bytes 0-2, the number of
+// selected bits in byte 3.
 __device__ __forceinline__ uint32_t compress_lut_entry(uint32_t b) {
   uint32_t m = b, mk = (~b & 0xFFu) >> 1, e = uint32_t(__popc(b)) << 24;
 #pragma unroll
@@ -619,33 +623,34 @@ __device__ __forceinline__ uint32_t compress_lut_entry(uint32_t b) {
   }
   return e;
 }
-// The byte move masks of mask word m (mv[0..2], byte k from the entry of mask
-// byte k: a 4x4 byte transpose of the four entries) and the shifts that join
-// the byte pieces (mv[3..5] for bytes 2, 1, 0: the bits not selected in the
-// bytes above, summed from the top by one multiply).
-__device__ __forceinline__ void compress_masks(const uint32_t* lut, uint32_t m, uint32_t (&mv)[6]) {
-  const uint32_t e0 = lut[m & 0xFFu], e1 = lut[(m >> 8) & 0xFFu], e2 = lut[(m >> 16) & 0xFFu], e3 = lut[m >> 24];
+// The byte move masks of a mask word whose bytes 0..3 have the entries
+// e0..e3 (mv[0..2], byte k from e_k: a 4x4 byte transpose) and the powers of
+// two that join the byte pieces (mv[3..5] for bytes 2, 1, 0: as many places
+// as bits are not selected in the bytes above, summed from the top by one
+// multiply).
+__device__ __forceinline__ void compress_masks(uint32_t e0, uint32_t e1, uint32_t e2, uint32_t e3, uint32_t (&mv)[6]) {
   const uint32_t l01 = __byte_perm(e0, e1, 0x5140), l23 = __byte_perm(e2, e3, 0x5140);
   const uint32_t h01 = __byte_perm(e0, e1, 0x7362), h23 = __byte_perm(e2, e3, 0x7362);
   mv[0] = __byte_perm(l01, l23, 0x5410);
   mv[1] = __byte_perm(l01, l23, 0x7632);
   mv[2] = __byte_perm(h01, h23, 0x5410);
   const uint32_t sh = __byte_perm(0x08080808u - __byte_perm(h01, h23, 0x7632), 0u, 0x0123) * 0x01010101u;
-  mv[3] = sh & 0xFFu;
-  mv[4] = (sh >> 8) & 0xFFu;
-  mv[5] = (sh >> 16) & 0xFFu;
+  // shifts of 0..24 in bytes 0..2: the wrapping shift takes each byte's low 5 bits
+  mv[3] = __funnelshift_l(0u, 1u, sh);
+  mv[4] = __funnelshift_l(0u, 1u, sh >> 8);
+  mv[5] = __funnelshift_l(0u, 1u, sh >> 16);
 }
 
 // The bits of x under m, in order, packed to the top of the word (mv: the
-// masks of m).
+// masks of m).  A move by k places of t, a part of x, to places free in x is
+// x + t * (2^k - 1): multiply-adds, which have a pipe of their own beside the
+// shifts and logic that bound these kernels.
 __device__ __forceinline__ uint32_t compress_apply(uint32_t x, uint32_t m, const uint32_t (&mv)[6]) {
   x &= m;
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    const uint32_t t = x & mv[i];
-    x = (x ^ t) | (t << (1 << i));
-  }
-  return (x & 0xFF000000u) | ((x & 0x00FF0000u) << mv[3]) | ((x & 0x0000FF00u) << mv[4]) | ((x & 0xFFu) << mv[5]);
+  x += x & mv[0];
+  x += (x & mv[1]) * 3u;
+  x += (x & mv[2]) * 15u;
+  return (x & 0xFFu) * mv[5] + ((x & 0xFF00u) * mv[4] + ((x & 0xFF0000u) * mv[3] + (x & 0xFF000000u)));
 }
 
 // OR the top `len` bits of v into a zeroed shared bit stream at bit `pos`
@@ -682,6 +687,42 @@ __device__ __forceinline__ void warp_exclusive_scan(const uint32_t* in, uint32_t
   }
 }
 
+// Planes of 32 keys of one byte (key i in byte i % 4 of w[i / 4]): pl[j] has
+// bit lo + K-1-j of key i in bit 31-i.  A byte transpose puts the keys of
+// every eighth place into one word, then 4x4 bit transposes inside its
+// nibbles: 44 operations for 4 planes.  lo + K <= 8.
+template <int K>
+__device__ __forceinline__ void key_planes(const uint32_t (&w)[8], uint32_t lo, uint32_t (&pl)[K]) {
+  uint32_t x[8];  // byte 3-q of x[j]: key 8q + j
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t l02 = __byte_perm(w[2 + h], w[h], 0x5140), h02 = __byte_perm(w[2 + h], w[h], 0x7362);
+    const uint32_t l46 = __byte_perm(w[6 + h], w[4 + h], 0x5140), h46 = __byte_perm(w[6 + h], w[4 + h], 0x7362);
+    x[4 * h] = __byte_perm(l46, l02, 0x5410);
+    x[4 * h + 1] = __byte_perm(l46, l02, 0x7632);
+    x[4 * h + 2] = __byte_perm(h46, h02, 0x5410);
+    x[4 * h + 3] = __byte_perm(h46, h02, 0x7632);
+  }
+#pragma unroll
+  for (int b0 = 0; b0 < K; b0 += 4) {  // key bits lo + b0 .. lo + b0 + 3
+    uint32_t n[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t hi = K == 4 ? x[j] << (4 - lo) : (x[j] >> (lo + b0)) << 4;
+      n[j] = (hi & 0xF0F0F0F0u) | ((x[4 + j] >> (lo + b0)) & 0x0F0F0F0Fu);
+    }
+    const uint32_t a0 = (n[0] & 0xCCCCCCCCu) | ((n[2] >> 2) & 0x33333333u);
+    const uint32_t a2 = ((n[0] << 2) & 0xCCCCCCCCu) | (n[2] & 0x33333333u);
+    const uint32_t a1 = (n[1] & 0xCCCCCCCCu) | ((n[3] >> 2) & 0x33333333u);
+    const uint32_t a3 = ((n[1] << 2) & 0xCCCCCCCCu) | (n[3] & 0x33333333u);
+    const uint32_t bit[4] = {((a2 << 1) & 0xAAAAAAAAu) | (a3 & 0x55555555u), (a2 & 0xAAAAAAAAu) | ((a3 >> 1) & 0x55555555u),
+                             ((a0 << 1) & 0xAAAAAAAAu) | (a1 & 0x55555555u), (a0 & 0xAAAAAAAAu) | ((a1 >> 1) & 0x55555555u)};
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+      if (b0 + b < K) pl[K - 1 - b0 - b] = bit[b];
+  }
+}
+
 // The load and the splits of a tile in bit-plane form (tile_pass_body with
 // PLANES; 1-byte keys, no S_{l+K}).  Leaves the streams of levels l..l+K-1
 // (plane j of set j % 2), the run sizes and starts of key_1..key_D, and the
@@ -710,8 +751,9 @@ __device__ __forceinline__ void tile_planes_splits(const TileArgs& a, const Tile
   const uint32_t NWt = BATCH ? uint32_t(THREADS * VP / 2) : uint32_t(NW);  // plane words of this tile
   const int wpt = BATCH ? (VP >= 2 ? VP / 2 : 1) : WPT;                     // of them per thread
   uint32_t* zpos = sbits + 2 * K * SBW;  // zeros before each plane word, current split
-  uint32_t* s_clut = zpos + NW;          // compress table
-  for (int b = tid; b < 256; b += THREADS) s_clut[b] = compress_lut_entry(uint32_t(b));
+  uint2* s_clut = reinterpret_cast<uint2*>(zpos + NW);  // compress table: a byte's ones, its zeros
+  for (int b = tid; b < 256; b += THREADS)
+    s_clut[b] = make_uint2(compress_lut_entry(uint32_t(b)), compress_lut_entry(uint32_t(b) ^ 0xFFu));
   const uint32_t nfull = n >> 5, nrem = n & 31;
   auto word_valid = [&](uint32_t w) -> uint32_t {
     return w < nfull ? ~0u : ((w == nfull && nrem) ? ~0u << (32 - nrem) : 0u);
@@ -738,43 +780,44 @@ __device__ __forceinline__ void tile_planes_splits(const TileArgs& a, const Tile
     const uint32_t nvec = (n + 15) >> 4;
     const uint32_t last_block = uint32_t((uint64_t(off) + n + 15) >> 4) - 1;  // last aligned block holding tile bytes
     const uint32_t lo = shift - uint32_t(K - 1);  // plane j is key bit lo + K-1-j
-#pragma unroll
-    for (int r = 0; r < V; ++r) {
-      if (BATCH && r >= VP) break;  // uniform over the CTA
-      const int gv = (warp * VP + r) * 32 + lane;
+    // two rounds of vectors at a time: lanes in pairs exchange halves, so that
+    // an even lane has both vectors of a plane word of the first round, its odd
+    // neighbour those of the second
+    const bool odd = lane & 1;
+    auto load = [&](int gv) -> uint4 {
       uint4 kv = make_uint4(0u, 0u, 0u, 0u);
       if (uint32_t(gv) < nvec) {
-        const uint4 x0 = __ldcs(av + gv);
-        if (off == 0) {
-          kv = x0;
-        } else {
+        kv = __ldcs(av + gv);
+        if (off) {
           const uint4 x1 = uint32_t(gv) + 1 <= last_block ? __ldcs(av + gv + 1) : make_uint4(0u, 0u, 0u, 0u);
-          kv = realign16(x0, x1, off);
+          kv = realign16(kv, x1, off);
         }
       }
-      const int rem = int(n) - gv * 16;
-      const int nvv = rem >= 16 ? 16 : (rem > 0 ? rem : 0);
-      const uint32_t vm = 0xFFFFu & ~((1u << (16 - nvv)) - 1u);  // valid keys, key 0 in bit 15
-      const uint32_t w0 = kv.x >> lo, w1 = kv.y >> lo, w2 = kv.z >> lo, w3 = kv.w >> lo;
-      uint32_t b[K];
+      return kv;
+    };
 #pragma unroll
-      for (int j = 0; j < K; ++j)
-        b[j] = __byte_perm(key_bits8(w2, w3, K - 1 - j), key_bits8(w0, w1, K - 1 - j), 0x0040) & vm;
-      // an even lane's vector is the upper half of the plane word, its odd
-      // neighbour's the lower half: one shuffle per two planes
-      const uint32_t pwi = uint32_t(gv) >> 1;
+    for (int r = 0; r < V; r += 2) {
+      if (BATCH && r >= VP) break;  // uniform over the CTA
+      const int gv = (warp * VP + r) * 32 + lane;
+      const bool two = !BATCH || r + 1 < VP;
+      const uint4 a0 = load(gv), a1 = two ? load(gv + 32) : make_uint4(0u, 0u, 0u, 0u);
+      uint32_t w[8];
+      {
+        const uint32_t m0[4] = {a0.x, a0.y, a0.z, a0.w}, m1[4] = {a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-      for (int j = 0; j < K; j += 2) {
-        if (j + 1 < K) {
-          const uint32_t odd = __shfl_down_sync(0xFFFFFFFFu, b[j] | (b[j + 1] << 16), 1);
-          if (!(lane & 1)) {
-            sbits[j * SBW + pwi] = (b[j] << 16) | (odd & 0xFFFFu);
-            sbits[(j + 1) * SBW + pwi] = (b[j + 1] << 16) | (odd >> 16);
-          }
-        } else {
-          const uint32_t odd = __shfl_down_sync(0xFFFFFFFFu, b[j], 1);
-          if (!(lane & 1)) sbits[j * SBW + pwi] = (b[j] << 16) | odd;
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t x = __shfl_xor_sync(0xFFFFFFFFu, odd ? m0[q] : m1[q], 1);
+          w[q] = odd ? x : m0[q];
+          w[4 + q] = odd ? m1[q] : x;
         }
+      }
+      const uint32_t pwi = (uint32_t(gv) >> 1) + (odd ? 16u : 0u);
+      uint32_t pl[K];
+      key_planes<K>(w, lo, pl);
+      const uint32_t vm = word_valid(pwi);
+      if (two || !odd) {
+#pragma unroll
+        for (int j = 0; j < K; ++j) sbits[j * SBW + pwi] = pl[j] & vm;
       }
     }
   }
@@ -881,12 +924,17 @@ __device__ __forceinline__ void tile_planes_splits(const TileArgs& a, const Tile
 #pragma unroll
       for (int p = s + 1; p < K; ++p) Pc[p * SBW + w] = 0u;  // read above; set again two splits on
       if (s + 1 < K) {
-        const uint32_t mz = ~m[k] & vmk[k], mo = m[k];
+        // (keys past the tile's end count as zeros after its last one: their bits are 0)
+        const uint32_t mo = m[k], mz = ~mo;
         const uint32_t nz = zc[k], no = __popc(mo);
         const uint32_t opos = ztot + 32u * w - zp;  // every word before w is whole
         uint32_t mvz[6], mvo[6];
-        compress_masks(s_clut, mz, mvz);
-        compress_masks(s_clut, mo, mvo);
+        {
+          const uint2 e0 = s_clut[mo & 0xFFu], e1 = s_clut[(mo >> 8) & 0xFFu], e2 = s_clut[(mo >> 16) & 0xFFu],
+                      e3 = s_clut[mo >> 24];
+          compress_masks(e0.x, e1.x, e2.x, e3.x, mvo);
+          compress_masks(e0.y, e1.y, e2.y, e3.y, mvz);
+        }
 #pragma unroll
         for (int p = s + 1; p < K; ++p) {
           or_stream_bits(Pn + p * SBW, zp, compress_apply(pw[p][k], mz, mvz), nz);
