@@ -37,13 +37,15 @@
 //   * writes every run of every level to the matrix and the tree at
 //     table start + look-back prefix in 64-bit words, and the runs of
 //     S_{l+K} to the next pass's input (one warp per run, round-robin; the
-//     level words word-parallel in passes of 5-8 levels and over 2- and
-//     4-byte keys).
+//     level words word-parallel in passes of 5-8 levels and of 2- and 4-byte
+//     keys split bit by bit).
 // A pass that writes no S_{l+K} over 1-byte keys (the last pass of every
 // text whose remaining levels fit a byte) runs the splits on bit planes
 // instead (tile_planes_splits): the K bits of every key as K planes of 32-key
 // words, each split a stable partition of the later planes' words; the
-// streams of the levels are then the planes themselves.
+// streams of the levels are then the planes themselves.  A pass of 4 levels
+// that does write S_{l+K} makes its streams the same way and sorts the keys by
+// all 4 bits at once (tile_rank_keys), where a thread has 32 keys or more.
 #pragma once
 
 #include "common.cuh"
@@ -125,7 +127,7 @@ struct TileCfg {
   static constexpr int WARPS = THREADS / 32;
   static constexpr int WSLICE = 32 * ITEMS;              // keys per warp
   static constexpr int NVEC = THREADS * V;               // vectors per tile
-  static constexpr int SBW = T / 32 + 2;                 // stream words per level (+2 for funnel reads)
+  static constexpr int SBW = T / 32 + 4;                 // stream words per level (+2 for funnel reads, +2 to align)
   static constexpr int NLB = 1 << D;                     // look-back counters per tile
   static constexpr int LPC = 32 / KPL;                   // lanes per 32-bit stream word
   static_assert(T <= 32768, "zero counts are packed in 16 bits");
@@ -149,20 +151,30 @@ struct TileCfg {
   }
   // Levels 1..K-1 written word-parallel (tile_pass_body): passes of 5..8
   // levels (levels 1..JW still a warp per run), and passes over 2- and
-  // 4-byte keys, whose smaller tiles give runs too short for a warp each
-  // (measured: 16-bit, 16 levels 4.48 -> 4.38 ms of passes; 32-bit, 20 levels
-  // 1.64 -> 1.58; slower over 1-byte keys: 4.71 -> 4.80 ms at 8 levels).
+  // 4-byte keys split bit by bit, whose small tiles give runs too short for a
+  // warp each (in the ranked form a warp a run is faster: passes of 2^26 16-bit
+  // keys 217 us word-parallel, 211; of 2^28 8-bit keys 579 and 517).
   static constexpr bool WORD_PARALLEL = K > kTileMaxLevels || (K > 1 && sizeof(KeyT) > 1);
   static constexpr int JW = K > kTileMaxLevels ? 3 : 0;
   // run records and word prefixes of the word-parallel writes
   static constexpr size_t deep_bytes() {
     return WORD_PARALLEL ? size_t(2 * ((1 << K) - 2)) * 16 + size_t(2 * (K - 1 - JW)) * ((1 << (K - 1)) + 1) * 4 : 0;
   }
-  // the bit-plane form (tile_pass_body with PLANES): two sets of K planes, a
-  // zero count per plane word, the 256-entry compress table, then the deep
-  // records
-  static constexpr size_t plane_area() { return size_t(2) * K * SBW * 4 + size_t(T / 32) * 4 + 256 * 8; }
+  // the bit-plane form (tile_pass_body with PLANES): two sets of K planes, the
+  // 256-entry compress table, then the deep records
+  static constexpr size_t plane_area() { return ((size_t(2) * K * SBW * 4 + 15) & ~size_t(15)) + 256 * 8; }
   static constexpr size_t plane_smem_bytes() { return plane_area() + deep_bytes(); }
+  // the ranked form (passes of 4 levels that write S_{l+4}, at least 32 keys
+  // a thread): the keys, the planes of set 0, the planes of set 1 (before the
+  // splits: a cursor per digit and thread), the compress table
+  static constexpr bool RANKABLE = OUT && K == 4 && V * KPL >= 32;
+  static constexpr size_t cursor_area() { return size_t(1 << K) * THREADS * 4; }
+  static constexpr size_t ranked_sets() {
+    const size_t set = size_t(K) * SBW * 4;
+    return (set + (set > cursor_area() ? set : cursor_area()) + 15) & ~size_t(15);
+  }
+  static constexpr size_t ranked_area() { return size_t(T) * sizeof(KeyT) + ranked_sets() + 256 * 8; }
+  static constexpr size_t ranked_smem_bytes() { return ranked_area(); }
 };
 
 // Bit q of the 8 keys of w0 (keys 0-3, key k in byte k) and w1 (keys 4-7),
@@ -609,9 +621,9 @@ __device__ __forceinline__ void bulk_load_tile(void* dst, const void* src, uint3
 // (Hacker's Delight 7-4 with every shift mirrored: round i moves the selected
 // bits whose remaining distance has bit i set) in bytes 0-2, the number of
 // selected bits in byte 3.
-__device__ __forceinline__ uint32_t compress_lut_entry(uint32_t b) {
-  uint32_t m = b, mk = (~b & 0xFFu) >> 1, e = uint32_t(__popc(b)) << 24;
-#pragma unroll
+constexpr uint32_t compress_lut_entry(uint32_t b) {
+  uint32_t m = b, mk = (~b & 0xFFu) >> 1, e = 0;
+  for (int i = 0; i < 8; ++i) e += ((b >> i) & 1u) << 24;
   for (int i = 0; i < 3; ++i) {
     uint32_t mp = mk ^ (mk >> 1);
     mp ^= mp >> 2;
@@ -623,6 +635,19 @@ __device__ __forceinline__ uint32_t compress_lut_entry(uint32_t b) {
   }
   return e;
 }
+// Per byte: the entry of its ones, the entry of its zeros.
+struct CompressLut {
+  uint2 e[256];
+};
+constexpr CompressLut make_compress_lut() {
+  CompressLut l{};
+  for (uint32_t b = 0; b < 256; ++b) {
+    l.e[b].x = compress_lut_entry(b);
+    l.e[b].y = compress_lut_entry(b ^ 0xFFu);
+  }
+  return l;
+}
+__device__ const CompressLut kCompressLut = make_compress_lut();
 // The byte move masks of a mask word whose bytes 0..3 have the entries
 // e0..e3 (mv[0..2], byte k from e_k: a 4x4 byte transpose) and the powers of
 // two that join the byte pieces (mv[3..5] for bytes 2, 1, 0: as many places
@@ -723,53 +748,59 @@ __device__ __forceinline__ void key_planes(const uint32_t (&w)[8], uint32_t lo, 
   }
 }
 
-// The load and the splits of a tile in bit-plane form (tile_pass_body with
-// PLANES; 1-byte keys, no S_{l+K}).  Leaves the streams of levels l..l+K-1
-// (plane j of set j % 2), the run sizes and starts of key_1..key_D, and the
-// finest-run counts (counted and published for the look-back, or given).
-// Per split s the thread owning plane words [tid * WPT, (tid + 1) * WPT)
-// reads its words of plane s (the split bit, in S_{l+s} order) and of the
-// later planes, scans the zero counts over the CTA, and ORs the compressed
-// zero and one parts of each later plane into the other set at the word's
-// zero and one cursors; its own words of the read set are then cleared for
-// the split after next.  BATCH: the tile has VP <= V vectors per thread, so
-// NWt = THREADS * VP / 2 plane words, max(VP / 2, 1) per thread (VP = 1:
-// the first half of the threads own one word each); the words above NWt stay
-// zero.
+// The W (1, 2 or 4) plane words of a thread, aligned: one load.
+template <int W>
+__device__ __forceinline__ void plane_words(const uint32_t* plane, int tid, uint32_t (&w)[W]) {
+  if constexpr (W == 4) {
+    const uint4 x = reinterpret_cast<const uint4*>(plane)[tid];
+    w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
+  } else if constexpr (W == 2) {
+    const uint2 x = reinterpret_cast<const uint2*>(plane)[tid];
+    w[0] = x.x, w[1] = x.y;
+  } else {
+    static_assert(W == 1, "a word, or an aligned vector of them");
+    w[0] = plane[tid];
+  }
+}
+template <int W>
+__device__ __forceinline__ void clear_plane_words(uint32_t* plane, int tid) {
+  if constexpr (W == 4) reinterpret_cast<uint4*>(plane)[tid] = make_uint4(0u, 0u, 0u, 0u);
+  else if constexpr (W == 2) reinterpret_cast<uint2*>(plane)[tid] = make_uint2(0u, 0u);
+  else plane[tid] = 0u;
+}
+
+// Bits of plane word w that belong to a tile of n keys.
+__device__ __forceinline__ uint32_t plane_word_valid(uint32_t n, uint32_t w) {
+  const uint32_t nfull = n >> 5, nrem = n & 31;
+  return w < nfull ? ~0u : ((w == nfull && nrem) ? ~0u << (32 - nrem) : 0u);
+}
+
+// The load of a tile in bit-plane form (tile_pass_body with PLANES; 1-byte
+// keys, no S_{l+K}): its planes in text order (set 0) and the counts of its
+// finest runs (counted and published for the look-back, or given).  BATCH:
+// the tile has VP <= V vectors per thread, so NWt = THREADS * VP / 2 plane
+// words; the words above NWt stay zero.
 template <int K, int THREADS, int V, bool BATCH>
-__device__ __forceinline__ void tile_planes_splits(const TileArgs& a, const TileText& s_tx, const TileSeg& s_sg,
-                                                   uint32_t g, uint32_t tl, uint64_t tstart, uint32_t n, int VP,
-                                                   uint32_t shift, bool given, uint32_t* sbits, uint32_t* s_cnt,
-                                                   unsigned long long* pre, uint32_t* s_wz, uint32_t* s_ztot,
-                                                   uint32_t (*rsz)[1 << (K - 1)], uint32_t (*rst)[1 << (K - 1)]) {
+__device__ __forceinline__ void tile_planes_load(const TileArgs& a, const TileText& s_tx, const TileSeg& s_sg,
+                                                 uint32_t g, uint32_t tl, uint64_t tstart, uint32_t n, int VP,
+                                                 uint32_t shift, bool given, uint32_t* sbits, uint32_t* s_cnt,
+                                                 unsigned long long* pre) {
   using C = TileCfg<uint8_t, K, false, THREADS, V>;
   constexpr int D = C::D, T = C::T, WARPS = C::WARPS, SBW = C::SBW, NLB = C::NLB;
   constexpr int NW = T / 32;         // plane words of a tile of V vectors per thread
   constexpr int WPT = NW / THREADS;  // plane words per thread in the splits
-  static_assert(K >= 1 && K <= kTileGivenMaxLevels && WPT * THREADS == NW, "up to 8 levels; whole words per thread");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t NWt = BATCH ? uint32_t(THREADS * VP / 2) : uint32_t(NW);  // plane words of this tile
   const int wpt = BATCH ? (VP >= 2 ? VP / 2 : 1) : WPT;                     // of them per thread
-  uint32_t* zpos = sbits + 2 * K * SBW;  // zeros before each plane word, current split
-  uint2* s_clut = reinterpret_cast<uint2*>(zpos + NW);  // compress table: a byte's ones, its zeros
-  for (int b = tid; b < 256; b += THREADS)
-    s_clut[b] = make_uint2(compress_lut_entry(uint32_t(b)), compress_lut_entry(uint32_t(b) ^ 0xFFu));
-  const uint32_t nfull = n >> 5, nrem = n & 31;
-  auto word_valid = [&](uint32_t w) -> uint32_t {
-    return w < nfull ? ~0u : ((w == nfull && nrem) ? ~0u << (32 - nrem) : 0u);
-  };
+  auto word_valid = [&](uint32_t w) { return plane_word_valid(n, w); };
 
   // set 1 and the words of set 0 above the tile's start cleared
   for (int i = tid; i < K * SBW; i += THREADS) sbits[K * SBW + i] = 0u;
   if (BATCH && NWt < uint32_t(NW)) {
     const uint32_t pad = uint32_t(SBW) - NWt;
     for (uint32_t i = tid; i < K * pad; i += THREADS) sbits[(i / pad) * SBW + NWt + i % pad] = 0u;
-  } else if (tid < 2 * K) {
-    sbits[(tid >> 1) * SBW + NW + (tid & 1)] = 0u;
-  }
-  if (tid == 0) {
-    rsz[0][0] = n;
-    rst[0][0] = 0;
+  } else if (tid < 4 * K) {
+    sbits[(tid >> 2) * SBW + NW + (tid & 3)] = 0u;
   }
 
   // ---- load; planes 0..K-1 in text order (set 0) ---------------------------
@@ -835,12 +866,14 @@ __device__ __forceinline__ void tile_planes_splits(const TileArgs& a, const Tile
       if (tid == 0) atomicOr(a.status, kErrBounds);
       for (int c = tid; c < NLB; c += THREADS) s_cnt[c] = 0, pre[c] = 0;
     } else {
-      // per-warp counts in the zero-count words (first written after split 0's barrier)
-      uint32_t (*s_wcnt)[NLB] = reinterpret_cast<uint32_t (*)[NLB]>(zpos);
-      static_assert(WARPS * NLB <= NW, "the counts fit the zero-count words");
-      uint32_t cnt[NLB];
+      __shared__ uint32_t s_wcnt[WARPS][NLB];
+      uint32_t cnt[NLB], words[D][WPT];
 #pragma unroll
       for (int c = 0; c < NLB; ++c) cnt[c] = 0;
+      if constexpr (!BATCH) {
+#pragma unroll
+        for (int t = 0; t < D; ++t) plane_words<WPT>(sbits + t * SBW, tid, words[t]);
+      }
 #pragma unroll
       for (int k = 0; k < WPT; ++k) {
         if (BATCH && k >= wpt) break;
@@ -848,7 +881,7 @@ __device__ __forceinline__ void tile_planes_splits(const TileArgs& a, const Tile
         const uint32_t vmk = word_valid(w);  // 0 above the tile's words
         uint32_t pl[D];
 #pragma unroll
-        for (int t = 0; t < D; ++t) pl[t] = sbits[t * SBW + w];
+        for (int t = 0; t < D; ++t) pl[t] = BATCH ? sbits[t * SBW + w] : words[t][k];
 #pragma unroll
         for (int c = 0; c < NLB; ++c) {
           uint32_t mt = vmk;
@@ -872,23 +905,111 @@ __device__ __forceinline__ void tile_planes_splits(const TileArgs& a, const Tile
       }
     }
   }
+}
 
-  // ---- the splits -------------------------------------------------------------
+// Sizes and starts of the runs of key_1..key_D from the counts of key_D's (in
+// tile order, key_j has level l least significant: a run of key_j is the
+// finest runs whose low j bits are its own).  Counts that do not make up the
+// tile: kErrBounds, and no run is written.
+template <int D>
+__device__ __forceinline__ void tile_run_sizes(const uint32_t* s_cnt, uint32_t n, uint32_t (*rsz)[1 << D],
+                                               uint32_t (*rst)[1 << D], uint32_t* status) {
+  static_assert(D <= kTileMaxLevels, "at most 16 finest runs");
+  const int e = int(threadIdx.x) + 2;  // run v of key_j: 2^j + v
+  if (e >= (2 << D)) return;
+  const int j = 31 - __clz(e), v = e - (1 << j);
+  uint32_t size = 0, start = 0, total = 0;
 #pragma unroll
-  for (int s = 0; s < D; ++s) {
+  for (int c = 0; c < (1 << D); ++c) {
+    const uint32_t x = s_cnt[c];
+    const int u = c & ((1 << j) - 1);
+    size += u == v ? x : 0u;
+    start += u < v ? x : 0u;
+    total += x;
+  }
+  if (total != n) {
+    if (e == 2) atomicOr(status, kErrBounds);
+    size = start = 0;
+  }
+  rsz[j][v] = size;
+  rst[j][v] = start;
+}
+// The same for up to 128 finest runs, by the whole CTA.
+template <int D, int WARPS>
+__device__ __forceinline__ void tile_run_sizes_deep(const uint32_t* s_cnt, uint32_t n, uint32_t (*rsz)[1 << D],
+                                                    uint32_t (*rst)[1 << D], uint32_t* status) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int c = tid; c < (1 << D); c += 32 * WARPS) rsz[D][c] = s_cnt[c];
+  __syncthreads();
+  if (warp == 0) {
+    for (int j = D - 1; j >= 1; --j) {
+      for (int v = lane; v < (1 << j); v += 32) rsz[j][v] = rsz[j + 1][v] + rsz[j + 1][v + (1 << j)];
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  const bool wrong = rsz[1][0] + rsz[1][1] != n;
+  __syncthreads();
+  if (wrong) {
+    if (tid == 0) atomicOr(status, kErrBounds);
+    for (int i = tid; i < (D + 1) << D; i += 32 * WARPS) rsz[i >> D][i & ((1 << D) - 1)] = 0;
+    __syncthreads();
+  }
+  for (int j = 1 + warp; j <= D; j += WARPS) warp_exclusive_scan(rsz[j], rst[j], 1 << j, lane);
+  __syncthreads();
+}
+
+// The splits of a tile's K planes (set 0, in text order; the streams of levels
+// l..l+K-1 are plane j of set j % 2 afterwards) and, from the counts of the
+// D-level runs in s_cnt (visible after the first barrier here), the run sizes.
+// Per split s the thread owning plane words [tid * WPT, (tid + 1) * WPT) reads
+// its words of plane s (the split bit, in S_{l+s} order) and of the later
+// planes, scans the zero counts over the CTA, and ORs the compressed zero and
+// one parts of each later plane into the other set at the word's zero and one
+// cursors; its own words of the read set are cleared for the split after next.
+// V: 16-byte vectors of 1-byte keys that fill the planes.  BATCH: max(VP / 2,
+// 1) words a thread (VP = 1: the first half of the threads own one word each).
+template <int K, int D, int THREADS, int V, bool BATCH>
+__device__ __forceinline__ void tile_planes_splits(uint32_t n, int VP, uint32_t* sbits, uint2* s_clut,
+                                                   const uint32_t* s_cnt, uint32_t* s_wz, uint32_t (*rsz)[1 << D],
+                                                   uint32_t (*rst)[1 << D], uint32_t* status) {
+  using C = TileCfg<uint8_t, K, false, THREADS, V>;
+  constexpr int WARPS = C::WARPS, SBW = C::SBW;
+  constexpr int NW = C::T / 32, WPT = NW / THREADS;
+  static_assert(K >= 1 && K <= kTileGivenMaxLevels && WPT * THREADS == NW, "up to 8 levels; whole words per thread");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wpt = BATCH ? (VP >= 2 ? VP / 2 : 1) : WPT;
+  for (int b = tid; b < 256; b += THREADS) s_clut[b] = kCompressLut.e[b];
+  if (tid == 0) {
+    rsz[0][0] = n;
+    rst[0][0] = 0;
+  }
+  uint32_t zeros[K];
+#pragma unroll
+  for (int s = 0; s < K - 1; ++s) {
     uint32_t* Pc = sbits + (s & 1) * K * SBW;        // planes in S_{l+s} order
     uint32_t* Pn = sbits + ((s & 1) ^ 1) * K * SBW;  // planes s+1.. in S_{l+s+1} order
     uint32_t m[WPT], vmk[WPT], zc[WPT], pw[K][WPT];
     uint32_t tsum = 0;
+    if constexpr (!BATCH) {  // a thread's words are one aligned vector; read, and cleared for the split after next
+      plane_words<WPT>(Pc + s * SBW, tid, m);
+#pragma unroll
+      for (int p = s + 1; p < K; ++p) {
+        plane_words<WPT>(Pc + p * SBW, tid, pw[p]);
+        clear_plane_words<WPT>(Pc + p * SBW, tid);
+      }
+    }
 #pragma unroll
     for (int k = 0; k < WPT; ++k) {
       const uint32_t w = uint32_t(tid) * wpt + k;  // < NW: every word read is inside the planes
-      vmk[k] = (BATCH && k >= wpt) ? 0u : word_valid(w);
-      m[k] = (BATCH && k >= wpt) ? 0u : Pc[s * SBW + w];
+      vmk[k] = (BATCH && k >= wpt) ? 0u : plane_word_valid(n, w);
+      if constexpr (BATCH) {
+        m[k] = k >= wpt ? 0u : Pc[s * SBW + w];
+#pragma unroll
+        for (int p = s + 1; p < K; ++p) pw[p][k] = k >= wpt ? 0u : Pc[p * SBW + w];
+      }
       zc[k] = __popc(~m[k] & vmk[k]);
       tsum += zc[k];
-#pragma unroll
-      for (int p = s + 1; p < K; ++p) pw[p][k] = (BATCH && k >= wpt) ? 0u : Pc[p * SBW + w];
     }
     uint32_t x = tsum;
 #pragma unroll
@@ -905,24 +1026,19 @@ __device__ __forceinline__ void tile_planes_splits(const TileArgs& a, const Tile
       ztot += z;
       zpre += w < warp ? z : 0u;
     }
-    if (tid == 0) *s_ztot = ztot;
-    if constexpr (K > kTileMaxLevels) {  // up to 64 runs: a warp scan
-      if (s >= 2 && warp == 0) warp_exclusive_scan(rsz[s], rst[s], 1 << s, lane);
-    } else if (s >= 2 && tid == 0) {
-      uint32_t run = 0;
-      for (int v = 0; v < (1 << s); ++v) {
-        rst[s][v] = run;
-        run += rsz[s][v];
-      }
+    zeros[s] = ztot;
+    if (s == 0) {
+      if constexpr (D >= 1 && D <= kTileMaxLevels) tile_run_sizes<D>(s_cnt, n, rsz, rst, status);
     }
     uint32_t zp = zpre + x - tsum;  // zeros before this thread's first word
 #pragma unroll
     for (int k = 0; k < WPT; ++k) {
       if (BATCH && k >= wpt) break;
       const uint32_t w = uint32_t(tid) * wpt + k;
-      zpos[w] = zp;
+      if constexpr (BATCH) {
 #pragma unroll
-      for (int p = s + 1; p < K; ++p) Pc[p * SBW + w] = 0u;  // read above; set again two splits on
+        for (int p = s + 1; p < K; ++p) Pc[p * SBW + w] = 0u;  // read above; set again two splits on
+      }
       if (s + 1 < K) {
         // (keys past the tile's end count as zeros after its last one: their bits are 0)
         const uint32_t mo = m[k], mz = ~mo;
@@ -944,26 +1060,201 @@ __device__ __forceinline__ void tile_planes_splits(const TileArgs& a, const Tile
       zp += zc[k];
     }
     __syncthreads();  // (B)
-    // ---- run sizes of key_{s+1} -------------------------------------------
-    if (s == 0) {
-      if (tid == 0) {
-        rsz[1][0] = ztot;
-        rsz[1][1] = n - ztot;
-        rst[1][0] = 0;
-        rst[1][1] = ztot;
+  }
+  if constexpr (D > kTileMaxLevels) tile_run_sizes_deep<D, WARPS>(s_cnt, n, rsz, rst, status);
+  // the counts must agree with the planes
+  if (tid == 0) {
+    bool wrong = false;
+#pragma unroll
+    for (int s = 0; s < K - 1; ++s) wrong |= rst[s + 1][1 << s] != zeros[s];
+    if (wrong) atomicOr(status, kErrBounds);
+  }
+}
+
+// The ranked form of a pass that writes S_{l+4}: the tile's keys into shared
+// memory, V * KPL in a row of a thread's own; its planes in text order (set
+// 0); and the keys, narrowed to KeyO, sorted by their 4 digits at once into
+// `buf`.  Each thread
+// counts its keys of every digit from its plane words (16 masks, two counts a
+// register), the counts are scanned over the CTA, and the thread takes its
+// keys in order through a column of 16 cursors of its own in shared memory.
+// Rows are stored with their 16-byte vectors rotated (exclusive or), so that
+// both the load and the threads' reads touch every bank.
+//
+// Splitting the keys bit by bit instead costs 16 shared stores a vector and
+// split, with 2.8 wavefronts each (80% of the shared-memory pipe at 2^27
+// bytes); here a key is stored once, and the splits move planes.  Passes of
+// 2^28 8-bit keys 589 -> 517 us; of 2^26 16-bit ones 316 -> 211, narrowing to
+// 8 bits 322 -> 214; of 2^25 32-bit ones 231 -> 169 (GB300, 80 registers, 3
+// CTAs an SM).  512 threads of half the keys: 588 us, 266 and 275: every
+// thread's scans and cursors weigh more than the warps gained.
+template <typename KeyT, typename KeyO, int THREADS, int V>
+__device__ __forceinline__ void tile_rank_keys(const TileArgs& a, const TileSeg& s_sg, uint32_t g, uint32_t tl,
+                                               uint64_t tstart, uint32_t n, uint32_t shift, bool given,
+                                               uint32_t blk0, KeyT* buf, uint32_t* sbits, uint32_t* s_cnt,
+                                               unsigned long long* pre) {
+  constexpr int K = 4, NB = 16, KB = int(sizeof(KeyT)), KO = int(sizeof(KeyO)), KPL = 16 / KB;
+  constexpr int ITEMS = V * KPL, WPT = ITEMS / 32;
+  using C = TileCfg<KeyT, K, true, THREADS, V>;
+  constexpr int SBW = C::SBW, WARPS = C::WARPS;
+  static_assert(C::RANKABLE && (V == 4 || V == 8), "whole plane words a thread, rows of 64 or 128 bytes");
+  static_assert(THREADS == 256, "the cursors' columns");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  auto turn = [](int row) { return V == 8 ? row & 7 : (row >> 1) & 3; };
+  uint4* rows = reinterpret_cast<uint4*>(buf);
+  {
+    const uintptr_t sa =
+        reinterpret_cast<uintptr_t>(static_cast<const unsigned char*>(a.in) + (s_sg.in_begin + tstart) * KB);
+    const uint32_t off = uint32_t(sa & 15), bytes = n * KB, nvec = (bytes + 15) >> 4;
+    const uint4* av = reinterpret_cast<const uint4*>(sa - off);
+    const uint32_t last_block = (off + bytes - 1) >> 4;  // last aligned block holding tile bytes (n >= 1)
+    uint4 kv[V];
+#pragma unroll
+    for (int r = 0; r < V; ++r) {
+      const uint32_t k = uint32_t(r * THREADS + tid);
+      kv[r] = k < nvec ? __ldcs(av + k) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (off) {
+#pragma unroll
+      for (int r = 0; r < V; ++r) {
+        const uint32_t k = uint32_t(r * THREADS + tid);
+        const uint4 hi = k < nvec && k + 1 <= last_block ? __ldcs(av + k + 1) : make_uint4(0u, 0u, 0u, 0u);
+        kv[r] = realign16(kv[r], hi, off);
       }
-    } else if (tid < (2 << s)) {
-      const int v = tid & ((1 << s) - 1);
-      const uint32_t st = rst[s][v], en = st + rsz[s][v];
-      auto zb = [&](uint32_t p) -> uint32_t {  // zeros of plane s before position p (S_{l+s} order)
-        if (p >= n) return *s_ztot;
-        const uint32_t w = p >> 5, k = p & 31;
-        return zpos[w] + k - (k ? __popc(Pc[s * SBW + w] >> (32 - k)) : 0u);
-      };
-      const uint32_t zin = zb(en) - zb(st);
-      rsz[s + 1][tid] = (tid >> s) ? rsz[s][v] - zin : zin;
+    }
+#pragma unroll
+    for (int r = 0; r < V; ++r) {
+      const int k = r * THREADS + tid, row = k / V;
+      rows[row * V + ((k % V) ^ turn(row))] = kv[r];
     }
   }
+  if (tid < 4 * K) sbits[(tid >> 2) * SBW + C::T / 32 + (tid & 3)] = 0u;  // the words after each plane
+  __syncthreads();
+
+  uint32_t kw[V * 4];  // the thread's keys
+#pragma unroll
+  for (int r = 0; r < V; ++r) {
+    const uint4 x = rows[tid * V + (r ^ turn(tid))];
+    kw[4 * r] = x.x, kw[4 * r + 1] = x.y, kw[4 * r + 2] = x.z, kw[4 * r + 3] = x.w;
+  }
+  const uint32_t lo = shift - uint32_t(K - 1);
+  uint32_t cnt[NB / 2];  // digits 2q and 2q+1 (key_4: bit t is plane t) in halves
+#pragma unroll
+  for (int q = 0; q < NB / 2; ++q) cnt[q] = 0;
+#pragma unroll
+  for (int k = 0; k < WPT; ++k) {
+    uint32_t w[8], pl[K];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if constexpr (KB == 1) {
+        w[i] = kw[8 * k + i];
+      } else if constexpr (KB == 2) {
+        w[i] = __byte_perm(kw[16 * k + 2 * i] >> lo, kw[16 * k + 2 * i + 1] >> lo, 0x6420);
+      } else {
+        const uint32_t* x = kw + 32 * k + 4 * i;
+        w[i] = __byte_perm(__byte_perm(x[0] >> lo, x[1] >> lo, 0x0040), __byte_perm(x[2] >> lo, x[3] >> lo, 0x0040),
+                           0x5410);
+      }
+    }
+    key_planes<K>(w, KB == 1 ? lo : 0u, pl);
+    const uint32_t wi = uint32_t(tid * WPT + k), vm = plane_word_valid(n, wi);
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      pl[j] &= vm;
+      sbits[j * SBW + wi] = pl[j];
+    }
+    const uint32_t z0 = vm & ~pl[0];
+    const uint32_t lowm[4] = {z0 & ~pl[1], pl[0] & ~pl[1], z0 & pl[1], pl[0] & pl[1]};
+    const uint32_t him[4] = {~pl[2] & ~pl[3], pl[2] & ~pl[3], ~pl[2] & pl[3], pl[2] & pl[3]};
+#pragma unroll
+    for (int q = 0; q < NB / 2; ++q)
+      cnt[q] += __popc(lowm[(2 * q) & 3] & him[q >> 1]) + (__popc(lowm[(2 * q + 1) & 3] & him[q >> 1]) << 16);
+  }
+  // ---- exclusive counts before this thread ----------------------------------
+  __shared__ uint32_t s_wcnt[WARPS][NB / 2];
+  __shared__ __align__(16) uint32_t s_base[WARPS][NB];
+  uint32_t ex[NB / 2];
+#pragma unroll
+  for (int q = 0; q < NB / 2; ++q) {
+    uint32_t x = cnt[q];
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+      if (lane >= d) x += y;
+    }
+    ex[q] = x - cnt[q];
+    if (lane == 31) s_wcnt[warp][q] = x;
+  }
+  __syncthreads();  // every key is in registers too
+  if (tid < NB * WARPS) {
+    const int c = tid & (NB - 1), w = tid / NB;
+    uint32_t before = 0, total = 0;
+#pragma unroll
+    for (int u = 0; u < WARPS; ++u) {
+      const uint32_t x = (s_wcnt[u][c >> 1] >> (16 * (c & 1))) & 0xFFFFu;
+      before += u < w ? x : 0u;
+      total += x;
+    }
+    uint32_t start = total;
+#pragma unroll
+    for (int d = 1; d < NB; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, start, d, NB);
+      if (c >= d) start += y;
+    }
+    s_base[w][c] = start - total + before;
+    if (w == 0) {
+      s_cnt[c] = total;
+      if (given) {
+        const uint64_t blk = a.text_blocks ? uint64_t(blk0) + tl / a.tiles_per_block : g / a.tiles_per_block;
+        if (a.tilecnt[uint64_t(g) * NB + c] != total) atomicOr(a.status, kErrBounds);  // counts must agree
+        pre[c] = a.blockpre[blk * NB + c] + a.relpre[uint64_t(g) * NB + c];
+      } else {
+        st_volatile(a.lookback + uint64_t(c) * a.tiles + g, (g == s_sg.tile0 ? kFlagPrefix : kFlagAggregate) | total);
+      }
+    }
+  }
+  __syncthreads();
+  // ---- the keys, in order, through the thread's cursors -----------------------
+  uint32_t* cur = sbits + K * SBW;  // 16 columns of a word a thread: a lane's own bank
+  {
+    const uint32_t kbase = uint32_t(__cvta_generic_to_shared(buf));
+#pragma unroll
+    for (int q = 0; q < NB / 2; ++q) {
+      // column of digit c: its bits in key order, level l highest
+      constexpr int rev[16] = {0, 8, 4, 12, 2, 10, 6, 14, 1, 9, 5, 13, 3, 11, 7, 15};
+      cur[rev[2 * q] * THREADS + tid] = kbase + (s_base[warp][2 * q] + (ex[q] & 0xFFFFu)) * KO;
+      cur[rev[2 * q + 1] * THREADS + tid] = kbase + (s_base[warp][2 * q + 1] + (ex[q] >> 16)) * KO;
+    }
+  }
+  const uint32_t first = uint32_t(tid * ITEMS), valid = n > first ? n - first : 0u;
+  const uint32_t cbase = uint32_t(__cvta_generic_to_shared(cur));
+  // eight keys at a time: their cursors' reads are in flight together
+  constexpr int BATCHED = 8;
+  auto place = [&](int i0, uint32_t count) {
+    uint32_t at[BATCHED];
+#pragma unroll
+    for (int i = 0; i < BATCHED; ++i) {
+      const uint32_t w = kw[(i0 + i) * KB / 4], b = uint32_t(8 * KB * ((i0 + i) % (4 / KB)));
+      const uint32_t col = (__funnelshift_l(w, w, 10u - b - lo) & (15u << 10)) | uint32_t(tid * 4);  // digit * 1024
+      at[i] = 0;
+      if (uint32_t(i) < count)
+        asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(at[i]) : "r"(cbase + col), "n"(KO) : "memory");
+    }
+#pragma unroll
+    for (int i = 0; i < BATCHED; ++i)
+      if (uint32_t(i) < count)
+        st_shared_key(at[i], kw[(i0 + i) * KB / 4] >> (8 * KB * ((i0 + i) % (4 / KB))), KO);
+  };
+  if (valid >= uint32_t(ITEMS)) {
+#pragma unroll
+    for (int i = 0; i < ITEMS; i += BATCHED) place(i, BATCHED);
+  } else {
+#pragma unroll
+    for (int i = 0; i < ITEMS; i += BATCHED)
+      if (uint32_t(i) < valid) place(i, valid - uint32_t(i));
+  }
+  __syncthreads();
+  for (int i = tid; i < K * SBW; i += THREADS) cur[i] = 0u;  // set 1 of the planes, for the splits
 }
 
 // One tile of a pass: tile g of the launch's segments.  BATCH: a pass of a
@@ -987,9 +1278,10 @@ __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in)
   KeyT* buf0 = reinterpret_cast<KeyT*>(smem_raw);
   // K streams of SBW words (PLANES: two sets of K planes, the stream of level
   // l+j being plane j of set j % 2)
+  constexpr bool RANKED = !BATCH && C::RANKABLE, WORD_PARALLEL = C::WORD_PARALLEL && !RANKED;
   uint32_t* sbits = reinterpret_cast<uint32_t*>(smem_raw + (PLANES ? size_t(0) : size_t(T) * KB));
   uint32_t* meta = sbits + K * SBW;  // D >= 2: per vector
-  auto stream = [&](int j) -> const uint32_t* { return sbits + ((PLANES ? (j & 1) * K : 0) + j) * SBW; };
+  auto stream = [&](int j) -> const uint32_t* { return sbits + ((PLANES || RANKED ? (j & 1) * K : 0) + j) * SBW; };
 
   __shared__ uint32_t s_tile, s_seg;
   __shared__ TileSeg s_sg;
@@ -1060,8 +1352,13 @@ __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in)
   if constexpr (PLANES) {
     static_assert(sizeof(KeyT) == 1 && !OUT, "bit planes: passes over 1-byte keys without S_{l+K}");
     static_assert(K <= kTileMaxLevels || !BATCH, "batched passes take at most 4 levels");
-    tile_planes_splits<K, THREADS, V, BATCH>(a, s_tx, s_sg, g, tl, tstart, n, VP, shift, given, sbits, s_cnt, pre,
-                                             s_wz, &s_ztot, rsz, rst);
+    tile_planes_load<K, THREADS, V, BATCH>(a, s_tx, s_sg, g, tl, tstart, n, VP, shift, given, sbits, s_cnt, pre);
+    uint2* s_clut = reinterpret_cast<uint2*>(smem_raw + C::plane_area() - 256 * 8);
+    tile_planes_splits<K, D, THREADS, V, BATCH>(n, VP, sbits, s_clut, s_cnt, s_wz, rsz, rst, a.status);
+  } else if constexpr (RANKED) {
+    tile_rank_keys<KeyT, KeyO, THREADS, V>(a, s_sg, g, tl, tstart, n, shift, given, s_tx.blk0, buf0, sbits, s_cnt, pre);
+    uint2* s_clut = reinterpret_cast<uint2*>(smem_raw + C::ranked_area() - 256 * 8);
+    tile_planes_splits<K, D, THREADS, V / KB, false>(n, V / KB, sbits, s_clut, s_cnt, s_wz, rsz, rst, a.status);
   } else {
   {
     const unsigned char* src = static_cast<const unsigned char*>(a.in) + (s_sg.in_begin + tstart) * KB;
@@ -1249,9 +1546,9 @@ __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in)
       rsz[s + 1][tid] = (tid >> s) ? rsz[s][v] - zin : zin;
     }
   }
-  }  // !PLANES
+  }  // keys split bit by bit
   __syncthreads();
-  if constexpr (D >= 2) {
+  if constexpr (D >= 2 && !PLANES && !RANKED) {
     if constexpr (K > kTileMaxLevels) {
       if (warp == 0) warp_exclusive_scan(rsz[D], rst[D], 1 << D, lane);
     } else if (tid == 0) {
@@ -1271,7 +1568,7 @@ __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in)
       write_bits64(st ? s_tx.wt : s_tx.wm, s_tx.nbits, dst, stream(0), 0, n, uint32_t(tid), uint32_t(THREADS),
                    a.status);
   }
-  if constexpr (D >= 1) {
+  if constexpr (D >= 1 && !PLANES && !RANKED) {
     if (tid < NLB && s_cnt[tid] != rsz[D][tid]) atomicOr(a.status, kErrBounds);  // counts must agree
   }
   if constexpr (D >= 1 && D <= kTileMaxLevels) {
@@ -1286,15 +1583,15 @@ __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in)
   // ---- runs of S_{l+K} and of levels 1..K-1, round-robin over the warps ---
   // prefix of run v of key_j (j >= 1): the finest runs with key_j == v
   constexpr int NINNER = (1 << K) - 2;  // runs of levels 1..K-1 of one structure
-  __shared__ unsigned long long runpre[C::WORD_PARALLEL ? (1 << K) : 1];
-  __shared__ RunRec recs[C::WORD_PARALLEL ? 1 : (NINNER > 0 ? 2 * NINNER : 1)];
+  __shared__ unsigned long long runpre[WORD_PARALLEL ? (1 << K) : 1];
+  __shared__ RunRec recs[WORD_PARALLEL ? 1 : (NINNER > 0 ? 2 * NINNER : 1)];
   if (tid < NINNER) {
     int j = 1;
     while (tid + 2 >= (2 << j)) ++j;
     const int v = tid + 2 - (1 << j);
     uint64_t p = 0;
     for (int h = 0; h < (1 << (D - j)); ++h) p += pre[v + (h << j)];
-    if constexpr (C::WORD_PARALLEL) {
+    if constexpr (WORD_PARALLEL) {
       runpre[tid] = p;
     } else {
       for (int st = 0; st < nstruct; ++st)
@@ -1304,7 +1601,7 @@ __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in)
     }
   }
   __syncthreads();
-  if constexpr (C::WORD_PARALLEL) {
+  if constexpr (WORD_PARALLEL) {
     // Levels 1..K-1 of both structures, word-parallel: a deep level has up to
     // 2^(K-1) runs, most of them a few words long (and the tiles of 2- and
     // 4-byte keys are short), so instead of a warp per run every thread
@@ -1458,7 +1755,11 @@ __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in)
         if (lane == 0) atomicOr(a.status, kErrBounds);
         continue;
       }
-      if constexpr (sizeof(KeyO) == sizeof(KeyT))
+      if constexpr (RANKED)
+        write_key_run(reinterpret_cast<unsigned char*>(static_cast<KeyO*>(a.out) + dst),
+                      reinterpret_cast<const unsigned char*>(reinterpret_cast<const KeyO*>(buf0) + rst[D][v]),
+                      len * uint32_t(sizeof(KeyO)));
+      else if constexpr (sizeof(KeyO) == sizeof(KeyT))
         write_key_run(reinterpret_cast<unsigned char*>(static_cast<KeyT*>(a.out) + dst),
                       reinterpret_cast<const unsigned char*>(cb + rst[D][v]), len * uint32_t(KB));
       else

@@ -14,7 +14,7 @@ template <typename KeyT, int K, bool OUT, typename KeyO = KeyT, bool PLANES = fa
 void launch_tile_one(const TileArgs& a, cudaStream_t s) {
   using C = TileCfg<KeyT, K, OUT, kTileThreads, V>;
   auto kern = tile_pass_kernel<KeyT, K, OUT, kTileThreads, V, KeyO, PLANES>;
-  constexpr size_t smem = PLANES ? C::plane_smem_bytes() : C::smem_bytes();
+  constexpr size_t smem = PLANES ? C::plane_smem_bytes() : C::RANKABLE ? C::ranked_smem_bytes() : C::smem_bytes();
   static bool configured = false;  // attribute set once per instantiation
   if (!configured) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
