@@ -26,12 +26,12 @@ __device__ __forceinline__ void batch_hist_planes(const uint8_t* text, const Bat
   constexpr uint32_t NB = 1u << (L - 1);  // D = L - 1: every text of up to 4 levels takes one pass
   auto* pairs = reinterpret_cast<uint32_t (*)[WARPS][8]>(smem);  // [2]
   const uint32_t tid = threadIdx.x, T = 1u << c.log2T;
-  const int nv = int(T / (16 * kBatchThreads));  // 1, 2 or 4 vectors a thread
+  const int nv = int(T / (16 * kBatchThreads));  // 1, 2, 4 or 8 vectors a thread
   uint32_t rel = 0, mine = 0, seen = 0;
   for (uint32_t k = 0; k < ntiles; ++k) {
     const uint64_t start = uint64_t(k) << c.log2T;
     const uint32_t len = uint32_t(c.len - start < T ? c.len - start : T);
-    count_tile_planes<L, kBatchThreads, 4>(text + start, len, nv, seen, pairs[k & 1], [](int, uint32_t, const uint4&) {});
+    count_tile_planes<L, kBatchThreads, 8>(text + start, len, nv, seen, pairs[k & 1], [](int, uint32_t, const uint4&) {});
     __syncthreads();
     const uint32_t (*pr)[8] = pairs[k & 1];
     if (tid < NB) {

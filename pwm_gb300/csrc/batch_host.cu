@@ -18,7 +18,7 @@ constexpr uint32_t kBatchMaxLevels = 12;        // per-text tables live in share
 constexpr uint64_t kBatchChunk = 65536;         // symbols per histogram CTA
 constexpr size_t kTuneMaxTexts = 4096;           // texts of a tuning sub-batch (at most)
 constexpr uint64_t kTuneSymbols = uint64_t(1) << 26;  // symbols of a tuning sub-batch (about)
-constexpr uint32_t kGivenBlockTiles = 16;        // first-pass tiles per histogram block (a CTA's)
+constexpr uint32_t kGivenBlockTiles = 16;        // first-pass tiles per histogram block (a CTA's); half the wide ones
 constexpr uint64_t kBatchRegroupWords = 1024;   // words per regroup CTA
 
 struct BatchPassGroup {
@@ -236,8 +236,18 @@ uint32_t tune_key(uint32_t width, uint32_t L, uint64_t n) {
 // left; a pass writes the next sequence unless it is the last.
 uint32_t tile_npass(uint32_t L) { return (L + uint32_t(kTileMaxLevels) - 1) / uint32_t(kTileMaxLevels); }
 
-uint8_t tile_variant(uint32_t K, bool out) {
+// Tiles of 8 vectors a thread (the single builds' double tiles): last passes
+// over 1-byte keys of texts tuned to 4 vectors that have four such tiles for
+// every segment of the pass.  4096 uneven texts, 85% of 3 levels: the kernel
+// 1.63 -> 1.57 ms (at 64 registers; 1.76 without them, at 48 1.63 either way).
+bool tile_wide(const pwmgpu_batch* b, uint32_t t, uint32_t l, uint32_t K, bool out) {
+  return b->width == 1 && !b->force_vpt && b->vpt[t] == 4 && !out && K >= 2 &&
+         b->info[t].n >= (uint64_t(4) << l) * tile_pass_elems(1, 8);
+}
+
+uint8_t tile_variant(uint32_t K, bool out, bool wide) {
   if (out) return kTileBatchK4Out;  // only passes of kTileMaxLevels levels write S_{l+K}
+  if (wide) return K == 4 ? kTileBatchK4Wide : K == 3 ? kTileBatchK3Wide : kTileBatchK2Wide;
   return K == 4 ? kTileBatchK4 : K == 3 ? kTileBatchK3 : K == 2 ? kTileBatchK2 : kTileBatchK1;
 }
 
@@ -251,7 +261,7 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
   b->drop_tile_plan();
   const uint32_t KPL = 16 / b->width;
   struct Item {
-    uint32_t t, p, l, K;
+    uint32_t t, p, l, K, vpt;
     bool out;
   };
   std::map<std::pair<uint32_t, uint8_t>, std::vector<Item>> by;
@@ -264,7 +274,8 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
     for (uint32_t p = 0; p < np; ++p) {
       const uint32_t l = p * uint32_t(kTileMaxLevels), K = std::min<uint32_t>(uint32_t(kTileMaxLevels), L - l);
       const bool out = l + K < L;
-      by[{p, tile_variant(K, out)}].push_back({t, p, l, K, out});
+      const bool wide = tile_wide(b, t, l, K, out);
+      by[{p, tile_variant(K, out, wide)}].push_back({t, p, l, K, wide ? 8u : b->vpt[t], out});
     }
   }
   if (by.size() > kTileBatchMaxGroups) throw Fail{PWMGPU_ERR_ARG, "too many pass shapes in one batch"};
@@ -313,7 +324,7 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
     const int TS = tile_table_size(int(K));
     uint64_t nsegs = 0, tiles_ub = 1;
     for (const Item& it : items) {
-      const uint64_t TT = uint64_t(256) * b->vpt[it.t] * KPL;
+      const uint64_t TT = uint64_t(256) * it.vpt * KPL;
       nsegs += uint64_t(1) << it.l;
       tiles_ub += (b->info[it.t].n + TT - 1) / TT + (uint64_t(1) << it.l);
     }
@@ -330,6 +341,7 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
     uint64_t seg_base = 0;
     const uint32_t D = out ? K : K - 1;
     const bool given = p == 0 && D >= 1;
+    const uint32_t block_tiles = items[0].vpt == 8 ? kGivenBlockTiles / 2 : kGivenBlockTiles;
     const uint64_t group_cnt_off = cnt_total, group_blk_off = blk_total;
     uint64_t group_tile = 0, group_blk = 0;  // tiles and blocks of the group's texts so far (device order)
     for (size_t i = 0; i < items.size(); ++i) {
@@ -342,14 +354,14 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
       x.stride = wpl;
       x.nbits = b->info[t].n;
       x.shift = b->L[t] - 1 - it.l;
-      x.vpt = b->vpt[t];
+      x.vpt = it.vpt;
       x.wait_idx = it.p ? first_slot[t] + it.p - 1 : ~0u;
       x.signal_idx = it.p + 1 < tile_npass(b->L[t]) ? first_slot[t] + it.p : ~0u;
       TileBatchPass P{};
       P.text = t;
       P.group = gi;
       P.level = it.l;
-      P.vpt = b->vpt[t];
+      P.vpt = it.vpt;
       P.seg_base = uint32_t(seg_base);
       P.tt_index = uint32_t(i);
       P.slot = first_slot[t] + it.p;
@@ -357,9 +369,9 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
       passes.push_back(P);
       seg_base += uint64_t(1) << it.l;
       if (given) {
-        // blocks of kGivenBlockTiles tiles, one histogram CTA each
-        const uint64_t TT = uint64_t(256) * b->vpt[t] * KPL, n = b->info[t].n, NB = uint64_t(1) << D;
-        const uint64_t nt = (n + TT - 1) / TT, nblk = (nt + kGivenBlockTiles - 1) / kGivenBlockTiles;
+        // blocks of tiles, one histogram CTA each
+        const uint64_t TT = uint64_t(256) * it.vpt * KPL, n = b->info[t].n, NB = uint64_t(1) << D;
+        const uint64_t nt = (n + TT - 1) / TT, nblk = (nt + block_tiles - 1) / block_tiles;
         uint32_t log2T = 0;
         while ((uint64_t(1) << log2T) < TT) ++log2T;
         TileBatchText& x0 = texts[t];
@@ -370,9 +382,9 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
         for (uint64_t k = 0; k < nblk; ++k) {
           BatchChunk ch{};
           ch.text = t;
-          ch.start = k * kGivenBlockTiles * TT;
-          ch.len = std::min<uint64_t>(kGivenBlockTiles * TT, n - ch.start);
-          ch.cnt_off = group_cnt_off + (group_tile + k * kGivenBlockTiles) * NB;
+          ch.start = k * block_tiles * TT;
+          ch.len = std::min<uint64_t>(block_tiles * TT, n - ch.start);
+          ch.cnt_off = group_cnt_off + (group_tile + k * block_tiles) * NB;
           ch.blk_off = x0.blk_off + k * NB;
           ch.D = D;
           ch.log2T = log2T;
@@ -406,7 +418,7 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
     a.done = b->d_done;
     a.need = b->d_need;
     if (given) {
-      a.tiles_per_block = kGivenBlockTiles;
+      a.tiles_per_block = block_tiles;
       a.text_blocks = 1;
       given_groups.push_back({args.size(), group_cnt_off, group_blk_off});  // arrays set below
     }
@@ -427,6 +439,9 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
         ch.len = std::min<uint64_t>(kBatchChunk, b->info[t].n - c0);
         b->tchunks.push_back(ch);
       }
+  // the chunks that take longest first: an atomic or two a symbol (8-bit texts of 2 to 4 levels are counted by planes)
+  std::stable_partition(b->tchunks.begin(), b->tchunks.end(),
+                        [&](const BatchChunk& c) { return b->width != 1 || !c.D || b->L[c.text] > 4; });
   b->d_tchunks = static_cast<BatchChunk*>(b->talloc(std::max<size_t>(b->tchunks.size(), 1) * sizeof(BatchChunk)));
   if (!b->tchunks.empty())
     CUDA_TRY(cudaMemcpy(b->d_tchunks, b->tchunks.data(), b->tchunks.size() * sizeof(BatchChunk),

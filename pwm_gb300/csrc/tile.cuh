@@ -69,7 +69,7 @@ struct TileText {
   uint64_t nbits;   // bits of every level
   uint32_t shift;   // level l+j tests key bit (shift - j)
   // Batched passes (tile_pass_body with BATCH) only; zero otherwise:
-  uint32_t vpt;         // 16-byte vectors per thread of this text's tiles (1, 2 or 4)
+  uint32_t vpt;         // 16-byte vectors per thread of this text's tiles (1, 2 or 4; 8 in the wide shapes)
   uint32_t wait_idx;    // ~0u, or a counter in TileArgs::done this pass waits for ...
   uint32_t signal_idx;  // ~0u, or a counter each of its tiles adds one to when done
   uint32_t blk0;        // with TileArgs::text_blocks: the text's first block of given prefixes
@@ -777,10 +777,10 @@ __device__ __forceinline__ uint32_t plane_word_valid(uint32_t n, uint32_t w) {
 
 // The load of a tile in bit-plane form (tile_pass_body with PLANES; 1-byte
 // keys, no S_{l+K}): its planes in text order (set 0) and the counts of its
-// finest runs (counted and published for the look-back, or given).  BATCH:
+// finest runs (counted and published for the look-back, or given).  VARY:
 // the tile has VP <= V vectors per thread, so NWt = THREADS * VP / 2 plane
 // words; the words above NWt stay zero.
-template <int K, int THREADS, int V, bool BATCH>
+template <int K, int THREADS, int V, bool VARY>
 __device__ __forceinline__ void tile_planes_load(const TileArgs& a, const TileText& s_tx, const TileSeg& s_sg,
                                                  uint32_t g, uint32_t tl, uint64_t tstart, uint32_t n, int VP,
                                                  uint32_t shift, bool given, uint32_t* sbits, uint32_t* s_cnt,
@@ -790,13 +790,13 @@ __device__ __forceinline__ void tile_planes_load(const TileArgs& a, const TileTe
   constexpr int NW = T / 32;         // plane words of a tile of V vectors per thread
   constexpr int WPT = NW / THREADS;  // plane words per thread in the splits
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t NWt = BATCH ? uint32_t(THREADS * VP / 2) : uint32_t(NW);  // plane words of this tile
-  const int wpt = BATCH ? (VP >= 2 ? VP / 2 : 1) : WPT;                     // of them per thread
+  const uint32_t NWt = VARY ? uint32_t(THREADS * VP / 2) : uint32_t(NW);  // plane words of this tile
+  const int wpt = VARY ? (VP >= 2 ? VP / 2 : 1) : WPT;                     // of them per thread
   auto word_valid = [&](uint32_t w) { return plane_word_valid(n, w); };
 
   // set 1 and the words of set 0 above the tile's start cleared
   for (int i = tid; i < K * SBW; i += THREADS) sbits[K * SBW + i] = 0u;
-  if (BATCH && NWt < uint32_t(NW)) {
+  if (VARY && NWt < uint32_t(NW)) {
     const uint32_t pad = uint32_t(SBW) - NWt;
     for (uint32_t i = tid; i < K * pad; i += THREADS) sbits[(i / pad) * SBW + NWt + i % pad] = 0u;
   } else if (tid < 4 * K) {
@@ -828,9 +828,9 @@ __device__ __forceinline__ void tile_planes_load(const TileArgs& a, const TileTe
     };
 #pragma unroll
     for (int r = 0; r < V; r += 2) {
-      if (BATCH && r >= VP) break;  // uniform over the CTA
+      if (VARY && r >= VP) break;  // uniform over the CTA
       const int gv = (warp * VP + r) * 32 + lane;
-      const bool two = !BATCH || r + 1 < VP;
+      const bool two = !VARY || r + 1 < VP;
       const uint4 a0 = load(gv), a1 = two ? load(gv + 32) : make_uint4(0u, 0u, 0u, 0u);
       uint32_t w[8];
       {
@@ -870,18 +870,18 @@ __device__ __forceinline__ void tile_planes_load(const TileArgs& a, const TileTe
       uint32_t cnt[NLB], words[D][WPT];
 #pragma unroll
       for (int c = 0; c < NLB; ++c) cnt[c] = 0;
-      if constexpr (!BATCH) {
+      if constexpr (!VARY) {
 #pragma unroll
         for (int t = 0; t < D; ++t) plane_words<WPT>(sbits + t * SBW, tid, words[t]);
       }
 #pragma unroll
       for (int k = 0; k < WPT; ++k) {
-        if (BATCH && k >= wpt) break;
+        if (VARY && k >= wpt) break;
         const uint32_t w = uint32_t(tid) * wpt + k;
         const uint32_t vmk = word_valid(w);  // 0 above the tile's words
         uint32_t pl[D];
 #pragma unroll
-        for (int t = 0; t < D; ++t) pl[t] = BATCH ? sbits[t * SBW + w] : words[t][k];
+        for (int t = 0; t < D; ++t) pl[t] = VARY ? sbits[t * SBW + w] : words[t][k];
 #pragma unroll
         for (int c = 0; c < NLB; ++c) {
           uint32_t mt = vmk;
@@ -967,9 +967,9 @@ __device__ __forceinline__ void tile_run_sizes_deep(const uint32_t* s_cnt, uint3
 // planes, scans the zero counts over the CTA, and ORs the compressed zero and
 // one parts of each later plane into the other set at the word's zero and one
 // cursors; its own words of the read set are cleared for the split after next.
-// V: 16-byte vectors of 1-byte keys that fill the planes.  BATCH: max(VP / 2,
+// V: 16-byte vectors of 1-byte keys that fill the planes.  VARY: max(VP / 2,
 // 1) words a thread (VP = 1: the first half of the threads own one word each).
-template <int K, int D, int THREADS, int V, bool BATCH>
+template <int K, int D, int THREADS, int V, bool VARY>
 __device__ __forceinline__ void tile_planes_splits(uint32_t n, int VP, uint32_t* sbits, uint2* s_clut,
                                                    const uint32_t* s_cnt, uint32_t* s_wz, uint32_t (*rsz)[1 << D],
                                                    uint32_t (*rst)[1 << D], uint32_t* status) {
@@ -978,7 +978,7 @@ __device__ __forceinline__ void tile_planes_splits(uint32_t n, int VP, uint32_t*
   constexpr int NW = C::T / 32, WPT = NW / THREADS;
   static_assert(K >= 1 && K <= kTileGivenMaxLevels && WPT * THREADS == NW, "up to 8 levels; whole words per thread");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wpt = BATCH ? (VP >= 2 ? VP / 2 : 1) : WPT;
+  const int wpt = VARY ? (VP >= 2 ? VP / 2 : 1) : WPT;
   for (int b = tid; b < 256; b += THREADS) s_clut[b] = kCompressLut.e[b];
   if (tid == 0) {
     rsz[0][0] = n;
@@ -991,7 +991,7 @@ __device__ __forceinline__ void tile_planes_splits(uint32_t n, int VP, uint32_t*
     uint32_t* Pn = sbits + ((s & 1) ^ 1) * K * SBW;  // planes s+1.. in S_{l+s+1} order
     uint32_t m[WPT], vmk[WPT], zc[WPT], pw[K][WPT];
     uint32_t tsum = 0;
-    if constexpr (!BATCH) {  // a thread's words are one aligned vector; read, and cleared for the split after next
+    if constexpr (!VARY) {  // a thread's words are one aligned vector; read, and cleared for the split after next
       plane_words<WPT>(Pc + s * SBW, tid, m);
 #pragma unroll
       for (int p = s + 1; p < K; ++p) {
@@ -1002,8 +1002,8 @@ __device__ __forceinline__ void tile_planes_splits(uint32_t n, int VP, uint32_t*
 #pragma unroll
     for (int k = 0; k < WPT; ++k) {
       const uint32_t w = uint32_t(tid) * wpt + k;  // < NW: every word read is inside the planes
-      vmk[k] = (BATCH && k >= wpt) ? 0u : plane_word_valid(n, w);
-      if constexpr (BATCH) {
+      vmk[k] = (VARY && k >= wpt) ? 0u : plane_word_valid(n, w);
+      if constexpr (VARY) {
         m[k] = k >= wpt ? 0u : Pc[s * SBW + w];
 #pragma unroll
         for (int p = s + 1; p < K; ++p) pw[p][k] = k >= wpt ? 0u : Pc[p * SBW + w];
@@ -1033,9 +1033,9 @@ __device__ __forceinline__ void tile_planes_splits(uint32_t n, int VP, uint32_t*
     uint32_t zp = zpre + x - tsum;  // zeros before this thread's first word
 #pragma unroll
     for (int k = 0; k < WPT; ++k) {
-      if (BATCH && k >= wpt) break;
+      if (VARY && k >= wpt) break;
       const uint32_t w = uint32_t(tid) * wpt + k;
-      if constexpr (BATCH) {
+      if constexpr (VARY) {
 #pragma unroll
         for (int p = s + 1; p < K; ++p) Pc[p * SBW + w] = 0u;  // read above; set again two splits on
       }
@@ -1260,7 +1260,7 @@ __device__ __forceinline__ void tile_rank_keys(const TileArgs& a, const TileSeg&
 // One tile of a pass: tile g of the launch's segments.  BATCH: a pass of a
 // batch of texts inside the persistent kernel (tile_batch.cu): the tile size
 // is the text's own (TileText::vpt vectors per thread, a warp's slice
-// shrinking with it), the tile first waits until every tile of the text's
+// shrinking with it; V = 8 fixes it), the tile first waits until every tile of the text's
 // previous pass is done and afterwards counts itself done; otherwise
 // TileText's batch fields are ignored.
 // KeyO: the key type of S_{l+K} (KeyT, or narrower when the levels left
@@ -1338,8 +1338,9 @@ __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in)
       __syncthreads();
     }
   }
-  const int VP = BATCH ? int(s_tx.vpt) : V;  // vectors per thread of this tile
-  const uint32_t TT = BATCH ? uint32_t(THREADS * VP * KPL) : uint32_t(T);
+  constexpr bool VARY = BATCH && V <= 4;            // tiles of the text's own size
+  const int VP = VARY ? int(s_tx.vpt) : V;  // vectors per thread of this tile
+  const uint32_t TT = VARY ? uint32_t(THREADS * VP * KPL) : uint32_t(T);
   const uint32_t tl = g - s_sg.tile0;
   const uint64_t tstart = uint64_t(tl) * TT;
   const uint32_t n = s_sg.m - tstart < uint64_t(TT) ? uint32_t(s_sg.m - tstart) : TT;
@@ -1352,9 +1353,9 @@ __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in)
   if constexpr (PLANES) {
     static_assert(sizeof(KeyT) == 1 && !OUT, "bit planes: passes over 1-byte keys without S_{l+K}");
     static_assert(K <= kTileMaxLevels || !BATCH, "batched passes take at most 4 levels");
-    tile_planes_load<K, THREADS, V, BATCH>(a, s_tx, s_sg, g, tl, tstart, n, VP, shift, given, sbits, s_cnt, pre);
+    tile_planes_load<K, THREADS, V, VARY>(a, s_tx, s_sg, g, tl, tstart, n, VP, shift, given, sbits, s_cnt, pre);
     uint2* s_clut = reinterpret_cast<uint2*>(smem_raw + C::plane_area() - 256 * 8);
-    tile_planes_splits<K, D, THREADS, V, BATCH>(n, VP, sbits, s_clut, s_cnt, s_wz, rsz, rst, a.status);
+    tile_planes_splits<K, D, THREADS, V, VARY>(n, VP, sbits, s_clut, s_cnt, s_wz, rsz, rst, a.status);
   } else if constexpr (RANKED) {
     tile_rank_keys<KeyT, KeyO, THREADS, V>(a, s_sg, g, tl, tstart, n, shift, given, s_tx.blk0, buf0, sbits, s_cnt, pre);
     uint2* s_clut = reinterpret_cast<uint2*>(smem_raw + C::ranked_area() - 256 * 8);

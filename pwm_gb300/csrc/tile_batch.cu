@@ -222,10 +222,11 @@ __global__ void __launch_bounds__(1024) tile_batch_scan_kernel(const TileBatchGr
 }
 
 // The persistent kernel: a CTA per resident slot (5 per SM, 48 registers a
-// thread) takes items until the queue is drained.  Item i of group k is tile
-// i - base(k) of that group's pass.
+// thread; over 1-byte keys 4 and 64, for the wide tiles) takes items until the
+// queue is drained.  Item i of group k is tile i - base(k) of that group's
+// pass.
 template <typename KeyT>
-__global__ void __launch_bounds__(256, 5) tile_batch_kernel(TileBatchQueue q) {
+__global__ void __launch_bounds__(256, sizeof(KeyT) == 1 ? 4 : 5) tile_batch_kernel(TileBatchQueue q) {
   __shared__ uint32_t s_base[kTileBatchMaxGroups + 1];
   __shared__ uint32_t s_item, s_gi;
   __shared__ __align__(16) TileArgs s_args;
@@ -263,6 +264,15 @@ __global__ void __launch_bounds__(256, 5) tile_batch_kernel(TileBatchQueue q) {
     const uint32_t g = s_item - s_base[k];
     // passes without S_{l+K} over 1-byte keys split bit planes
     constexpr bool PL = sizeof(KeyT) == 1;
+    if constexpr (PL) {
+      const uint8_t variant = q.variant[k];
+      if (variant >= kTileBatchK4Wide) {
+        if (variant == kTileBatchK4Wide) tile_pass_body<KeyT, 4, false, 256, 8, true, KeyT, true>(s_args, g);
+        else if (variant == kTileBatchK3Wide) tile_pass_body<KeyT, 3, false, 256, 8, true, KeyT, true>(s_args, g);
+        else tile_pass_body<KeyT, 2, false, 256, 8, true, KeyT, true>(s_args, g);
+        continue;
+      }
+    }
     switch (q.variant[k]) {
       case kTileBatchK4Out: tile_pass_body<KeyT, 4, true, 256, 4, true>(s_args, g); break;
       case kTileBatchK4: tile_pass_body<KeyT, 4, false, 256, 4, true, KeyT, PL>(s_args, g); break;
@@ -275,13 +285,16 @@ __global__ void __launch_bounds__(256, 5) tile_batch_kernel(TileBatchQueue q) {
 
 template <typename KeyT>
 size_t batch_kernel_smem() {
-  using C = TileCfg<KeyT, 4, true, 256, 4>;  // the largest shape's buffers
+  // the largest shape's buffers
+  constexpr size_t keys = TileCfg<KeyT, 4, true, 256, 4>::smem_bytes();
+  constexpr size_t planes = sizeof(KeyT) == 1 ? TileCfg<KeyT, 4, false, 256, 8>::plane_smem_bytes() : 0;
+  constexpr size_t bytes = keys > planes ? keys : planes;
   static bool configured = false;  // attribute set once per key width
   if (!configured) {
-    cudaFuncSetAttribute(tile_batch_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(C::smem_bytes()));
+    cudaFuncSetAttribute(tile_batch_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
     configured = true;
   }
-  return C::smem_bytes();
+  return bytes;
 }
 
 template <typename KeyT>

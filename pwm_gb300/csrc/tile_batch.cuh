@@ -9,11 +9,21 @@
 namespace pwmgpu {
 
 constexpr uint32_t kTileBatchMaxLevels = 12;  // a text's prefix tables fit one CTA's planning
-constexpr uint32_t kTileBatchMaxGroups = 16;  // pass groups of one batch
+constexpr uint32_t kTileBatchMaxGroups = 24;  // pass groups of one batch
 
 // Pass shapes of the persistent kernel: passes of 4 levels that write the
-// next sequence, and last passes of 1..4 levels.
-enum : uint8_t { kTileBatchK4Out = 0, kTileBatchK4 = 1, kTileBatchK3 = 2, kTileBatchK2 = 3, kTileBatchK1 = 4 };
+// next sequence, last passes of 1..4 levels, and last passes of 2..4 levels
+// over 1-byte keys in tiles of 8 vectors a thread.
+enum : uint8_t {
+  kTileBatchK4Out = 0,
+  kTileBatchK4 = 1,
+  kTileBatchK3 = 2,
+  kTileBatchK2 = 3,
+  kTileBatchK1 = 4,
+  kTileBatchK4Wide = 5,
+  kTileBatchK3Wide = 6,
+  kTileBatchK2Wide = 7,
+};
 
 // Offsets of a text's planning scratch: the natural prefix counts of levels
 // 0..L (level m at 2^m - 1), then the exclusive prefixes of every level in
