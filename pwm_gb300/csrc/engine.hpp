@@ -261,18 +261,17 @@ struct Structure {
   uint64_t n = 0;
   std::vector<uint64_t> bits, offs;
   uint64_t total_words = 0;
+  void* slab = nullptr;          // the one allocation that holds everything below
   uint64_t* d_words = nullptr;
   std::vector<uint64_t> zeros;   // host (matrix)
   uint64_t* d_zeros = nullptr;   // device copy (matrix), read by queries
   // rank/select
   bool rs = false;
-  void* d_rs = nullptr;          // l0, l12, samples and meta of all levels
-  size_t rs_bytes = 0;
   std::vector<RankSelectLevel> rs_levels;
   RankSelectLevel* d_rs_levels = nullptr;
   QueryLevel* d_q_levels = nullptr;
-  std::vector<QueryLevel> q_host;   // source of the asynchronous copy to d_q_levels
-  cudaStream_t alloc_stream = nullptr;  // stream-ordered allocations (nullptr: cudaMalloc)
+  std::vector<unsigned char> desc_host;  // source of the asynchronous copy to d_rs_levels and d_q_levels
+  cudaStream_t alloc_stream = nullptr;   // stream-ordered allocation (nullptr: cudaMalloc)
 
   void set_layout(const std::vector<uint64_t>& level_bits) {
     levels = uint32_t(level_bits.size());
@@ -283,19 +282,13 @@ struct Structure {
     total_words = off;
   }
   void release() {
-    auto fr = [&](void* p) {
-      if (!p) return;
-      if (alloc_stream) cudaFreeAsync(p, alloc_stream);
-      else cudaFree(p);
-    };
-    fr(d_words);
-    fr(d_zeros);
-    fr(d_rs);
-    fr(d_rs_levels);
-    fr(d_q_levels);
-    d_words = nullptr; d_zeros = nullptr; d_rs = nullptr; d_rs_levels = nullptr; d_q_levels = nullptr;
+    if (slab) {
+      if (alloc_stream) cudaFreeAsync(slab, alloc_stream);
+      else cudaFree(slab);
+    }
+    slab = nullptr;
+    d_words = nullptr; d_zeros = nullptr; d_rs_levels = nullptr; d_q_levels = nullptr;
     rs = false;
-    rs_bytes = 0;
   }
 };
 
@@ -382,18 +375,7 @@ inline uint64_t rs_n0(uint64_t nwords) { return nwords / (4294967295ull / 64) + 
 inline uint64_t rs_n12(uint64_t nwords) { return nwords / 32 + 1; }
 inline uint64_t rs_ns(uint64_t nwords) { return nwords * 64 / 8192 + 2; }
 
-// cudaMalloc, or a stream-ordered allocation on `stream` (no device-wide
-// synchronisation when freed).
-template <typename P>
-void dev_alloc(P** p, size_t bytes, cudaStream_t stream) {
-  void* v = nullptr;
-  if (stream) CUDA_TRY(cudaMallocAsync(&v, bytes, stream));
-  else CUDA_TRY(cudaMalloc(&v, bytes));
-  *p = static_cast<P*>(v);
-}
-
 // ---- structures and rank/select storage (engine.cu) ------------------------
-void alloc_rank_select(Structure& s);
 void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint64_t n, bool tree, bool huff,
                      bool rank_select, cudaStream_t stream, cudaStream_t alloc_stream = nullptr);
 // Rank/select blocks of every level of the given structures (asynchronous),
