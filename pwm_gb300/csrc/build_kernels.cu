@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(kTileHistThreads) tile_hist_kernel(const T* te
   // into column k, so the 32 lanes of an atomic never meet on an address or
   // a bank, however skewed the text (at most 8 warps x 128 symbols x 16
   // tiles = 16384 per counter).
+  chain_next();
   __shared__ __align__(16) uint32_t h[BINS * 32];
   __shared__ uint32_t s_tc[BINS / 2];  // runs of the first D <= 7 bits
   const int tid = threadIdx.x;
@@ -253,6 +254,7 @@ __global__ void __launch_bounds__(kTileHistThreads) tile_hist_planes_kernel(
     uint64_t* level0_b, uint32_t* status) {
   constexpr int WARPS = kTileHistThreads / 32, HV = 8;
   constexpr uint32_t NB = 1u << (L - 1);  // runs of the first L - 1 bits
+  chain_next();
   __shared__ uint32_t pairs[2][WARPS][8];
   const uint32_t tid = threadIdx.x, lane = tid & 31;
   const uint32_t block = block0 + blockIdx.x;
@@ -340,6 +342,8 @@ __global__ void __launch_bounds__(1024) tile_block_scan_kernel(unsigned long lon
                                                                uint32_t NB, const unsigned long long* hist,
                                                                uint32_t levels, uint32_t K, uint32_t out,
                                                                uint32_t tree, uint64_t* table, TileOnePass one) {
+  chain_next();
+  chain_wait();
   __shared__ unsigned long long wsum[32];
   const uint32_t tid = threadIdx.x;
   if (blockIdx.x < NB) {
@@ -1162,9 +1166,8 @@ void launch_tile_block_scan(unsigned long long* blocksum, uint32_t nblocks, uint
                             uint32_t levels, uint32_t K, bool out, bool tree, uint64_t* table, cudaStream_t s,
                             uint64_t* launches, const TileOnePass* one) {
   if (nblocks == 0) return;
-  tile_block_scan_kernel<<<(1u << D) + (table ? 1u : 0u), 1024, 0, s>>>(blocksum, nblocks, 1u << D, hist, levels, K,
-                                                                        out ? 1u : 0u, tree ? 1u : 0u, table,
-                                                                        one ? *one : TileOnePass{});
+  launch_chained(tile_block_scan_kernel, (1u << D) + (table ? 1u : 0u), 1024, 0, s, blocksum, nblocks, 1u << D, hist,
+                 levels, K, out ? 1u : 0u, tree ? 1u : 0u, table, one ? *one : TileOnePass{});
   ++*launches;
 }
 

@@ -101,4 +101,32 @@ __host__ __device__ inline uint32_t word_select1(uint64_t v, uint32_t rank) {
   return 64 - s;
 }
 
+// Programmatic dependent launch: a kernel launched with launch_chained may be
+// put on the SMs while the kernel before it in the stream still runs, once all
+// of that one's CTAs have called chain_next or ended; before it touches memory
+// it waits, in chain_wait, until the earlier kernel is complete and its writes
+// are visible.  Every thread of such a kernel calls chain_wait first, so that
+// when it is complete all kernels before it are.  Launched in any other way
+// both calls do nothing.  The tables after the histogram and rank/select after
+// a pass are chained: 4099 bytes with both structures and queries 79.8 -> 77.1
+// us, 10^6 bytes 93.1 -> 87.7, 2^26 symbols of 2 levels 61.1 -> 59.2.  Not the
+// pass itself or the queries: their CTAs then start packed onto fewer SMs
+// (10^6 bytes 104 and 112 us).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);  // an error is also the next cudaGetLastError's
+}
+
 }  // namespace pwmgpu

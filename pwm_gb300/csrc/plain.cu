@@ -247,10 +247,11 @@ constexpr uint64_t kDoubleTileMin = uint64_t(1) << 24;  // symbols, up to 4 leve
 // 8 levels of bytes in one pass: its tiles cost more than two 4-level passes
 // (127 runs at the deepest level), but a text saves the second pass, the
 // host's plan of it and the regroup.  One pass against two: both structures
-// 36 and 86 us at 2^20 bytes, 131 and 160 at 2^24, 236 and 233 at 2^25, 432
-// and 388 at 2^26; the matrix alone 207 and 235 at 2^25, 368 and 361 at 2^26.
-constexpr uint64_t kOnePass8Tree = uint64_t(30) << 20;    // symbols, with a tree
-constexpr uint64_t kOnePass8Matrix = uint64_t(60) << 20;  // a matrix alone
+// 48 and 88 us at 2^22 bytes, 116 and 130 at 2^24, 166 either way at 24 2^20,
+// 195 and 189 at 30 2^20, 356 and 302 at 60 2^20; the matrix alone 144 and 156
+// at 24 2^20, 215 and 213 at 40 2^20, 302 and 278 at 60 2^20.
+constexpr uint64_t kOnePass8Tree = uint64_t(24) << 20;    // symbols, with a tree
+constexpr uint64_t kOnePass8Matrix = uint64_t(40) << 20;  // a matrix alone
 
 void build_one_pass(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text) {
   cudaStream_t s = ctx->stream;

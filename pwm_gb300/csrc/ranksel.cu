@@ -112,6 +112,8 @@ __device__ __forceinline__ bool thread_block_select(const uint64_t* data, uint64
 // 512-bit L2 block; the counts are then gathered so that lane b holds block
 // b's.
 __global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSelectArgs a) {
+  chain_next();
+  chain_wait();
   const uint32_t y = blockIdx.x;
   RankSelectLevel L, twin{};
   bool twinned = false;
@@ -750,7 +752,7 @@ void launch_rank_select(const RankSelectArgs& a, uint64_t max_words, cudaStream_
   const uint32_t levels = a.nfirst + a.nsecond;
   if (levels == 0) return;
   const dim3 grid(levels, unsigned(rank_select_state_words(max_words) - 1));  // at most 8192 CTAs a level (2^32 bits)
-  rank_select_kernel<<<grid, kRsThreads, 0, s>>>(a);
+  launch_chained(rank_select_kernel, grid, kRsThreads, 0, s, a);
   ++*launches;
 }
 

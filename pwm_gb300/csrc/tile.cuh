@@ -715,9 +715,10 @@ __device__ __forceinline__ void warp_exclusive_scan(const uint32_t* in, uint32_t
 // Planes of 32 keys of one byte (key i in byte i % 4 of w[i / 4]): pl[j] has
 // bit lo + K-1-j of key i in bit 31-i.  A byte transpose puts the keys of
 // every eighth place into one word, then 4x4 bit transposes inside its
-// nibbles: 44 operations for 4 planes.  lo + K <= 8.
+// nibbles: 44 operations for 4 planes.  lo + K <= 8; four planes take any lo
+// if `bits` masks off the bits of lo .. lo + 3 that a key does not have.
 template <int K>
-__device__ __forceinline__ void key_planes(const uint32_t (&w)[8], uint32_t lo, uint32_t (&pl)[K]) {
+__device__ __forceinline__ void key_planes(const uint32_t (&w)[8], uint32_t lo, uint32_t (&pl)[K], uint32_t bits = 15u) {
   uint32_t x[8];  // byte 3-q of x[j]: key 8q + j
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -733,8 +734,12 @@ __device__ __forceinline__ void key_planes(const uint32_t (&w)[8], uint32_t lo, 
     uint32_t n[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const uint32_t hi = K == 4 ? x[j] << (4 - lo) : (x[j] >> (lo + b0)) << 4;
-      n[j] = (hi & 0xF0F0F0F0u) | ((x[4 + j] >> (lo + b0)) & 0x0F0F0F0Fu);
+      if constexpr (K == 4) {
+        n[j] = (__funnelshift_l(x[j], x[j], 4 - lo) & (bits * 0x10101010u)) |
+               (__funnelshift_r(x[4 + j], x[4 + j], lo) & (bits * 0x01010101u));
+      } else {
+        n[j] = (((x[j] >> (lo + b0)) << 4) & 0xF0F0F0F0u) | ((x[4 + j] >> (lo + b0)) & 0x0F0F0F0Fu);
+      }
     }
     const uint32_t a0 = (n[0] & 0xCCCCCCCCu) | ((n[2] >> 2) & 0x33333333u);
     const uint32_t a2 = ((n[0] << 2) & 0xCCCCCCCCu) | (n[2] & 0x33333333u);
@@ -1138,6 +1143,8 @@ __device__ __forceinline__ void tile_rank_keys(const TileArgs& a, const TileSeg&
     kw[4 * r] = x.x, kw[4 * r + 1] = x.y, kw[4 * r + 2] = x.z, kw[4 * r + 3] = x.w;
   }
   const uint32_t lo = shift - uint32_t(K - 1);
+  // (a text can have more levels than its symbols have bits: the top ones are all 0)
+  const uint32_t bits = lo + K <= 8 * KB ? 15u : (lo >= 8 * KB ? 0u : (1u << (8 * KB - lo)) - 1u);
   uint32_t cnt[NB / 2];  // digits 2q and 2q+1 (key_4: bit t is plane t) in halves
 #pragma unroll
   for (int q = 0; q < NB / 2; ++q) cnt[q] = 0;
@@ -1156,7 +1163,7 @@ __device__ __forceinline__ void tile_rank_keys(const TileArgs& a, const TileSeg&
                            0x5410);
       }
     }
-    key_planes<K>(w, KB == 1 ? lo : 0u, pl);
+    key_planes<K>(w, KB == 1 ? lo : 0u, pl, bits);
     const uint32_t wi = uint32_t(tid * WPT + k), vm = plane_word_valid(n, wi);
 #pragma unroll
     for (int j = 0; j < K; ++j) {
@@ -1235,7 +1242,7 @@ __device__ __forceinline__ void tile_rank_keys(const TileArgs& a, const TileSeg&
 #pragma unroll
     for (int i = 0; i < BATCHED; ++i) {
       const uint32_t w = kw[(i0 + i) * KB / 4], b = uint32_t(8 * KB * ((i0 + i) % (4 / KB)));
-      const uint32_t col = (__funnelshift_l(w, w, 10u - b - lo) & (15u << 10)) | uint32_t(tid * 4);  // digit * 1024
+      const uint32_t col = (__funnelshift_l(w, w, 10u - b - lo) & (bits << 10)) | uint32_t(tid * 4);  // digit * 1024
       at[i] = 0;
       if (uint32_t(i) < count)
         asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(at[i]) : "r"(cbase + col), "n"(KO) : "memory");
@@ -1807,6 +1814,7 @@ template <typename KeyT, int K, bool OUT, int THREADS, int V, typename KeyO = Ke
 __global__ void __launch_bounds__(THREADS, tile_threads_per_sm<KeyT, K, V, PLANES>() / THREADS)
     tile_pass_kernel(TileArgs a) {
   __shared__ uint32_t s_g;
+  chain_next();  // rank/select may follow
   if (threadIdx.x == 0) s_g = a.tile_base + atomicAdd(a.tile_counter, 1u);
   __syncthreads();
   tile_pass_body<KeyT, K, OUT, THREADS, V, false, KeyO, PLANES>(a, s_g);

@@ -13,13 +13,14 @@ SIZES = [1, 31, 32, 33, 63, 64, 65, 127, 129, 4095, 8191, 8193, 16383, 16384, 16
 
 
 @pytest.mark.parametrize("shape", [(True, True), (True, False), (False, True)])
-@pytest.mark.parametrize("width,L", [(1, 8), (1, 6), (2, 9), (2, 12), (2, 16), (4, 11), (4, 14), (4, 18)])
+@pytest.mark.parametrize("width,L", [(1, 8), (1, 6), (1, 9), (1, 11), (1, 13), (2, 9), (2, 12), (2, 16), (2, 17),
+                                     (2, 22), (4, 11), (4, 14), (4, 18)])
 def test_levels(pg, orc, width, L, shape):
     torch = pytest.importorskip("torch")
     ctx = pg.Context()
     ctx.set_pass_levels(4)
     rng = np.random.default_rng(L)
-    top = (1 << L) - 1
+    top = (1 << min(L, 8 * width)) - 1
     for n in SIZES:
         for kind in ("skewed", "even"):
             if kind == "skewed":
