@@ -15,42 +15,82 @@ __device__ __forceinline__ uint32_t rev_bits_dev(uint32_t v, uint32_t bits) {
   return bits == 0 ? 0u : (__brev(v) >> (32 - bits));
 }
 
-// Counts of one chunk (whole first-pass tiles) of an 8-bit text of L = 2..4
-// levels by planes (plane_count.cuh): the finest runs of every tile, their
-// prefixes in the chunk and totals, and the text's histogram.
-template <int L>
+constexpr uint32_t kHistColumns = 256 * 32;  // 8-bit symbols x lanes
+
+// Counts of one chunk (whole first-pass tiles) of an 8-bit text by planes
+// (plane_count.cuh): the finest runs of every tile, their prefixes in the chunk
+// and totals, and the text's histogram.  FULL = false: texts of L = 2..4
+// levels, whose runs and histogram both follow from the L planes.  FULL: texts
+// of more, the runs from planes of the top L = 4 levels, the histogram an
+// atomic a symbol into a column per lane (h: 256 x 32; with two atomics a symbol
+// and 16 columns the counts of 4096 uneven texts, 85% of 3 levels, took 318 us,
+// now 269; at 4 CTAs an SM 302, at 6, 40 registers, 285).
+template <int L, bool FULL>
 __device__ __forceinline__ void batch_hist_planes(const uint8_t* text, const BatchChunk& c, uint32_t ntiles,
-                                                  uint32_t* smem, unsigned long long* hist, uint32_t* tilecnt,
-                                                  uint32_t* relpre, unsigned long long* blocksum, uint32_t* status) {
+                                                  uint32_t levels, uint32_t* smem, unsigned long long* hist,
+                                                  uint32_t* tilecnt, uint32_t* relpre, unsigned long long* blocksum,
+                                                  uint32_t* status) {
   constexpr int WARPS = kBatchThreads / 32;
-  constexpr uint32_t NB = 1u << (L - 1);  // D = L - 1: every text of up to 4 levels takes one pass
-  auto* pairs = reinterpret_cast<uint32_t (*)[WARPS][8]>(smem);  // [2]
-  const uint32_t tid = threadIdx.x, T = 1u << c.log2T;
+  constexpr int D = FULL ? L : L - 1;  // levels of the finest runs: every text of up to 4 levels takes one pass
+  constexpr uint32_t NB = 1u << D;
+  uint32_t* h = smem;
+  auto* pairs = reinterpret_cast<uint32_t (*)[WARPS][8]>(smem + (FULL ? kHistColumns : 0));  // [2]
+  const uint32_t tid = threadIdx.x, lane = tid & 31, T = 1u << c.log2T;
   const int nv = int(T / (16 * kBatchThreads));  // 1, 2, 4 or 8 vectors a thread
+  if constexpr (FULL) {
+    for (uint32_t i = tid; i < kHistColumns; i += kBatchThreads) h[i] = 0;
+    __syncthreads();
+  }
   uint32_t rel = 0, mine = 0, seen = 0;
   for (uint32_t k = 0; k < ntiles; ++k) {
     const uint64_t start = uint64_t(k) << c.log2T;
     const uint32_t len = uint32_t(c.len - start < T ? c.len - start : T);
-    count_tile_planes<L, kBatchThreads, 8>(text + start, len, nv, seen, pairs[k & 1], [](int, uint32_t, const uint4&) {});
+    count_tile_planes<L, kBatchThreads, FULL ? 4 : 8>(
+        text + start, len, nv, seen, pairs[k & 1],
+        [&](int, uint32_t i, const uint4& v) {
+          if constexpr (FULL) {
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            if (16 * i + 16 <= len) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) atomicAdd(&h[((w[e >> 2] >> (8 * (e & 3))) & 0xFFu) * 32 + lane], 1u);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 16; ++e)
+                if (16 * i + e < len) atomicAdd(&h[((w[e >> 2] >> (8 * (e & 3))) & 0xFFu) * 32 + lane], 1u);
+            }
+          }
+        },
+        FULL ? levels - L : 0u);
     __syncthreads();
     const uint32_t (*pr)[8] = pairs[k & 1];
     if (tid < NB) {
-      const uint32_t q = __brev(tid) >> (32 - (L - 1));
+      const uint32_t q = __brev(tid) >> (32 - D);
       uint32_t x = 0;
 #pragma unroll
-      for (int w = 0; w < WARPS; ++w) x += (pr[w][q] & 0xFFFFu) + (pr[w][q] >> 16);
+      for (int w = 0; w < WARPS; ++w)
+        x += FULL ? (pr[w][q >> 1] >> (16 * (q & 1))) & 0xFFFFu : (pr[w][q] & 0xFFFFu) + (pr[w][q] >> 16);
       tilecnt[c.cnt_off + k * NB + tid] = x;
       relpre[c.cnt_off + k * NB + tid] = rel;
       rel += x;
-    } else if (tid >= 32 && tid < 32 + (1u << L)) {
+    } else if (!FULL && tid >= 32 && tid < 32 + (1u << L)) {
       const uint32_t s = tid - 32;
 #pragma unroll
       for (int w = 0; w < WARPS; ++w) mine += (pr[w][s >> 1] >> (16 * (s & 1))) & 0xFFFFu;
     }
   }
-  if (seen & ~(((1u << L) - 1u) * 0x01010101u)) atomicOr(status, kErrSymbol);
+  const uint32_t allowed = FULL ? (levels >= 8 ? 0xFFu : (1u << levels) - 1u) : (1u << L) - 1u;
+  if (seen & ~(allowed * 0x01010101u)) atomicOr(status, kErrSymbol);
   if (tid < NB) blocksum[c.blk_off + tid] = rel;
-  if (tid >= 32 && tid < 32 + (1u << L) && mine) atomicAdd(&hist[tid - 32], (unsigned long long)mine);
+  if constexpr (FULL) {
+    __syncthreads();
+    for (uint32_t s = tid; s <= allowed; s += kBatchThreads) {
+      for (uint32_t q = 0; q < 32; ++q) mine += h[s * 32 + ((q + lane) & 31)];
+      if (mine) atomicAdd(&hist[s], (unsigned long long)mine);
+      mine = 0;
+    }
+  } else {
+    if (tid >= 32 && tid < 32 + (1u << L) && mine) atomicAdd(&hist[tid - 32], (unsigned long long)mine);
+  }
 }
 
 // Leaf histogram of one chunk of one text (2^L <= 4096 bins in shared
@@ -62,9 +102,9 @@ __device__ __forceinline__ void batch_hist_planes(const uint8_t* text, const Bat
 // batch also counts, per first-pass tile, the tile's finest runs (the
 // D-bit digit of the top symbol bits, counter = the digit bit-reversed), a
 // column per lane, for the pass's given prefixes.
-constexpr uint32_t kHistTileCounters = 16 * 16 * 32;  // tiles x counters x lanes
+constexpr uint32_t kHistTileCounters = 16 * 16 * 32;  // tiles x counters x lanes (2- and 4-byte symbols)
 template <typename T>
-__global__ void __launch_bounds__(kBatchThreads) batch_hist_kernel(const T* __restrict__ texts,
+__global__ void __launch_bounds__(kBatchThreads, sizeof(T) == 1 ? 5 : 1) batch_hist_kernel(const T* __restrict__ texts,
                                                                    const BatchChunk* __restrict__ chunks,
                                                                    const BatchText* __restrict__ info,
                                                                    unsigned long long* hist, uint32_t* tilecnt,
@@ -81,18 +121,21 @@ __global__ void __launch_bounds__(kBatchThreads) batch_hist_kernel(const T* __re
   const uint32_t mine = threadIdx.x % copies, lane = threadIdx.x & 31;
   const uint32_t D = c.D, dsh = t.levels - c.D;  // the digit: symbol bits [L-D, L)
   const uint32_t ntiles = D ? uint32_t((c.len + (uint64_t(1) << c.log2T) - 1) >> c.log2T) : 0u;
-  // Up to 16 bins: counts per (tile, bin) serve both the text's histogram and
-  // the tiles' finest-run counts (each a sum over bins), of 8-bit texts by
-  // planes, of wider ones a counter per (tile, bin, lane) and one shared atomic
-  // per symbol; else a text histogram (per-thread copies) and the tiles' digit
-  // counters.
+  // 8-bit texts with first-pass tiles by planes.  Wider ones of up to 16 bins:
+  // counts per (tile, bin) serve both the text's histogram and the tiles'
+  // finest-run counts (each a sum over bins), a counter per (tile, bin, lane)
+  // and one shared atomic per symbol; else a text histogram (per-thread copies)
+  // and the tiles' digit counters.
   const bool by_tile = D && bins <= 16;
   if constexpr (sizeof(T) == 1) {
-    if (by_tile) {
+    if (D) {
+      const uint8_t* text = texts + t.offset + c.start;
+      unsigned long long* out = hist + t.hist_off;
       switch (t.levels) {
-        case 2: batch_hist_planes<2>(texts + t.offset + c.start, c, ntiles, hsm, hist + t.hist_off, tilecnt, relpre, blocksum, status); break;
-        case 3: batch_hist_planes<3>(texts + t.offset + c.start, c, ntiles, hsm, hist + t.hist_off, tilecnt, relpre, blocksum, status); break;
-        default: batch_hist_planes<4>(texts + t.offset + c.start, c, ntiles, hsm, hist + t.hist_off, tilecnt, relpre, blocksum, status); break;
+        case 2: batch_hist_planes<2, false>(text, c, ntiles, t.levels, hsm, out, tilecnt, relpre, blocksum, status); break;
+        case 3: batch_hist_planes<3, false>(text, c, ntiles, t.levels, hsm, out, tilecnt, relpre, blocksum, status); break;
+        case 4: batch_hist_planes<4, false>(text, c, ntiles, t.levels, hsm, out, tilecnt, relpre, blocksum, status); break;
+        default: batch_hist_planes<4, true>(text, c, ntiles, t.levels, hsm, out, tilecnt, relpre, blocksum, status); break;
       }
       return;
     }
@@ -330,7 +373,7 @@ template <typename T>
 void launch_hist_w(const void* texts, const BatchChunk* chunks, uint32_t nchunks, const BatchText* info,
                    unsigned long long* hist, uint32_t* tilecnt, uint32_t* relpre, unsigned long long* blocksum,
                    uint32_t* status, cudaStream_t s) {
-  constexpr size_t smem = (4096 + kHistTileCounters) * 4;
+  constexpr size_t smem = (sizeof(T) == 1 ? kHistColumns + 2 * (kBatchThreads / 32) * 8 : 4096 + kHistTileCounters) * 4;
   static bool configured = false;  // attribute set once per width
   if (!configured) {
     cudaFuncSetAttribute(batch_hist_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));

@@ -68,10 +68,11 @@ __device__ __forceinline__ void count_planes(const uint4& a, const uint4& b, uin
 // to pairs[warp][i], value 2 i in the low half, 2 i + 1 in the high one.
 // each(r, i, v): vector i (symbols 16 i.. of the tile; cut off at n, zero
 // past it) is v, the thread's r-th; called by whole warps.  seen: OR of the
-// symbols.
+// symbols.  shift: the values counted are the symbols' bits shift .. shift +
+// L - 1.
 template <int L, int THREADS, int VMAX, typename F>
 __device__ __forceinline__ void count_tile_planes(const unsigned char* p, uint32_t n, int nv, uint32_t& seen,
-                                                  uint32_t (*pairs)[8], F&& each) {
+                                                  uint32_t (*pairs)[8], F&& each, uint32_t shift = 0) {
   const uint32_t tid = threadIdx.x, nvec = (n + 15) >> 4;
   const uint32_t off = uint32_t(reinterpret_cast<uintptr_t>(p) & 15);
   const uint4* av = reinterpret_cast<const uint4*>(p - off);
@@ -86,7 +87,8 @@ __device__ __forceinline__ void count_tile_planes(const unsigned char* p, uint32
       if (off) v[r] = realign16(v[r], i + 1 <= last_block ? __ldcs(av + i + 1) : make_uint4(0u, 0u, 0u, 0u), off);
     }
   }
-  constexpr uint32_t kBits = ((1u << L) - 1u) * 0x01010101u;
+  // (a text may have more levels than 8: bits above a symbol's are 0)
+  const uint32_t kBits = (shift + L <= 8 ? (1u << L) - 1u : (shift >= 8 ? 0u : (1u << (8 - shift)) - 1u)) * 0x01010101u;
   uint32_t cnt[1 << L], counted = 0, valid = 0;
 #pragma unroll
   for (int k = 0; k < (1 << L); ++k) cnt[k] = 0;
@@ -99,7 +101,8 @@ __device__ __forceinline__ void count_tile_planes(const unsigned char* p, uint32
     valid += uint32_t(k);
     each(r, i, v[r]);
     seen |= v[r].x | v[r].y | v[r].z | v[r].w;
-    v[r] = make_uint4(v[r].x & kBits, v[r].y & kBits, v[r].z & kBits, v[r].w & kBits);
+    v[r] = make_uint4((v[r].x >> shift) & kBits, (v[r].y >> shift) & kBits, (v[r].z >> shift) & kBits,
+                      (v[r].w >> shift) & kBits);
   }
 #pragma unroll
   for (int r = 0; r < VMAX; r += 2) {
