@@ -243,12 +243,13 @@ __global__ void __launch_bounds__(kTileHistThreads) tile_hist_kernel(const T* te
 }
 
 // The same for 8-bit texts of 2 to 4 levels, counted by planes
-// (plane_count.cuh): 2^26 symbols of 2 levels 34 -> 20 us, where an atomic a
-// symbol bounded it.  Per tile one barrier: the warps' sums lie in one of two
+// (plane_count.cuh): 2^26 symbols of 2 levels 34 us by an atomic a symbol, 19
+// so (23 at the 2 CTAs an SM of its own choice of registers; 2^28 of 3 levels
+// 94 and 76).  Per tile one barrier: the warps' sums lie in one of two
 // buffers, so the threads that add them up (one a run, one a symbol value) read
 // one while the next tile fills the other.
 template <int L>
-__global__ void __launch_bounds__(kTileHistThreads) tile_hist_planes_kernel(
+__global__ void __launch_bounds__(kTileHistThreads, 4) tile_hist_planes_kernel(
     const uint8_t* text, uint64_t n, uint32_t tile_keys, uint32_t tiles_per_block, uint32_t block0,
     unsigned long long* hist, uint32_t* tilecnt, uint32_t* relpre, unsigned long long* blocksum, uint64_t* level0_a,
     uint64_t* level0_b, uint32_t* status) {
