@@ -43,7 +43,10 @@ namespace pwmgpu {
 // A structure in one allocation: its words, zero counts, and with rank/select
 // the blocks of every level and their descriptors.  As five allocations and two
 // copies, 64 requests of a server with 8 slots spent 10 ms of its threads' time
-// in them: 4.60 -> 3.06 ms the requests.
+// in them: 4.60 -> 3.06 ms the requests.  Without a stream (cudaMalloc) the words
+// have one of their own, first: past 1 MiB an allocation maps memory of its own
+// (both structures of 10^6 bytes created and freed: five allocations each 104 us,
+// one 271, two 65).
 // stream: where the structure is built (its words are zeroed there, so that
 // the first build comes after).
 void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint64_t n, bool tree, bool huff,
@@ -62,7 +65,7 @@ void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint
     return o;
   };
   const size_t word_bytes = std::max<uint64_t>(s.total_words, 16) * 8, nl = std::max<uint32_t>(s.levels, 1);
-  take(word_bytes);
+  if (alloc_stream) take(word_bytes);
   const size_t off_zeros = take(nl * 8);
   std::vector<size_t> off0(s.levels), off12(s.levels), offs0(s.levels), offs1(s.levels), offm(s.levels);
   size_t off_desc = 0;
@@ -78,11 +81,12 @@ void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint
     off_desc = take((sizeof(RankSelectLevel) + sizeof(QueryLevel)) * nl);
   }
   void* slab = nullptr;
+  if (!alloc_stream) CUDA_TRY(cudaMalloc(&s.words_slab, word_bytes));
   if (alloc_stream) CUDA_TRY(cudaMallocAsync(&slab, bytes, alloc_stream));
   else CUDA_TRY(cudaMalloc(&slab, bytes));
   s.slab = slab;
   char* base = static_cast<char*>(slab);
-  s.d_words = reinterpret_cast<uint64_t*>(base);
+  s.d_words = static_cast<uint64_t*>(alloc_stream ? slab : s.words_slab);
   s.d_zeros = reinterpret_cast<uint64_t*>(base + off_zeros);
   // padding bits and words are never written by a build: zero from here on
   CUDA_TRY(cudaMemsetAsync(s.d_words, 0, word_bytes, stream));

@@ -261,7 +261,8 @@ struct Structure {
   uint64_t n = 0;
   std::vector<uint64_t> bits, offs;
   uint64_t total_words = 0;
-  void* slab = nullptr;          // the one allocation that holds everything below
+  void* slab = nullptr;          // the allocation that holds everything below
+  void* words_slab = nullptr;    // the words' own one, where they have it (alloc_structure)
   uint64_t* d_words = nullptr;
   std::vector<uint64_t> zeros;   // host (matrix)
   uint64_t* d_zeros = nullptr;   // device copy (matrix), read by queries
@@ -282,11 +283,12 @@ struct Structure {
     total_words = off;
   }
   void release() {
-    if (slab) {
-      if (alloc_stream) cudaFreeAsync(slab, alloc_stream);
-      else cudaFree(slab);
+    for (void* p : {slab, words_slab}) {
+      if (!p) continue;
+      if (alloc_stream) cudaFreeAsync(p, alloc_stream);
+      else cudaFree(p);
     }
-    slab = nullptr;
+    slab = words_slab = nullptr;
     d_words = nullptr; d_zeros = nullptr; d_rs_levels = nullptr; d_q_levels = nullptr;
     rs = false;
   }
