@@ -94,8 +94,9 @@ PWMGPU_API pwmgpu_status pwmgpu_ctx_profile_read(pwmgpu_ctx* ctx, char* buf, uin
 /* Tuning: levels fused into one split pass (1..4; 0 restores the default).
  * A pass reads its input sequence once and writes the bits of that many
  * levels.  Sets the width of both engines.  Defaults: the tile engine builds
- * a text of up to 7 levels in one pass of all its levels and deeper texts in
- * passes of 4; the warp-pass engine uses passes of 2. */
+ * a text of up to 7 levels, and an 8-bit one of 8 levels of up to some 10^7
+ * symbols, in one pass of all its levels and others in passes of 4; the
+ * warp-pass engine uses passes of 2. */
 PWMGPU_API pwmgpu_status pwmgpu_ctx_set_pass_levels(pwmgpu_ctx* ctx, int levels_per_pass);
 
 /* Stream-ordered device allocations (cudaMallocAsync / cudaFreeAsync on the

@@ -177,16 +177,6 @@ struct TileCfg {
   static constexpr size_t ranked_smem_bytes() { return ranked_area(); }
 };
 
-// Bit q of the 8 keys of w0 (keys 0-3, key k in byte k) and w1 (keys 4-7),
-// key 0 in bit 7 of the result (higher bits are not cleared).  The 8 bits are
-// spread to byte bit 0 (w1) and bit 4 (w0) and collected by one 32x32->64-bit
-// multiply by 2^4 + 2^13 + 2^22 + 2^31: the 32 partial products land on
-// distinct bit positions, so no carries disturb bits 28-35.
-__device__ __forceinline__ uint32_t key_bits8(uint32_t w0, uint32_t w1, int q) {
-  const uint32_t t0 = (w0 >> q) & 0x01010101u, t1 = (w1 >> q) & 0x01010101u;
-  return uint32_t((uint64_t(t0 * 16u + t1) * 0x80402010ull) >> 28);
-}
-
 // Split bits of the keys of one 16-byte vector, MSB first: bit KPL-1-i is the
 // bit of key i.
 template <typename KeyT>
@@ -196,8 +186,7 @@ __device__ __forceinline__ uint32_t vector_bits(const uint4& v, uint32_t sh) {
   uint32_t m = 0;
   if constexpr (sizeof(KeyT) == 1) {
     // byte k of a word lands at bit 3-k: ((w >> sh) & 0x01010101) * 0x80402010 >> 28
-    // (one 32-bit multiply per word measured faster in this form than
-    // key_bits8's 64-bit multiply per two words)
+    // (one 32-bit multiply per word; a 64-bit one per two words was slower)
 #pragma unroll
     for (int q = 0; q < 4; ++q) m |= ((((w[q] >> sh) & 0x01010101u) * 0x80402010u) >> 28) << (12 - 4 * q);
   } else if constexpr (sizeof(KeyT) == 2) {

@@ -4,11 +4,13 @@
 // segment, the barriers and scans of every split, the set-up of each of its 44
 // runs.  With 8 vectors a thread (32768 keys of 8 bits, 16384 of 16, 8192 of
 // 32; 80 registers, 3 CTAs an SM) they serve twice as many, and the runs are
-// twice as long.  Measured (GB300), whole builds: 2^30 bytes, both structures
-// of 8 levels, 5.55 -> 5.00 ms; 2^28 16-bit symbols, 16 levels, 4.79 -> 4.40;
-// 2^26 32-bit symbols, the matrix of 20 levels, 1.87 -> 1.64 (with 4 CTAs an SM
-// at 64 registers 16-bit 4.55, 32-bit 1.72).  Texts too short to fill the SMs
-// with such tiles keep the usual ones.
+// twice as long.  Measured (GB300), whole builds with keys split bit by bit:
+// 2^30 bytes, both structures of 8 levels, 5.55 -> 5.00 ms; 2^28 16-bit
+// symbols, 16 levels, 4.79 -> 4.40; 2^26 32-bit symbols, the matrix of 20
+// levels, 1.87 -> 1.64 (with 4 CTAs an SM at 64 registers 16-bit 4.55, 32-bit
+// 1.72).  Sorted by 4 bits at once (tile_rank_keys) passes in these tiles take
+// 517 us for 2^28 8-bit keys and 211 for 2^26 16-bit ones, in the usual ones
+// 563 and 270.  Texts too short to fill the SMs with such tiles keep those.
 #include "kernels.cuh"
 #include "tile_launch.cuh"
 
