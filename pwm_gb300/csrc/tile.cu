@@ -12,7 +12,9 @@ void launch_k(int K, const TileArgs& a, cudaStream_t s) {
     case 1: launch_tile_one<KeyT, 1, OUT, KeyO, PLANES>(a, s); break;
     case 2: launch_tile_one<KeyT, 2, OUT, KeyO, PLANES>(a, s); break;
     case 3: launch_tile_one<KeyT, 3, OUT, KeyO, PLANES>(a, s); break;
-    default: launch_tile_one<KeyT, 4, OUT, KeyO, PLANES>(a, s); break;
+    default:  // (4-byte keys that write S_{l+4} have tiles of 8 or 16 vectors: tile_wide.cu)
+      if constexpr (!OUT || sizeof(KeyT) < 4) launch_tile_one<KeyT, 4, OUT, KeyO, PLANES>(a, s);
+      break;
   }
 }
 
@@ -46,7 +48,9 @@ void launch_tile_pass(uint32_t key_bytes, uint32_t out_bytes, int K, bool out, c
   // beyond 4 levels: only as the last pass of a text whose prefixes the histogram gives
   if (deep && (out || !a.blockpre || K > kTileGivenMaxLevels)) return;
   if (out && a.tile_vectors) {
-    if (K != kTileMaxLevels || a.tile_vectors != 2 * uint32_t(kTileVectors)) return;
+    if (K != kTileMaxLevels || (a.tile_vectors != 2 * uint32_t(kTileVectors) &&
+                                (key_bytes != 4 || a.tile_vectors != 4 * uint32_t(kTileVectors))))
+      return;
     launch_tile_pass_wide(key_bytes, out_bytes, a, s);
   } else if (deep || a.tile_vectors) {
     if (a.tile_vectors && key_bytes != 1) return;

@@ -1091,10 +1091,10 @@ __device__ __forceinline__ void tile_rank_keys(const TileArgs& a, const TileSeg&
   constexpr int ITEMS = V * KPL, WPT = ITEMS / 32;
   using C = TileCfg<KeyT, K, true, THREADS, V>;
   constexpr int SBW = C::SBW, WARPS = C::WARPS;
-  static_assert(C::RANKABLE && (V == 4 || V == 8), "whole plane words a thread, rows of 64 or 128 bytes");
+  static_assert(C::RANKABLE && (V == 4 || V == 8 || V == 16), "whole plane words a thread, rows of 64 to 256 bytes");
   static_assert(THREADS == 256, "the cursors' columns");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  auto turn = [](int row) { return V == 8 ? row & 7 : (row >> 1) & 3; };
+  auto turn = [](int row) { return V == 4 ? (row >> 1) & 3 : row & 7; };
   uint4* rows = reinterpret_cast<uint4*>(buf);
   {
     const uintptr_t sa =
@@ -1793,10 +1793,12 @@ __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in)
 // counter.  Threads per SM (registers a thread): the bit-plane form 1536 (40),
 // with double tiles 1280 (48), 1024 (64) for 5-8 levels; the key form over
 // 1-byte keys 1280 (48), over wider keys 1024 (64; at 48 they spill more and
-// measured slower), 768 (80) with double tiles and for 5-8 levels.
+// measured slower), 768 (80) with double tiles and for 5-8 levels, 512 (128)
+// with quadruple ones.
 template <typename KeyT, int K, int V, bool PLANES>
 constexpr int tile_threads_per_sm() {
   if (PLANES) return K > kTileMaxLevels ? (V > 4 ? 768 : 1024) : (V > 4 ? 1280 : 1536);
+  if (V > 8) return 512;
   return K > kTileMaxLevels || V > 4 ? 768 : (sizeof(KeyT) == 1 ? 1280 : 1024);
 }
 template <typename KeyT, int K, bool OUT, int THREADS, int V, typename KeyO = KeyT, bool PLANES = false>

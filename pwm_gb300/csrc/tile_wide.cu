@@ -11,6 +11,11 @@
 // 1.72).  Sorted by 4 bits at once (tile_rank_keys) passes in these tiles take
 // 517 us for 2^28 8-bit keys and 211 for 2^26 16-bit ones, in the usual ones
 // 563 and 270.  Texts too short to fill the SMs with such tiles keep those.
+//
+// 4-byte keys take tiles of 16 vectors (16384 keys, 128 registers, 2 CTAs an
+// SM) in turn: with 32 keys a thread its scans and cursors weigh as much as its
+// keys.  2^25 keys narrowed to 16 bits 169 -> 144 us, 2^26 symbols of 20 levels
+// 1.25 -> 1.20 ms.  (2-byte keys in such tiles: 217 us against 211.)
 #include "kernels.cuh"
 #include "tile_launch.cuh"
 
@@ -19,6 +24,12 @@ namespace pwmgpu {
 namespace {
 template <typename KeyT, typename KeyO>
 void launch(const TileArgs& a, cudaStream_t s) {
+  if constexpr (sizeof(KeyT) == 4) {
+    if (a.tile_vectors == 4 * uint32_t(kTileVectors)) {
+      launch_tile_one<KeyT, kTileMaxLevels, true, KeyO, false, 4 * kTileVectors>(a, s);
+      return;
+    }
+  }
   launch_tile_one<KeyT, kTileMaxLevels, true, KeyO, false, 2 * kTileVectors>(a, s);
 }
 }  // namespace

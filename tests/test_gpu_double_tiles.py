@@ -1,4 +1,4 @@
-"""GPU: tile passes in tiles of 8 vectors a thread, on both sides of the sizes
+"""GPU: tile passes in tiles of 8 or 16 vectors a thread, on both sides of the sizes
 where texts take them: texts of one pass, passes that write the next sequence,
 last passes over narrowed keys; sizes a symbol around a tile's end, every
 symbol width, skewed and even texts, one run a level, texts off a 16-byte
@@ -15,7 +15,8 @@ DT = {1: np.uint8, 2: np.uint16, 4: np.uint32}
 @pytest.mark.parametrize("width,L,edge,tile", [
     (1, 4, 1 << 24, 32768), (1, 3, 1 << 24, 32768), (1, 2, 1 << 24, 32768), (1, 6, 1 << 25, 32768),
     (1, 8, 1 << 25, 32768), (2, 12, 1 << 24, 16384), (2, 11, 1 << 24, 16384), (4, 12, 1 << 23, 8192),
-    (4, 9, 1 << 24, 8192)])
+    (4, 9, 1 << 24, 8192), (2, 16, 1 << 21, 16384), (2, 9, 1 << 21, 16384), (4, 20, 1 << 21, 16384),
+    (4, 11, 1 << 21, 16384), (4, 18, 1 << 13, 8192)])
 def test_sizes_around_the_change(pg, orc, width, L, edge, tile, shape):
     torch = pytest.importorskip("torch")
     rng = np.random.default_rng(L)
