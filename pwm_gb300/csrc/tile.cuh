@@ -33,7 +33,8 @@
 //     publishes them at once; after its splits and the write of the level-l
 //     run (which needs no prefix) the CTA completes the decoupled look-back
 //     (restarted at every segment's first tile; counter-major state, one
-//     coalesced load per counter, 256 predecessors per round trip);
+//     coalesced load per counter and warp, 128 predecessors in the first round
+//     trip, 256 in the later ones);
 //   * writes every run of every level to the matrix and the tree at
 //     table start + look-back prefix in 64-bit words, and the runs of
 //     S_{l+K} to the next pass's input (one warp per run, round-robin; the
@@ -1260,8 +1261,9 @@ __device__ __forceinline__ void tile_rank_keys(const TileArgs& a, const TileSeg&
 // previous pass is done and afterwards counts itself done; otherwise
 // TileText's batch fields are ignored.
 // KeyO: the key type of S_{l+K} (KeyT, or narrower when the levels left
-// after this pass fit it).  PLANES (1-byte keys, a pass without S_{l+K}, up
-// to 4 levels): the splits move bit planes instead of keys.
+// after this pass fit it).  PLANES (1-byte keys, a pass without S_{l+K}): the
+// splits move bit planes instead of keys; so they do in the ranked form (passes
+// of 4 levels that write S_{l+4}, outside batches), which stores the keys once.
 template <typename KeyT, int K, bool OUT, int THREADS, int V, bool BATCH, typename KeyO = KeyT, bool PLANES = false>
 __device__ __forceinline__ void tile_pass_body(const TileArgs& a, uint32_t g_in) {
   using C = TileCfg<KeyT, K, OUT, THREADS, V>;
