@@ -237,12 +237,13 @@ uint32_t tune_key(uint32_t width, uint32_t L, uint64_t n) {
 uint32_t tile_npass(uint32_t L) { return (L + uint32_t(kTileMaxLevels) - 1) / uint32_t(kTileMaxLevels); }
 
 // Tiles of 8 vectors a thread (the single builds' double tiles): last passes
-// over 1-byte keys of texts tuned to 4 vectors that have four such tiles for
-// every segment of the pass.  4096 uneven texts, 85% of 3 levels: the kernel
-// 1.63 -> 1.57 ms (at 64 registers; 1.76 without them, at 48 1.63 either way).
+// over 1-byte keys of texts tuned to 4 vectors that have such a tile for every
+// segment of the pass.  4096 uneven texts, 85% of 3 levels: the kernel 1.63 ->
+// 1.53 ms (at 64 registers; 1.76 without them, at 48 1.63 either way; from two
+// tiles a segment 1.55, from four 1.57).
 bool tile_wide(const pwmgpu_batch* b, uint32_t t, uint32_t l, uint32_t K, bool out) {
   return b->width == 1 && !b->force_vpt && b->vpt[t] == 4 && !out && K >= 2 &&
-         b->info[t].n >= (uint64_t(4) << l) * tile_pass_elems(1, 8);
+         b->info[t].n >= (uint64_t(1) << l) * tile_pass_elems(1, 8);
 }
 
 uint8_t tile_variant(uint32_t K, bool out, bool wide) {

@@ -123,20 +123,24 @@ __global__ void __launch_bounds__(256) tile_batch_fold_kernel(const TileBatchTex
     warp_exclusive_scan_u64(len, [&](uint64_t i) { return c[rev_bits(uint32_t(i), m)]; }, pk + tile_batch_level_at(m),
                             lane);
   }
-  // the first pass's block prefixes: per counter, exclusive sums over the
-  // text's blocks of tiles (lane i takes a run of consecutive blocks)
+  // the first pass's block prefixes: per counter (2 to 16), exclusive sums over
+  // the text's blocks of tiles.  Lanes take the counters side by side, and every
+  // nb-th lane a run of consecutive blocks (a counter after another, all lanes on
+  // its blocks: the kernel 36 us for 4096 texts, so 27).
   const uint32_t nb = t.nb0, nt = t.nblk0;
-  for (uint32_t cn = 0; cn < nb; ++cn) {
-    const uint32_t per = (nt + 31) / 32, b = min(nt, lane * per), e = min(nt, b + per);
+  if (nb) {
+    const uint32_t cn = lane & (nb - 1), part = lane / nb, parts = 32 / nb;
+    const uint32_t per = (nt + parts - 1) / parts, b = min(nt, part * per), e = min(nt, b + per);
     unsigned long long sum = 0;
+#pragma unroll 4
     for (uint32_t i = b; i < e; ++i) sum += blocksum[t.blk_off + uint64_t(i) * nb + cn];
     unsigned long long x = sum;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
+    for (uint32_t d = nb; d < 32; d <<= 1) {
       const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-      if (int(lane) >= d) x += y;
+      if (lane >= d) x += y;
     }
     unsigned long long run = x - sum;
+#pragma unroll 4
     for (uint32_t i = b; i < e; ++i) {
       const uint64_t at = t.blk_off + uint64_t(i) * nb + cn;
       const unsigned long long v = blocksum[at];

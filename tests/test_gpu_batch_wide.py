@@ -17,7 +17,7 @@ def test_wide_texts(pg, orc, tree):
     rng = np.random.default_rng(5)
     parts, levels = [], []
     for L in (1, 2, 3, 4, 7, 8):
-        edge = 4 * TILE if L <= 4 else 64 * TILE  # the last pass's segments: 1 or 16
+        edge = TILE if L <= 4 else 16 * TILE  # the last pass's segments: 1 or 16
         for n in (edge - 1, edge, edge + 1, edge + TILE - 1, edge + TILE + 1, 1000):
             top = (1 << L) - 1
             t = np.minimum(rng.geometric(0.2, n) - 1, top) if n % 2 else rng.integers(0, top + 1, n)
