@@ -199,6 +199,7 @@ pwmgpu_status pwmgpu_ctx_profile_read(pwmgpu_ctx* ctx, char* buf, uint64_t cap) 
 pwmgpu_status pwmgpu_wx_merge(pwmgpu_ctx* ctx, const pwmgpu_wx* const* shards, uint32_t count, pwmgpu_wx* out) {
   if (!ctx || !out || (count && !shards)) return PWMGPU_ERR_ARG;
   return guarded(ctx, [&]() {
+    after_creation(ctx, out);
     merge_shards(ctx, std::vector<const pwmgpu_wx*>(shards, shards + count), out);
     return PWMGPU_OK;
   });
@@ -208,6 +209,7 @@ pwmgpu_status pwmgpu_wx_build_sharded(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void
   if (!ctx || !wx || shards == 0 || (!d_text && wx->n)) return PWMGPU_ERR_ARG;
   if (wx->huffman) return fail(ctx, PWMGPU_ERR_ARG, "a Huffman-shaped wx is built by pwmgpu_wx_build_huffman");
   return guarded(ctx, [&]() {
+    after_creation(ctx, wx);
     d_text = build_input(ctx, wx, d_text);
     if (shards == 1 || wx->n == 0) {
       build_plain(ctx, wx, d_text);
@@ -254,7 +256,11 @@ pwmgpu_status pwmgpu_wx_create(pwmgpu_ctx* ctx, uint64_t size, uint32_t word_wid
     if (!(shape_flags & (PWMGPU_MATRIX | PWMGPU_TREE))) throw Fail{PWMGPU_ERR_ARG, "need PWMGPU_MATRIX or PWMGPU_TREE"};
     if ((shape_flags & PWMGPU_RANK_SELECT) && size >= 4294967295ull - 64)
       throw Fail{PWMGPU_ERR_ARG, "rank/select support needs levels below 2^32-1 bits"};
-    *out = make_wx(ctx, size, word_width, levels, shape_flags).release();
+    auto wx = make_wx(ctx, size, word_width, levels, shape_flags);
+    if (!ctx->created->event) CUDA_TRY(cudaEventCreateWithFlags(&ctx->created->event, cudaEventDisableTiming));
+    CUDA_TRY(cudaEventRecord(ctx->created->event, ctx->stream));
+    wx->created = ctx->created;
+    *out = wx.release();
     return PWMGPU_OK;
   });
 }
@@ -263,6 +269,7 @@ pwmgpu_status pwmgpu_wx_build(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text
   if (!ctx || !wx || (!d_text && wx->n)) return PWMGPU_ERR_ARG;
   if (wx->huffman) return fail(ctx, PWMGPU_ERR_ARG, "a Huffman-shaped wx is built by pwmgpu_wx_build_huffman");
   return guarded(ctx, [&]() {
+    after_creation(ctx, wx);
     build_plain(ctx, wx, build_input(ctx, wx, d_text));
     return PWMGPU_OK;
   });
@@ -272,6 +279,7 @@ pwmgpu_status pwmgpu_wx_build_host(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* h
   if (!ctx || !wx || (!host_text && wx->n)) return PWMGPU_ERR_ARG;
   if (wx->huffman) return fail(ctx, PWMGPU_ERR_ARG, "a Huffman-shaped wx is built by pwmgpu_wx_build_huffman");
   return guarded(ctx, [&]() {
+    after_creation(ctx, wx);
     if (wx->in_width == 5) {
       build_plain(ctx, wx, upload_wide_host_text(ctx, wx, host_text));
       return PWMGPU_OK;
@@ -291,6 +299,7 @@ pwmgpu_status pwmgpu_wx_compute_host(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void*
   if ((wm_bv && (!wx->wm.present || wx->wm_internal)) || (wt_bv && !wx->wt.present))
     return fail(ctx, PWMGPU_ERR_ARG, "an output structure the wx does not hold");
   return guarded(ctx, [&]() {
+    after_creation(ctx, wx);
     HostIO io;
     io.wm = wm_bv;
     io.wt = wt_bv;
@@ -339,6 +348,7 @@ pwmgpu_status pwmgpu_wx_download(pwmgpu_ctx* ctx, const pwmgpu_wx* wx, int which
   const Structure& s = which ? wx->wt : wx->wm;
   if (!s.present) return PWMGPU_ERR_ARG;
   return guarded(ctx, [&]() {
+    after_creation(ctx, wx);
     device_to_host(ctx, bv, s.d_words, s.total_words * 8, ctx->stream);
     if (zeros && !s.is_tree) std::memcpy(zeros, s.zeros.data(), s.levels * 8);
     return PWMGPU_OK;
@@ -351,6 +361,7 @@ pwmgpu_status pwmgpu_wx_rank_select_blocks(pwmgpu_ctx* ctx, const pwmgpu_wx* wx,
   const Structure& s = which ? wx->wt : wx->wm;
   if (!s.present || !s.rs || level >= s.levels) return PWMGPU_ERR_ARG;
   return guarded(ctx, [&]() {
+    after_creation(ctx, wx);
     const RankSelectLevel& r = s.rs_levels[level];
     uint64_t meta[3];
     CUDA_TRY(cudaMemcpyAsync(meta, r.meta, 24, cudaMemcpyDeviceToHost, ctx->stream));
@@ -375,6 +386,7 @@ pwmgpu_status pwmgpu_wx_query(pwmgpu_ctx* ctx, const pwmgpu_wx* wx, int which, i
   if (!s.present || !s.rs || (which == 0 && wx->wm_internal))
     return fail(ctx, PWMGPU_ERR_ARG, "queries need a structure with rank/select");
   return guarded(ctx, [&]() {
+    after_creation(ctx, wx);
     QueryStructure q{s.levels, s.is_tree ? 1u : 0u, s.n, s.d_q_levels, s.d_zeros};
     ProfScope ps(ctx, "queries", count * 24);
     if (s.huffman) launch_huff_queries(q, wx->hq, op, d_a, d_b, count, d_out, ctx->stream, &ctx->launches);
@@ -392,6 +404,7 @@ pwmgpu_status pwmgpu_wx_query_host(pwmgpu_ctx* ctx, const pwmgpu_wx* wx, int whi
   if (!s.present || !s.rs || (which == 0 && wx->wm_internal))
     return fail(ctx, PWMGPU_ERR_ARG, "queries need a structure with rank/select");
   return guarded(ctx, [&]() {
+    after_creation(ctx, wx);
     auto* d = static_cast<uint64_t*>(ctx->grow("query_io", count * 3 * 8));
     cudaStream_t st = ctx->stream;
     CUDA_TRY(cudaMemcpyAsync(d, a, count * 8, cudaMemcpyHostToDevice, st));
@@ -420,6 +433,7 @@ pwmgpu_status pwmgpu_wx_query_batch_host(pwmgpu_ctx* ctx, const pwmgpu_wx* wx, i
     return fail(ctx, PWMGPU_ERR_ARG, "queries need a structure with rank/select");
   if (s.huffman) return fail(ctx, PWMGPU_ERR_ARG, "mixed query batches need a plain structure");
   return guarded(ctx, [&]() {
+    after_creation(ctx, wx);
     // a, b and the kinds staged in pinned memory and uploaded in one copy;
     // on the device the answers follow them (8-byte aligned)
     const uint64_t in_bytes = count * 16 + count, out_off = count * 2 + (count + 7) / 8;

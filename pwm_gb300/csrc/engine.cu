@@ -47,8 +47,8 @@ namespace pwmgpu {
 // have one of their own, first: past 1 MiB an allocation maps memory of its own
 // (both structures of 10^6 bytes created and freed: five allocations each 104 us,
 // one 271, two 65).
-// stream: where the structure is built (its words are zeroed there, so that
-// the first build comes after).
+// stream: the context's (its words are zeroed there, so that a build on it
+// comes after; one of another context waits for them, after_creation).
 void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint64_t n, bool tree, bool huff,
                      bool rank_select, cudaStream_t stream, cudaStream_t alloc_stream) {
   s.release();

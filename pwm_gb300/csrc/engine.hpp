@@ -61,6 +61,17 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
+// Recorded on a context's stream after every wx it creates (the words are
+// zeroed there); each of those structures shares it, so that another context
+// can wait for it whether or not the first still exists.  A later record only
+// makes that wait longer.
+struct CreationEvent {
+  cudaEvent_t event = nullptr;
+  ~CreationEvent() {
+    if (event) cudaEventDestroy(event);
+  }
+};
+
 struct ProfRecord {
   const char* name;
   uint64_t bytes;
@@ -100,6 +111,7 @@ struct pwmgpu_ctx {
   bool async_alloc = false;  // stream-ordered allocations on `stream`
   uint64_t scratch_bytes = 0;
   pwmgpu_wx* compute_cache = nullptr;  // reused by pwmgpu_compute for equal shapes
+  std::shared_ptr<CreationEvent> created = std::make_shared<CreationEvent>();  // see CreationEvent
   std::vector<std::unique_ptr<pwmgpu_wx>> shard_cache;  // reused by pwmgpu_wx_build_sharded
   std::unique_ptr<pwmgpu_wx> semi_shard[2];             // semi-external pieces: full-size and last
   // CUDA-event timing of every launch group while profiling is on
@@ -299,6 +311,7 @@ struct Structure {
 
 struct pwmgpu_wx {
   pwmgpu_ctx* ctx = nullptr;
+  std::shared_ptr<CreationEvent> created;  // the creating context's (pwmgpu_wx_create)
   uint64_t n = 0;
   uint32_t width = 1;     // key bytes of the build
   uint32_t in_width = 0;  // bytes of an input symbol when they differ (5: pwm's uint40_t, widened to 4)
@@ -340,6 +353,17 @@ pwmgpu_status guarded(pwmgpu_ctx* ctx, F&& f) {
   } catch (const std::exception& e) {  // nothing else may cross the C ABI
     return fail(ctx, PWMGPU_ERR_CUDA, std::string("host error: ") + e.what());
   }
+}
+
+// What pwmgpu_wx_create enqueued, before whatever `ctx` enqueues next: nothing
+// to do on the context that created the wx, whose stream has the order, nor on
+// a stream that is being captured, which cannot wait for work outside (a
+// captured query needs a structure built before).
+inline void after_creation(pwmgpu_ctx* ctx, const pwmgpu_wx* wx) {
+  if (!wx->created || wx->created == ctx->created) return;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  CUDA_TRY(cudaStreamIsCapturing(ctx->stream, &capture));
+  if (capture == cudaStreamCaptureStatusNone) CUDA_TRY(cudaStreamWaitEvent(ctx->stream, wx->created->event, 0));
 }
 
 inline bool valid_width(uint32_t w) { return w == 1 || w == 2 || w == 4; }
