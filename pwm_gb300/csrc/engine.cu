@@ -47,8 +47,9 @@ namespace pwmgpu {
 // have one of their own, first: past 1 MiB an allocation maps memory of its own
 // (both structures of 10^6 bytes created and freed: five allocations each 104 us,
 // one 271, two 65).
-// stream: the context's (its words are zeroed there, so that a build on it
-// comes after; one of another context waits for them, after_creation).
+// stream: the context's (its words are zeroed and its descriptors copied
+// there, so that a build on it comes after; one of another context waits for
+// them, after_creation).
 void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint64_t n, bool tree, bool huff,
                      bool rank_select, cudaStream_t stream, cudaStream_t alloc_stream) {
   s.release();
@@ -109,12 +110,10 @@ void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint
     std::memcpy(s.desc_host.data() + sizeof(RankSelectLevel) * l, &r, sizeof(r));
     std::memcpy(s.desc_host.data() + sizeof(RankSelectLevel) * s.levels + sizeof(QueryLevel) * l, &q, sizeof(q));
   }
-  if (s.levels) {
-    if (alloc_stream)
-      CUDA_TRY(cudaMemcpyAsync(s.d_rs_levels, s.desc_host.data(), s.desc_host.size(), cudaMemcpyHostToDevice,
-                               alloc_stream));
-    else CUDA_TRY(cudaMemcpy(s.d_rs_levels, s.desc_host.data(), s.desc_host.size(), cudaMemcpyHostToDevice));
-  }
+  // on `stream`: the kernels of a build read their pointers from here, and
+  // nothing orders the default stream before them
+  if (s.levels)
+    CUDA_TRY(cudaMemcpyAsync(s.d_rs_levels, s.desc_host.data(), s.desc_host.size(), cudaMemcpyHostToDevice, stream));
   s.rs = true;
 }
 

@@ -1,0 +1,65 @@
+"""GPU: what a context uploads goes up on its own stream, which alone orders it
+before the kernels that read it.
+
+The default stream is kept busy for a tenth of a second.  A copy issued there
+would wait for it, and so would the call; a call that uses its context's
+stream alone returns with the right answers while the default stream is still
+at it.
+"""
+from contextlib import nullcontext
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+BUSY_CYCLES = 200_000_000  # about 0.1 s at 2 GHz
+
+
+class DefaultStreamBusy:
+    """Work on the default stream that must outlast the block."""
+
+    def __enter__(self):
+        import torch
+        torch.cuda.synchronize()
+        torch.cuda._sleep(BUSY_CYCLES)
+        self.done = torch.cuda.Event()
+        self.done.record()
+        return self
+
+    def __exit__(self, kind, value, trace):
+        import torch
+        waited = self.done.query()
+        torch.cuda.synchronize()
+        if kind is None:
+            assert not waited, "a call waited for the default stream"
+
+
+def device_words(a):
+    import torch
+    return torch.from_numpy(np.asarray(a, np.uint64).view(np.int64)).cuda()
+
+
+@pytest.mark.parametrize("tree", [False, True])
+def test_level_descriptors(pg, tree):
+    """The rank/select kernels and the queries take their pointers from the
+    descriptors that pwmgpu_wx_create uploads."""
+    torch = pytest.importorskip("torch")
+    n, L, q = 70_001, 8, 500
+    rng = np.random.default_rng(5)
+    text = rng.integers(0, 256, n).astype(np.uint8)
+    ctx = pg.Context()
+    d = torch.from_numpy(text).cuda()
+    pos = rng.integers(0, n, q)
+    d_pos, d_out = device_words(pos), device_words(np.zeros(q))
+    kept = []
+    for first in (True, False):  # the first time loads the kernels and makes the context's scratch
+        with nullcontext() if first else DefaultStreamBusy():
+            ds = pg.DeviceStructure(n, 1, L, matrix=not tree, tree=tree, rank_select=True, context=ctx)
+            kept.append(ds)  # freeing one would wait for the device
+            ds.build(d.data_ptr())
+            ds.query(int(tree), pg.Q_ACCESS, d_pos.data_ptr(), None, q, d_out.data_ptr())
+            ctx.sync()
+    assert np.array_equal(d_out.cpu().numpy(), text[pos].astype(np.int64))
+    for ds in kept:
+        ds.free()
