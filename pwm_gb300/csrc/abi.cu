@@ -558,12 +558,12 @@ pwmgpu_status pwmgpu_wx_build_huffman(pwmgpu_ctx* ctx, const void* d_text, uint6
     // word), level sizes; made and copied while the passes run
     const uint64_t nsym = wx->code_len.size();
     std::vector<std::pair<uint64_t, uint64_t>> dec;
+    std::vector<uint64_t> blob;
     auto query_tables = [&]() {
       const Structure& S = tree ? wx->wt : wx->wm;
       for (uint64_t c = 0; c < nsym; ++c)
         if (wx->code_len[c]) dec.emplace_back((wx->code_len[c] << 56) | wx->code_word[c], c);
       std::sort(dec.begin(), dec.end());
-      std::vector<uint64_t> blob;
       blob.reserve(2 * nsym + 2 * dec.size() + S.levels);
       blob.insert(blob.end(), wx->code_len.begin(), wx->code_len.end());
       blob.insert(blob.end(), wx->code_word.begin(), wx->code_word.end());
@@ -571,7 +571,8 @@ pwmgpu_status pwmgpu_wx_build_huffman(pwmgpu_ctx* ctx, const void* d_text, uint6
       for (const auto& d : dec) blob.push_back(d.second);
       blob.insert(blob.end(), S.bits.begin(), S.bits.end());
       CUDA_TRY(cudaMalloc(&wx->d_huff, std::max<size_t>(blob.size(), 1) * 8));
-      CUDA_TRY(cudaMemcpy(wx->d_huff, blob.data(), blob.size() * 8, cudaMemcpyHostToDevice));
+      // on the context's stream, as the queries; build_huffman waits for it before it returns
+      CUDA_TRY(cudaMemcpyAsync(wx->d_huff, blob.data(), blob.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
     };
     build_huffman(ctx, d_text, size, word_width, tree, wx->code_len, wx->code_word, L, wx->wm,
                   tree ? &wx->wt : nullptr, rs, counts.device ? &counts : nullptr, query_tables);

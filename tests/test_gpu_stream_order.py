@@ -63,3 +63,27 @@ def test_level_descriptors(pg, tree):
     assert np.array_equal(d_out.cpu().numpy(), text[pos].astype(np.int64))
     for ds in kept:
         ds.free()
+
+
+@pytest.mark.parametrize("width", [1, 2])
+def test_huffman_query_tables(pg, width):
+    """The code tables that the queries of a Huffman-shaped structure read.  (A
+    matrix: the build of a tree frees its source, which waits for the device.)"""
+    torch = pytest.importorskip("torch")
+    n, q = 70_001, 500
+    rng = np.random.default_rng(6)
+    text = np.minimum(rng.geometric(0.02, n), 255 if width == 1 else 900).astype(np.uint8 if width == 1 else np.uint16)
+    ctx = pg.Context()
+    d = torch.from_numpy(text.view(np.uint8).copy()).cuda()
+    pos = rng.integers(0, n, q)
+    d_pos, d_out = device_words(pos), device_words(np.zeros(q))
+    kept = []
+    for first in (True, False):
+        with nullcontext() if first else DefaultStreamBusy():
+            ds = pg.DeviceStructure.huffman(d.data_ptr(), n, width, rank_select=True, context=ctx)
+            kept.append(ds)
+            ds.query(0, pg.Q_ACCESS, d_pos.data_ptr(), None, q, d_out.data_ptr())
+            ctx.sync()
+    assert np.array_equal(d_out.cpu().numpy(), text[pos].astype(np.int64))
+    for ds in kept:
+        ds.free()
