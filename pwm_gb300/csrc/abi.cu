@@ -42,7 +42,7 @@ pwmgpu_status pwmgpu_ctx_create(int device, void* cuda_stream, pwmgpu_ctx** out)
       ctx->own_stream = true;
     }
     CUDA_TRY(cudaMalloc(&ctx->d_status, kStatusBytes));
-    CUDA_TRY(cudaMemset(ctx->d_status, 0, kStatusBytes));
+    CUDA_TRY(cudaMemsetAsync(ctx->d_status, 0, kStatusBytes, ctx->stream));
     // a kernel of this library must be loadable on this device
     cudaFuncAttributes attr;
     cudaError_t e = cudaFuncGetAttributes(&attr, reinterpret_cast<const void*>(&pwmgpu_ctx_create));

@@ -118,6 +118,10 @@ struct pwmgpu_batch {
 
 namespace {
 
+// Everything a batch uploads goes up on its context's stream, on which its
+// kernels run: nothing orders the default stream before them.  (A copy from a
+// pageable host vector returns once the data is staged.)
+
 // Pass groups (pass index, K) and their per-text split arguments.
 void batch_plan(pwmgpu_batch* b, const void* d_texts) {
   pwmgpu_ctx* ctx = b->ctx;
@@ -189,9 +193,10 @@ void batch_plan(pwmgpu_batch* b, const void* d_texts) {
         a.L = b->L[t];
         pass_starts_base[t] += uint64_t((2 << K) - 2);
       }
-      CUDA_TRY(cudaMemcpy(g.d_args, args.data(), sizeof(SplitArgs) * args.size(), cudaMemcpyHostToDevice));
-      CUDA_TRY(cudaMemcpy(g.d_tile_base, tile_base.data(), sizeof(uint32_t) * tile_base.size(),
-                          cudaMemcpyHostToDevice));
+      CUDA_TRY(cudaMemcpyAsync(g.d_args, args.data(), sizeof(SplitArgs) * args.size(),
+                               cudaMemcpyHostToDevice, ctx->stream));
+      CUDA_TRY(cudaMemcpyAsync(g.d_tile_base, tile_base.data(), sizeof(uint32_t) * tile_base.size(),
+                               cudaMemcpyHostToDevice, ctx->stream));
       b->groups.push_back(std::move(g));
     }
   }
@@ -399,7 +404,7 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
       cnt_total += group_tile * (uint64_t(1) << D);
       blk_total += group_blk * (uint64_t(1) << D);
     }
-    CUDA_TRY(cudaMemcpy(d_tx, tx.data(), tx.size() * sizeof(TileText), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(d_tx, tx.data(), tx.size() * sizeof(TileText), cudaMemcpyHostToDevice, ctx->stream));
     const size_t lb_bytes = (uint64_t(1) << D) * tiles_ub * 8;
     void* lb = b->talloc(lb_bytes);
     b->lookback.push_back({lb, lb_bytes});
@@ -445,8 +450,8 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
                         [&](const BatchChunk& c) { return b->width != 1 || !c.D || b->L[c.text] > 4; });
   b->d_tchunks = static_cast<BatchChunk*>(b->talloc(std::max<size_t>(b->tchunks.size(), 1) * sizeof(BatchChunk)));
   if (!b->tchunks.empty())
-    CUDA_TRY(cudaMemcpy(b->d_tchunks, b->tchunks.data(), b->tchunks.size() * sizeof(BatchChunk),
-                        cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(b->d_tchunks, b->tchunks.data(), b->tchunks.size() * sizeof(BatchChunk),
+                             cudaMemcpyHostToDevice, ctx->stream));
   b->d_tilecnt = static_cast<uint32_t*>(b->talloc(std::max<uint64_t>(cnt_total, 1) * 4));
   b->d_relpre = static_cast<uint32_t*>(b->talloc(std::max<uint64_t>(cnt_total, 1) * 4));
   b->d_blocksum = static_cast<unsigned long long*>(b->talloc(std::max<uint64_t>(blk_total, 1) * 8));
@@ -462,12 +467,15 @@ void tile_plan(pwmgpu_batch* b, const void* d_texts) {
   b->d_pfx = static_cast<uint64_t*>(b->talloc(std::max<uint64_t>(pfx, 1) * 8));
   auto* d_args = static_cast<TileArgs*>(b->talloc(std::max<size_t>(args.size(), 1) * sizeof(TileArgs)));
   if (!texts.empty())
-    CUDA_TRY(cudaMemcpy(b->d_tb_texts, texts.data(), texts.size() * sizeof(TileBatchText), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(b->d_tb_texts, texts.data(), texts.size() * sizeof(TileBatchText),
+                             cudaMemcpyHostToDevice, ctx->stream));
   if (!passes.empty())
-    CUDA_TRY(cudaMemcpy(b->d_tb_passes, passes.data(), passes.size() * sizeof(TileBatchPass), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(b->d_tb_passes, passes.data(), passes.size() * sizeof(TileBatchPass),
+                             cudaMemcpyHostToDevice, ctx->stream));
   if (!groups.empty()) {
-    CUDA_TRY(cudaMemcpy(b->d_tb_groups, groups.data(), groups.size() * sizeof(TileBatchGroup), cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(d_args, args.data(), args.size() * sizeof(TileArgs), cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(b->d_tb_groups, groups.data(), groups.size() * sizeof(TileBatchGroup),
+                             cudaMemcpyHostToDevice, ctx->stream));
+    CUDA_TRY(cudaMemcpyAsync(d_args, args.data(), args.size() * sizeof(TileArgs), cudaMemcpyHostToDevice, ctx->stream));
   }
   q.args = d_args;
   q.group_tiles = b->d_group_tiles;
@@ -633,8 +641,8 @@ std::unique_ptr<pwmgpu_batch> make_batch(pwmgpu_ctx* ctx, uint32_t count, const 
       b->d_segs = static_cast<uint64_t*>(b->dalloc(b->segs_n * 8));
     } else {
       // the tile engine never writes padding words: zero once
-      CUDA_TRY(cudaMemset(b->d_wm, 0, std::max<uint64_t>(b->wm_words, 1) * 8));
-      if (b->d_wt) CUDA_TRY(cudaMemset(b->d_wt, 0, std::max<uint64_t>(b->wt_words, 1) * 8));
+      CUDA_TRY(cudaMemsetAsync(b->d_wm, 0, std::max<uint64_t>(b->wm_words, 1) * 8, ctx->stream));
+      if (b->d_wt) CUDA_TRY(cudaMemsetAsync(b->d_wt, 0, std::max<uint64_t>(b->wt_words, 1) * 8, ctx->stream));
     }
     b->d_hist = static_cast<unsigned long long*>(b->dalloc(b->hist_n * 8));
     b->d_keys_a = b->dalloc(b->symbols * word_width);
@@ -661,12 +669,15 @@ std::unique_ptr<pwmgpu_batch> make_batch(pwmgpu_ctx* ctx, uint32_t count, const 
       }
       b->d_regroup = static_cast<BatchRegroup*>(b->dalloc(sizeof(BatchRegroup) * std::max<size_t>(b->regroup.size(), 1)));
       if (!b->regroup.empty())
-        CUDA_TRY(cudaMemcpy(b->d_regroup, b->regroup.data(), sizeof(BatchRegroup) * b->regroup.size(),
-                            cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpyAsync(b->d_regroup, b->regroup.data(), sizeof(BatchRegroup) * b->regroup.size(),
+                                 cudaMemcpyHostToDevice, ctx->stream));
     }
-    if (count) CUDA_TRY(cudaMemcpy(b->d_info, b->info.data(), sizeof(BatchText) * count, cudaMemcpyHostToDevice));
+    if (count)
+      CUDA_TRY(cudaMemcpyAsync(b->d_info, b->info.data(), sizeof(BatchText) * count, cudaMemcpyHostToDevice,
+                               ctx->stream));
     if (!b->chunks.empty())
-      CUDA_TRY(cudaMemcpy(b->d_chunks, b->chunks.data(), sizeof(BatchChunk) * b->chunks.size(), cudaMemcpyHostToDevice));
+      CUDA_TRY(cudaMemcpyAsync(b->d_chunks, b->chunks.data(), sizeof(BatchChunk) * b->chunks.size(),
+                               cudaMemcpyHostToDevice, ctx->stream));
     return b;
 }
 

@@ -87,3 +87,32 @@ def test_huffman_query_tables(pg, width):
     assert np.array_equal(d_out.cpu().numpy(), text[pos].astype(np.int64))
     for ds in kept:
         ds.free()
+
+
+@pytest.mark.parametrize("engine", ["tile", "warp"])
+def test_batch_plan(pg, orc, engine):
+    """The text table, the passes' arguments and the zeroed words of a batch."""
+    torch = pytest.importorskip("torch")
+    lengths, levels = [1000, 40_003, 0, 70_001], [3, 8, 4, 5]
+    offsets = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint64)
+    rng = np.random.default_rng(7)
+    texts = [rng.integers(0, 1 << l, n).astype(np.uint8) for n, l in zip(lengths, levels)]
+    ctx = pg.Context()
+    ctx.set_engine(pg.ENGINE_TILE if engine == "tile" else pg.ENGINE_WARP)
+    d = torch.from_numpy(np.concatenate(texts)).cuda()
+    kept = []
+    for first in (True, False):
+        with nullcontext() if first else DefaultStreamBusy():
+            b = pg.Batch(offsets, levels, tree=True, context=ctx)
+            kept.append(b)
+            if engine == "tile":
+                b.set_tile_vectors(2)  # no tuning, whose batches are freed
+            b.build(d.data_ptr())
+            b.check()
+    for t, (text, l) in enumerate(zip(texts, levels)):
+        for which in (0, 1):
+            if text.size:
+                ref, ws = orc.build(text, l, which == 1, "ps"), kept[1].download(t, which)
+                assert all(np.array_equal(ws.bvs()[m], ref.level(m)) for m in range(l))
+    for b in kept:
+        b.free()
