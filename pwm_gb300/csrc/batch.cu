@@ -374,11 +374,8 @@ void launch_hist_w(const void* texts, const BatchChunk* chunks, uint32_t nchunks
                    unsigned long long* hist, uint32_t* tilecnt, uint32_t* relpre, unsigned long long* blocksum,
                    uint32_t* status, cudaStream_t s) {
   constexpr size_t smem = (sizeof(T) == 1 ? kHistColumns + 2 * (kBatchThreads / 32) * 8 : 4096 + kHistTileCounters) * 4;
-  static bool configured = false;  // attribute set once per width
-  if (!configured) {
-    cudaFuncSetAttribute(batch_hist_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    configured = true;
-  }
+  static OncePerDevice allowed;
+  if (allow_shared(allowed, reinterpret_cast<const void*>(batch_hist_kernel<T>), smem) != cudaSuccess) return;
   batch_hist_kernel<T><<<nchunks, kBatchThreads, smem, s>>>(static_cast<const T*>(texts), chunks, info, hist, tilecnt,
                                                             relpre, blocksum, status);
 }
@@ -398,11 +395,8 @@ void launch_batch_tables(const unsigned long long* hist, const BatchText* info, 
                          uint64_t* launches) {
   if (ntexts == 0) return;
   const size_t smem = (size_t(2) << max_levels) * 8;
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(batch_tables_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(8 << 13));
-    configured = true;
-  }
+  static OncePerDevice allowed;
+  if (allow_shared(allowed, reinterpret_cast<const void*>(batch_tables_kernel), 8 << 13) != cudaSuccess) return;
   batch_tables_kernel<<<ntexts, kBatchThreads, smem, s>>>(hist, info, kmax, zeros, starts, segs);
   ++*launches;
 }

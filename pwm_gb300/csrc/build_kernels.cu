@@ -580,11 +580,8 @@ void hist_dispatch(const T* text, uint64_t n, uint32_t levels, unsigned long lon
   else if (levels <= 13)
     leaf_hist_smem<T, 8192, false><<<grid, kHistThreads, 0, s>>>(text, n, levels, hist, status);
   else if (levels <= 16) {
-    static bool configured = false;
-    if (!configured) {
-      cudaFuncSetAttribute(leaf_hist_packed<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (1 << 15) * 4);
-      configured = true;
-    }
+    static OncePerDevice allowed;
+    if (allow_shared(allowed, reinterpret_cast<const void*>(leaf_hist_packed<T>), (1 << 15) * 4) != cudaSuccess) return;
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1332,12 +1329,10 @@ void launch_pass_digits(const void* text, uint64_t n, uint32_t width, const Pass
                         unsigned long long* digits, unsigned int* done, uint32_t* status, uint64_t* out,
                         cudaStream_t s, uint64_t* launches) {
   const size_t smem = size_t(pd.npasses) * 16 * 32 * 4;
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(pass_digits_kernel<kPassDigitsMaxPasses>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(kPassDigitsMaxPasses * 16 * 32 * 4));
-    configured = true;
-  }
+  static OncePerDevice allowed;
+  if (allow_shared(allowed, reinterpret_cast<const void*>(pass_digits_kernel<kPassDigitsMaxPasses>),
+                   kPassDigitsMaxPasses * 16 * 32 * 4) != cudaSuccess)
+    return;
   const uint64_t vecs = (n * width + 15) / 16;
   const uint64_t want = (vecs + 255) / 256;
   int sms = 0;

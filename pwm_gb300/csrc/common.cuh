@@ -4,6 +4,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "device_once.hpp"
+
 namespace pwmgpu {
 
 // Device status word bits (set by kernels, read by the host after a sync).
@@ -99,6 +101,19 @@ __host__ __device__ inline uint32_t word_select1(uint64_t v, uint32_t rank) {
   t = uint32_t((v >> (s - 1)) & 0x1);
   s -= ((t - r) & 256) >> 8;
   return 64 - s;
+}
+
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device
+// (more than 48 KB are allowed kernel by kernel, and on each device for
+// itself).  `once` belongs to the kernel.  An error is also the next
+// cudaGetLastError's.
+inline cudaError_t allow_shared(OncePerDevice& once, const void* kernel, size_t bytes) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return cudaError_t(once.run(device, [&]() {
+    return int(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+  }));
 }
 
 // Programmatic dependent launch: a kernel launched with launch_chained may be

@@ -22,12 +22,9 @@ void launch_one(const SplitArgs& a, uint32_t L, cudaStream_t s) {
   using Tr = typename std::conditional<HUFF, HuffKeys<Key>, PlainKeys<Key>>::type;
   using P = SplitPass<Key, Tr, K, kSplitThreads, G::ITEMS>;
   auto kern = split_pass_kernel<Key, Tr, K, kSplitThreads, G::ITEMS, KeyO>;
-  static bool configured = false;  // one attribute call per instantiation and process
+  static OncePerDevice allowed;
   const size_t smem = P::smem_bytes();
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    configured = true;
-  }
+  if (allow_shared(allowed, reinterpret_cast<const void*>(kern), smem) != cudaSuccess) return;
   Tr tr{L};
   kern<<<a.tiles, kSplitThreads, smem, s>>>(a, tr);
 }
@@ -40,12 +37,9 @@ void launch_batched_one(const SplitArgs* args, const uint32_t* tile_base, uint32
   using Tr = typename std::conditional<HUFF, HuffKeys<Key>, PlainKeys<Key>>::type;
   using P = SplitPass<Key, Tr, K, kSplitThreads, G::ITEMS>;
   auto kern = split_pass_batched_kernel<Key, Tr, K, kSplitThreads, G::ITEMS>;
-  static bool configured = false;
+  static OncePerDevice allowed;
   const size_t smem = P::smem_bytes();
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    configured = true;
-  }
+  if (allow_shared(allowed, reinterpret_cast<const void*>(kern), smem) != cudaSuccess) return;
   kern<<<tiles, kSplitThreads, smem, s>>>(args, tile_base, ntexts, counter);
 }
 

@@ -293,11 +293,8 @@ size_t batch_kernel_smem() {
   constexpr size_t keys = TileCfg<KeyT, 4, true, 256, 4>::smem_bytes();
   constexpr size_t planes = sizeof(KeyT) == 1 ? TileCfg<KeyT, 4, false, 256, 8>::plane_smem_bytes() : 0;
   constexpr size_t bytes = keys > planes ? keys : planes;
-  static bool configured = false;  // attribute set once per key width
-  if (!configured) {
-    cudaFuncSetAttribute(tile_batch_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-    configured = true;
-  }
+  static OncePerDevice allowed;  // (an error is reported with the launch)
+  allow_shared(allowed, reinterpret_cast<const void*>(tile_batch_kernel<KeyT>), bytes);
   return bytes;
 }
 

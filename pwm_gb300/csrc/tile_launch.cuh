@@ -15,11 +15,8 @@ void launch_tile_one(const TileArgs& a, cudaStream_t s) {
   using C = TileCfg<KeyT, K, OUT, kTileThreads, V>;
   auto kern = tile_pass_kernel<KeyT, K, OUT, kTileThreads, V, KeyO, PLANES>;
   constexpr size_t smem = PLANES ? C::plane_smem_bytes() : C::RANKABLE ? C::ranked_smem_bytes() : C::smem_bytes();
-  static bool configured = false;  // attribute set once per instantiation
-  if (!configured) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    configured = true;
-  }
+  static OncePerDevice allowed;
+  if (allow_shared(allowed, reinterpret_cast<const void*>(kern), smem) != cudaSuccess) return;
   kern<<<a.launch_tiles, kTileThreads, smem, s>>>(a);
 }
 
