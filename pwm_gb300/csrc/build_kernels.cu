@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kHistThreads) leaf_hist_global(const T* text, 
 // D symbol bits read with the first bit least significant.  Block b walks
 // tiles [b*tiles_per_block, ...) in order; per tile it writes the counts and
 // their prefix inside the block, at the end the block's totals.
-constexpr int kTileHistThreads = 256;
+constexpr int kTileHistThreads = kTileThreads;
 
 // BYTES8: 8-bit symbols and 8 levels, so that every byte is a bin: a key
 // costs a byte extract, an address and the atomic.
@@ -124,11 +124,11 @@ __global__ void __launch_bounds__(kTileHistThreads) tile_hist_kernel(const T* te
     atomicAdd(&mine[(c & binmask) * 32], 1u);  // an out-of-range symbol fails the build below
   };
   constexpr int PER = 16 / sizeof(T);
-  // whole aligned units (a tile, or half of a double one) of HV 16-byte
+  // whole aligned units (a tile, or a part of a wider one) of HV 16-byte
   // vectors per thread, loaded one unit ahead so that the loads overlap the
   // counting of the previous one
-  constexpr int HV = 4;
-  const uint32_t tile_units = tile_keys * sizeof(T) > 16 * HV * kTileHistThreads ? 2 : 1;
+  constexpr int HV = kTileVectors;
+  const uint32_t tile_units = tile_hist_units(tile_keys * sizeof(T));
   const uint32_t unit_keys = tile_keys / tile_units, units = tiles_per_block * tile_units;
   const uint32_t unit_vecs = uint32_t(unit_keys * sizeof(T) / 16);
   const bool vec = unit_keys * sizeof(T) % (16 * kTileHistThreads) == 0 && unit_vecs <= HV * kTileHistThreads &&

@@ -6,9 +6,6 @@
 
 namespace pwmgpu {
 
-constexpr int kTileThreads = 256;
-constexpr int kTileVectors = 4;  // 16-byte vectors per thread: 64 bytes of keys
-
 // PLANES: the bit-plane form of a pass without S_{l+K} over 1-byte keys.
 template <typename KeyT, int K, bool OUT, typename KeyO = KeyT, bool PLANES = false, int V = kTileVectors>
 void launch_tile_one(const TileArgs& a, cudaStream_t s) {

@@ -2,6 +2,8 @@
 // shared by the kernels and the host planner (compiles with or without CUDA).
 #pragma once
 
+#include <cstdint>
+
 #if defined(__CUDACC__)
 #define PWMGPU_HOST_DEVICE __host__ __device__
 #else
@@ -15,6 +17,18 @@ constexpr int kTileMaxLevels = 4;
 // texts of at most 8 levels) neither counts nor looks back, and may split up
 // to 7 times: all levels of such a text in one pass.
 constexpr int kTileGivenMaxLevels = 8;
+
+constexpr int kTileThreads = 256;
+constexpr int kTileVectors = 4;  // 16-byte vectors per thread: 64 bytes of keys
+
+// The histogram kernel reads a tile in equal units of at most kTileVectors
+// vectors a thread, each loaded while the one before is counted: one for the
+// usual tiles and smaller ones, 2 or 4 for those of 8 or 16 vectors.
+PWMGPU_HOST_DEVICE constexpr uint32_t tile_hist_units(uint64_t tile_bytes) {
+  return tile_bytes <= uint64_t(16 * kTileVectors) * kTileThreads
+             ? 1u
+             : uint32_t(tile_bytes / (uint64_t(16 * kTileVectors) * kTileThreads));
+}
 
 // Table entries of one segment: matrix starts (level j, run v) at
 // (1 << j) - 1 + v, tree starts after them, then the S_out starts (2^K).

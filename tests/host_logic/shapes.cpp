@@ -1,0 +1,28 @@
+// The tiles' geometry (pwm_gb300/csrc/tile_layout.hpp): prints "ok", or what
+// does not fit.
+#include <cstdio>
+#include <initializer_list>
+
+#include "../../pwm_gb300/csrc/tile_layout.hpp"
+
+using namespace pwmgpu;
+
+// Every tile is whole units of whole vectors a thread, as many as the
+// histogram kernel holds.
+static int units() {
+  for (int vectors : {1, 2, 4, 8, 16}) {
+    const uint64_t bytes = uint64_t(vectors) * 16 * kTileThreads;
+    const uint32_t u = tile_hist_units(bytes);
+    if (u == 0 || bytes % u || bytes / u % (16 * kTileThreads) || bytes / u > uint64_t(16 * kTileVectors) * kTileThreads) {
+      printf("tiles of %d vectors: %u units\n", vectors, u);
+      return 1;
+    }
+  }
+  return 0;
+}
+
+int main() {
+  if (units()) return 1;
+  printf("ok\n");
+  return 0;
+}
