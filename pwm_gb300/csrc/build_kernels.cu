@@ -1176,11 +1176,9 @@ int grid_for(uint64_t n, int threads) {
 
 }  // namespace
 
-uint32_t tile_hist_tiles_per_block() { return 16; }
-
-uint32_t tile_hist_blocks(uint64_t n, uint32_t tile_keys) {
-  const uint64_t tiles = (n + tile_keys - 1) / tile_keys;
-  return uint32_t((tiles + tile_hist_tiles_per_block() - 1) / tile_hist_tiles_per_block());
+uint32_t tile_hist_blocks(uint64_t n, uint32_t tile_keys, uint32_t width) {
+  const uint64_t tiles = (n + tile_keys - 1) / tile_keys, per = tile_hist_tiles_per_block(uint64_t(tile_keys) * width);
+  return uint32_t((tiles + per - 1) / per);
 }
 
 void launch_tile_histogram_blocks(const void* text, uint64_t n, uint32_t width, uint32_t levels, uint32_t D,

@@ -18,14 +18,13 @@ void launch_leaf_histogram(const void* text, uint64_t n, uint32_t width, uint32_
 // Leaf histogram of a text with levels <= 8 that also counts, per tile of
 // tile_keys symbols (a multiple of 64), the 2^D runs of the first D symbol
 // bits (first bit least significant): tilecnt[tile][run], relpre[tile][run]
-// (prefix inside a block of tile_hist_tiles_per_block() tiles) and
+// (prefix inside a block of `per` tiles) and
 // blocksum[block][run].  Blocks [block0, block0 + nblk) of the
-// tile_hist_blocks(n, tile_keys) blocks run, so a text can be counted piece
+// tile_hist_blocks(n, tile_keys, width) blocks run, so a text can be counted piece
 // by piece as it arrives; when level0_a is set, they also write level 0
 // (the symbols' top bits in text order) to level0_a and level0_b (if set).
 // hist must be zeroed.  launch_tile_block_scan then turns blocksum into each
 // block's exclusive prefix.
-uint32_t tile_hist_tiles_per_block();
 // 40-bit symbols (5 little-endian bytes each) widened to 32 bits (values of
 // 2^32 and more become 0xFFFFFFFF).
 void launch_widen40(const void* in, uint64_t n, uint32_t* out, cudaStream_t s, uint64_t* launches);
@@ -73,8 +72,8 @@ void launch_first_positions(const void* text, uint64_t n, uint32_t width, uint64
 // out[i] = map[text[i]] (same width; in place allowed).
 void launch_remap(const void* text, uint64_t n, uint32_t width, const uint32_t* map, uint64_t nmap, void* out,
                   uint32_t* status, cudaStream_t s, uint64_t* launches);
-uint32_t tile_hist_blocks(uint64_t n, uint32_t tile_keys);
-// per: the tiles of a block (tile_hist_tiles_per_block(), or fewer).
+uint32_t tile_hist_blocks(uint64_t n, uint32_t tile_keys, uint32_t width);
+// per: the tiles of a block (tile_hist_tiles_per_block, or fewer).
 void launch_tile_histogram_blocks(const void* text, uint64_t n, uint32_t width, uint32_t levels, uint32_t D,
                                   uint32_t tile_keys, uint32_t per, uint32_t block0, uint32_t nblk,
                                   unsigned long long* hist,

@@ -274,7 +274,7 @@ void build_one_pass(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text) {
   // tiles of a histogram block: one while there are few; then, counted by planes (nothing to set up or sum at a
   // block's end), blocks for every SM several times over, else longer ones
   const uint32_t per =
-      tiles <= 2 * 152 ? 1u : std::min(tile_hist_tiles_per_block(), std::max(1u, tiles / (w == 1 && L <= 4 ? 152 * 6 : 152)));
+      tiles <= 2 * 152 ? 1u : std::min(kTileHistMaxTiles, std::max(1u, tiles / (w == 1 && L <= 4 ? 152 * 6 : 152)));
   const uint32_t nblocks = (tiles + per - 1) / per, D = L - 1;
   const uint64_t NB = uint64_t(1) << D;
   // zeroed with the status word: the histogram, the pass's tile counter and,
@@ -484,8 +484,8 @@ void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostI
   if (tile_hist) {
     const uint32_t T = tile_pass_elems(wx->width, pass_vectors(wx->width, L, kmax, 0, n));
     const uint64_t tiles = (n + T - 1) / T;
-    const uint32_t per = tile_hist_tiles_per_block();
-    const uint32_t nblocks = tile_hist_blocks(n, T);
+    const uint32_t per = tile_hist_tiles_per_block(uint64_t(T) * wx->width);
+    const uint32_t nblocks = tile_hist_blocks(n, T, wx->width);
     const uint64_t NB = uint64_t(1) << D0;
     auto* base = static_cast<unsigned char*>(ctx->grow("tile_first", tiles * NB * 8 + nblocks * NB * 8 + 256));
     first.tilecnt = reinterpret_cast<uint32_t*>(base);
@@ -601,11 +601,11 @@ void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostI
     const TileBlob b0 = tile_blob(early, 0, 1, L, n, wx->wm, want_tree ? &wx->wt : nullptr);
     auto* d_b0 = static_cast<unsigned char*>(ctx->grow("tile_plan0", b0.bytes.size()));
     CUDA_TRY(cudaMemcpyAsync(d_b0, b0.bytes.data(), b0.bytes.size(), cudaMemcpyHostToDevice, s));
-    launch_tile_block_scan(const_cast<unsigned long long*>(first.blockpre), tile_hist_blocks(n, T), D0, d_hist, L,
+    launch_tile_block_scan(const_cast<unsigned long long*>(first.blockpre), tile_hist_blocks(n, T, wx->width), D0, d_hist, L,
                            uint32_t(p0.K), p0.out, want_tree, reinterpret_cast<uint64_t*>(d_b0 + b0.table[0]), s,
                            &ctx->launches);
     std::vector<uint32_t> bounds0;
-    const uint32_t nblk = tile_hist_blocks(n, T);
+    const uint32_t nblk = tile_hist_blocks(n, T, wx->width);
     const uint32_t C = ctx->stream_chunks;
     if (stream_out && C > 1 && nblk >= 2 * C) {
       // chunk c of C takes a share c + 1 of C (C + 1) / 2: the first is small,

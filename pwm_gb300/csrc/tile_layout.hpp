@@ -30,6 +30,14 @@ PWMGPU_HOST_DEVICE constexpr uint32_t tile_hist_units(uint64_t tile_bytes) {
              : uint32_t(tile_bytes / (uint64_t(16 * kTileVectors) * kTileThreads));
 }
 
+// Tiles of a histogram block: at most 16 (one-pass builds choose); else 16 of
+// the usual size, and as many bytes of wider ones, so that a text keeps its
+// number of blocks.
+constexpr uint32_t kTileHistMaxTiles = 16;
+PWMGPU_HOST_DEVICE constexpr uint32_t tile_hist_tiles_per_block(uint64_t tile_bytes) {
+  return kTileHistMaxTiles / tile_hist_units(tile_bytes);
+}
+
 // Table entries of one segment: matrix starts (level j, run v) at
 // (1 << j) - 1 + v, tree starts after them, then the S_out starts (2^K).
 PWMGPU_HOST_DEVICE constexpr int tile_table_size(int K) { return 2 * ((1 << K) - 1) + (1 << K); }

@@ -21,8 +21,22 @@ static int units() {
   return 0;
 }
 
+// A histogram block holds no more of a text in wide tiles than in the usual
+// ones: the same number of blocks works on it.
+static int blocks() {
+  const uint64_t usual = uint64_t(kTileVectors) * 16 * kTileThreads;
+  for (int vectors : {4, 8, 16}) {
+    const uint64_t bytes = uint64_t(vectors) * 16 * kTileThreads;
+    if (tile_hist_tiles_per_block(bytes) * bytes != tile_hist_tiles_per_block(usual) * usual) {
+      printf("blocks of tiles of %d vectors: %u\n", vectors, tile_hist_tiles_per_block(bytes));
+      return 1;
+    }
+  }
+  return 0;
+}
+
 int main() {
-  if (units()) return 1;
+  if (units() || blocks()) return 1;
   printf("ok\n");
   return 0;
 }
