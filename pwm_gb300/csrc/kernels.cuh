@@ -152,10 +152,6 @@ void launch_split_pass_batched(uint32_t key_bytes, int K, const SplitArgs* args,
                                uint64_t* launches);
 
 // ---- segmented tile passes (plain keys, matrix and tree together) ------------
-// Keys of one tile for a key width and the vectors a thread of
-// TileArgs::tile_vectors (0: the usual).
-uint32_t tile_pass_elems(uint32_t key_bytes, uint32_t vectors = 0);
-// One pass of K levels over a.tiles tiles; `out`: the pass writes S_{l+K}.
 // Digit counts of the passes of a matrix-only build (pass_digits_kernel):
 // pass p covers levels level[p]..level[p]+K[p]-1, its natural digit is
 // (symbol >> lo[p]) & mask[p].
@@ -181,11 +177,11 @@ void launch_pass_digits(const void* text, uint64_t n, uint32_t width, const Pass
 bool launch_flat_digits(const uint64_t* flat, uint32_t L, const uint32_t* level, const uint32_t* K, uint32_t count,
                         unsigned long long* digits, cudaStream_t s, uint64_t* launches);
 
-// The narrowest key width (1, 2 or 4 bytes) holding `bits` bits.
-uint32_t tile_key_bytes(uint32_t bits);
-// One tile pass over keys of key_bytes; a pass writing S_{l+K} (out) writes
-// it in keys of out_bytes <= key_bytes, their low bits.
-void launch_tile_pass(uint32_t key_bytes, uint32_t out_bytes, int K, bool out, const TileArgs& a, cudaStream_t s,
+// One tile pass of K levels over a.tiles tiles of keys of key_bytes; a pass
+// writing S_{l+K} (out) writes it in keys of out_bytes <= key_bytes, their low
+// bits.  False, and nothing launched, for a shape without a kernel
+// (tile_pass_has_kernel).
+bool launch_tile_pass(uint32_t key_bytes, uint32_t out_bytes, int K, bool out, const TileArgs& a, cudaStream_t s,
                       uint64_t* launches);
 
 // ---- wavelet tree from the matrix --------------------------------------------

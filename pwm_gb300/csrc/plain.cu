@@ -21,35 +21,8 @@ struct TileFirstPass {
   bool level0_written = false;  // the histogram kernel wrote level 0 of both structures
 };
 
-// Key width of S_l for the pass starting at level l of an L-level text of
-// `width`-byte symbols: the text itself at l = 0; later the narrowest width
-// that holds the L - l bits the remaining levels split on (a pass writes
-// only the low bits of its keys), never wider than the text.
-uint32_t tile_pass_key_bytes(uint32_t width, uint32_t L, uint32_t l) {
-  return l == 0 ? width : std::min(width, tile_key_bytes(L - l));
-}
-
-// 16-byte vectors a thread of the tiles of the pass from level l (0: the
-// usual).  Passes that write the next sequence: over 1-byte keys double tiles
-// from 1024 on (3 CTAs an SM: 456 at once; a tree's segments each end in a part
-// of one: 2^24 symbols of 16 levels, whose third pass has 256, 393 us so, 428
-// with them from 512).  Over 2-byte keys from 128 on (2^22 symbols of 16 levels,
-// matrix, 141 us without, 131 with; 2^23 200 and 182; 2^20 106 either way).
-// Over 4-byte keys always, the usual tiles being too small to sort by 4 bits at
-// once (20 levels, 2^14 symbols 113 and 110 us, 2^20 133 and 127), and quadruple
-// ones from 128 on (2^22 symbols 169 and 160 us, 2^25 617 and 597).  Last passes
-// over 1-byte keys from 512 double tiles (5 an SM): at 4 levels in one pass 51 us
-// either way at 2^24 symbols, 75 against 85 at 2^25.
-uint32_t pass_vectors(uint32_t width, uint32_t L, int kmax, uint32_t l, uint64_t n) {
-  const uint32_t K = std::min<uint32_t>(uint32_t(kmax), L - l), kb = tile_pass_key_bytes(width, L, l);
-  auto fills = [&](uint32_t vectors, uint64_t tiles) { return n >= tiles * tile_pass_elems(kb, vectors); };
-  if (l + K < L) {
-    if (K != uint32_t(kTileMaxLevels)) return 0u;
-    if (kb == 4) return fills(16, 128) ? 16u : 8u;
-    return fills(8, kb == 2 ? 128 : 1024) ? 8u : 0u;
-  }
-  return kb == 1 && K <= uint32_t(kTileMaxLevels) && fills(8, 512) ? 8u : 0u;
-}
+// A shape the planner must not ask for (tile_pass_has_kernel).
+Fail no_pass_kernel() { return Fail{PWMGPU_ERR_CUDA, "internal: no kernel for a tile pass of this shape"}; }
 
 // Device descriptors of passes [from, to): per pass its segments, its level
 // descriptor and its start tables, at offsets of one uploaded blob.
@@ -165,7 +138,7 @@ const void* enqueue_tile_pass(pwmgpu_ctx* ctx, const std::vector<TilePassHost>& 
     a.launch_tiles = b[c + 1] - b[c];
     {
       ProfScope ps(ctx, "split_pass", p.tiles ? bytes * a.launch_tiles / p.tiles : 0);
-      launch_tile_pass(in_bytes, out_bytes, p.K, p.out, a, s, &ctx->launches);
+      if (!launch_tile_pass(in_bytes, out_bytes, p.K, p.out, a, s, &ctx->launches)) throw no_pass_kernel();
     }
     CUDA_TRY(cudaGetLastError());
     if (after_chunk) after_chunk(c);
@@ -339,7 +312,7 @@ void build_one_pass(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text) {
   const uint64_t structs = one.text.wt ? 2 : 1;
   {
     ProfScope ps(ctx, "split_pass", structs * (L * (n * w + words_for(n) * 8) - words_for(n) * 8));
-    launch_tile_pass(w, w, int(L), false, a, s, &ctx->launches);
+    if (!launch_tile_pass(w, w, int(L), false, a, s, &ctx->launches)) throw no_pass_kernel();
   }
   build_rank_select(ctx, rs_wm, rs_wt, true, 0, ~0u, nullptr, "",
                     rs_fits ? reinterpret_cast<unsigned long long*>(words + kState) : nullptr);

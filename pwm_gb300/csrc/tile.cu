@@ -35,30 +35,17 @@ void launch_key(int K, bool out, uint32_t out_bytes, const TileArgs& a, cudaStre
 
 }  // namespace
 
-uint32_t tile_pass_elems(uint32_t key_bytes, uint32_t vectors) {
-  return uint32_t(kTileThreads) * (vectors ? vectors : uint32_t(kTileVectors)) * (16 / key_bytes);
-}
-
-uint32_t tile_key_bytes(uint32_t bits) { return bits <= 8 ? 1u : (bits <= 16 ? 2u : 4u); }
-
-void launch_tile_pass(uint32_t key_bytes, uint32_t out_bytes, int K, bool out, const TileArgs& a, cudaStream_t s,
+bool launch_tile_pass(uint32_t key_bytes, uint32_t out_bytes, int K, bool out, const TileArgs& a, cudaStream_t s,
                       uint64_t* launches) {
-  if (a.launch_tiles == 0) return;
-  const bool deep = K > kTileMaxLevels;
-  // beyond 4 levels: only as the last pass of a text whose prefixes the histogram gives
-  if (deep && (out || !a.blockpre || K > kTileGivenMaxLevels)) return;
-  if (out && a.tile_vectors) {
-    if (K != kTileMaxLevels || (a.tile_vectors != 2 * uint32_t(kTileVectors) &&
-                                (key_bytes != 4 || a.tile_vectors != 4 * uint32_t(kTileVectors))))
-      return;
-    launch_tile_pass_wide(key_bytes, out_bytes, a, s);
-  } else if (deep || a.tile_vectors) {
-    if (a.tile_vectors && key_bytes != 1) return;
-    launch_tile_pass_deep(key_bytes, K, a, s);
-  } else if (key_bytes == 1) launch_key<uint8_t>(K, out, out_bytes, a, s);
+  if (a.launch_tiles == 0) return true;
+  if (!tile_pass_has_kernel(key_bytes, out_bytes, K, out, a.tile_vectors, a.blockpre != nullptr)) return false;
+  if (out && a.tile_vectors) launch_tile_pass_wide(key_bytes, out_bytes, a, s);
+  else if (K > kTileMaxLevels || a.tile_vectors) launch_tile_pass_deep(key_bytes, K, a, s);
+  else if (key_bytes == 1) launch_key<uint8_t>(K, out, out_bytes, a, s);
   else if (key_bytes == 2) launch_key<uint16_t>(K, out, out_bytes, a, s);
   else launch_key<uint32_t>(K, out, out_bytes, a, s);
   ++*launches;
+  return true;
 }
 
 }  // namespace pwmgpu

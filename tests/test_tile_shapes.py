@@ -1,5 +1,6 @@
-"""CPU: the shapes of the tile passes (pwm_gb300/csrc/tile_layout.hpp, checked
-by tests/host_logic/shapes.cpp).  GPU: texts of 4-byte symbols whose first pass
+"""CPU: the shapes of the tile passes (pwm_gb300/csrc/tile_layout.hpp and
+host_tables.hpp, checked by tests/host_logic/shapes.cpp): every pass of a plan
+has a kernel, and a launch without one is refused.  GPU: texts of 4-byte symbols whose first pass
 takes the widest tiles and its prefixes from the histogram kernel, against the
 oracle (pwm's wx_ps, include/wx_ps.hpp:37-56)."""
 import os
