@@ -20,18 +20,18 @@ void launch_deep_key(int K, const TileArgs& a, cudaStream_t s) {
 }
 
 // Tiles of V vectors a thread: half-size ones for short texts, which fill
-// twice as many SMs; double ones for long texts (tile_wide.cu says why).
+// twice as many SMs (2 to 8 levels); double ones for long texts (1 to 7;
+// tile_wide.cu says why, and 8 levels are no faster in them).
 template <int V>
 void launch_sized(int K, const TileArgs& a, cudaStream_t s) {
   switch (K) {
-    case 1: launch_tile_one<uint8_t, 1, false, uint8_t, true, V>(a, s); return;
-    case 2: launch_tile_one<uint8_t, 2, false, uint8_t, true, V>(a, s); return;
-    case 3: launch_tile_one<uint8_t, 3, false, uint8_t, true, V>(a, s); return;
-    case 4: launch_tile_one<uint8_t, 4, false, uint8_t, true, V>(a, s); return;
+    case 2: launch_tile_one<uint8_t, 2, false, uint8_t, true, V>(a, s); break;
+    case 3: launch_tile_one<uint8_t, 3, false, uint8_t, true, V>(a, s); break;
+    case 4: launch_tile_one<uint8_t, 4, false, uint8_t, true, V>(a, s); break;
     case 5: launch_tile_one<uint8_t, 5, false, uint8_t, true, V>(a, s); break;
     case 6: launch_tile_one<uint8_t, 6, false, uint8_t, true, V>(a, s); break;
     case 7: launch_tile_one<uint8_t, 7, false, uint8_t, true, V>(a, s); break;
-    default: launch_tile_one<uint8_t, 8, false, uint8_t, true, V>(a, s); break;
+    default: launch_tile_one<uint8_t, V < kTileVectors ? 8 : 1, false, uint8_t, true, V>(a, s); break;
   }
 }
 

@@ -19,7 +19,7 @@ void launch_tile_one(const TileArgs& a, cudaStream_t s) {
 
 // Last passes of 5..8 levels with given prefixes (tile_deep.cu); with
 // TileArgs::tile_vectors, last passes over 1-byte keys (half: 2..8 levels,
-// double: 1..8).
+// double: 1..7).
 void launch_tile_pass_deep(uint32_t key_bytes, int K, const TileArgs& a, cudaStream_t s);
 // Passes of kTileMaxLevels levels that write S_{l+K}, double tiles
 // (tile_wide.cu).

@@ -46,7 +46,9 @@ PWMGPU_HOST_DEVICE constexpr bool tile_pass_has_kernel(uint32_t key_bytes, uint3
   // beyond 4 levels: only as the last pass of a text whose prefixes the histogram gives
   if (deep && (!given || K > kTileGivenMaxLevels)) return false;
   if (vectors == 0) return true;
-  return key_bytes == 1 && (vectors == kTileVectors / 2 || vectors == 2 * kTileVectors);
+  // half-size tiles: whole texts of 2 to 8 levels; double ones: those of up to 7, and last passes
+  if (key_bytes != 1) return false;
+  return vectors == kTileVectors / 2 ? K >= 2 : vectors == 2 * kTileVectors && K < kTileGivenMaxLevels;
 }
 
 // The histogram kernel reads a tile in equal units of at most kTileVectors

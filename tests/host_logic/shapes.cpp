@@ -76,6 +76,7 @@ static int refused() {
       {1, 1, 5, false, 0, false},  // 5 levels and more with a look-back
       {1, 1, 5, true, 0, true},   {1, 1, 9, false, 0, true},  {1, 1, 0, false, 0, false}, {3, 1, 4, false, 0, false},
       {8, 1, 4, false, 0, false}, {4, 3, 4, true, 8, false},
+      {1, 1, 1, false, 2, false}, {1, 1, 8, false, 8, true},
   };
   for (const Shape& s : none)
     if (tile_pass_has_kernel(s.kb, s.ob, s.K, s.out, s.vectors, s.given)) {
