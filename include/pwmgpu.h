@@ -132,8 +132,8 @@ PWMGPU_API pwmgpu_status pwmgpu_ctx_set_host_copy_threads(pwmgpu_ctx* ctx, int t
  * chunks run; 1 launches each pass whole and streams level groups per pass. */
 PWMGPU_API pwmgpu_status pwmgpu_ctx_set_stream_chunks(pwmgpu_ctx* ctx, uint32_t chunks);
 
-/* Bound on the polls of one decoupled look-back wait of the tile engine
- * (each poll sleeps about 64 ns; 0 restores the default of 2^24, about a
+/* Bound on the polls of one decoupled look-back wait of the tile engine and
+ * of rank/select builds (each poll sleeps about 64 ns; 0 restores the default of 2^24, about a
  * second).  A wait that runs out records a timeout in the context's status
  * word and the kernel carries on with a zero prefix, so it always returns;
  * the call that reads the status (pwmgpu_wx_check, the host-to-host calls)
@@ -143,7 +143,8 @@ PWMGPU_API pwmgpu_status pwmgpu_ctx_set_spin_limit(pwmgpu_ctx* ctx, uint32_t pol
 /* Failure injection for tests, on the host side: while enabled, every
  * look-back pass of a device-text plain build is launched without its first
  * tile, so that tile never publishes its counts and the tiles of its segment
- * wait until the spin limit.  The build then reports PWMGPU_ERR_TIMEOUT (its
+ * wait until the spin limit; a rank/select build likewise leaves out the first
+ * 2^20 bits of longer levels.  The build then reports PWMGPU_ERR_TIMEOUT (its
  * output is undefined, every write stays in bounds).  Off by default. */
 PWMGPU_API pwmgpu_status pwmgpu_ctx_test_withhold_tile(pwmgpu_ctx* ctx, int enable);
 
@@ -456,6 +457,9 @@ PWMGPU_API pwmgpu_status pwmgpu_generate_batch(uint64_t seed, uint32_t count, ui
  *   d_l12      2 * (nwords/32 + 1) u32 (for nwords == 0 one zeroed entry)
  *   d_select0, d_select1   nwords*64/8192 + 2 u32 each
  *   d_counts   3 u64: select0 samples, select1 samples, total ones (cleared here)
+ * The kernel's blocks of the level wait for one another, each wait bounded
+ * (about a second); where one gives up the total of ones is UINT64_MAX, and
+ * the other outputs are not to be used.
  * Work is enqueued on `cuda_stream` (NULL: the default stream) of the current
  * device.  The first call on a device looks up the scratch array's device
  * address and keeps it for the life of the process; make that first call

@@ -150,7 +150,8 @@ void build_rank_select(pwmgpu_ctx* ctx, Structure* wm, Structure* wt, bool share
   a.stride = rank_select_state_words(max_words);
   const uint64_t state_bytes = a.stride * (a.nfirst + a.nsecond) * 8;
   a.status = ctx->d_status;
-  a.spin_limit = kSpinLimit;
+  a.spin_limit = ctx->spin_limit;
+  a.withhold = ctx->withhold_first_tile ? 1u : 0u;
   a.state = zeroed_state;
   if (!a.state) {
     a.state = static_cast<unsigned long long*>(ctx->grow("rs_state" + std::string(tag), state_bytes));

@@ -97,11 +97,11 @@ struct pwmgpu_ctx {
   int engine = PWMGPU_ENGINE_TILE;
   uint64_t upload_piece = uint64_t(64) << 20;  // bytes of text per uploaded piece
   uint32_t stream_chunks = 4;                   // chunks of a pass whose words stream to pinned outputs
-  uint32_t spin_limit = kSpinLimit;             // polls of one look-back wait of the tile engine
+  uint32_t spin_limit = kSpinLimit;             // polls of one look-back wait of the tile passes and of rank/select
   // batched tile engine: vectors per thread of the tiles of each (key width,
   // levels, log2 length) class, measured on first use
   std::map<uint32_t, uint32_t> batch_tune;
-  bool withhold_first_tile = false;             // test hook: look-back passes skip their first tile
+  bool withhold_first_tile = false;             // test hook: look-backs lack their first tile or CTA
   // pageable host buffers move through pinned staging pieces filled and
   // drained by host threads (-1: automatic count, 0: the driver copies them)
   int host_copy_threads = -1;

@@ -247,6 +247,7 @@ struct RankSelectArgs {
   uint32_t first_lo, nfirst, second_lo, nsecond;
   uint32_t twin;
   uint32_t spin_limit;
+  uint32_t withhold;  // test hook: levels of several CTAs without their first
   uint64_t stride;
   unsigned long long* state;
   uint32_t* status;

@@ -101,7 +101,9 @@ __device__ __forceinline__ bool thread_block_select(const uint64_t* data, uint64
 // bits 261 -> 254 us, 171 of them the reading and counting, the rest waits on
 // predecessors and samples.)  CTAs take their place in
 // the level by ticket, so a CTA waits only for CTAs that already run; the wait
-// is bounded (kErrTimeout, a zero prefix).  Consecutive CTAs belong to
+// is bounded: a CTA that gives up records kErrTimeout, goes on with a zero
+// prefix and marks its own (kLost), as do all that build on it, and the last
+// one writes all ones for the level's number of ones.  Consecutive CTAs belong to
 // different levels: with the resident CTAs all in one level, prefixes reached
 // them too slowly (8 levels of 2^30 bits 388 against 273 us, both with 256
 // threads; 512 threads 254).  Looking back over 64 to 256 CTAs a step changed
@@ -111,6 +113,7 @@ __device__ __forceinline__ bool thread_block_select(const uint64_t* data, uint64
 // step i, lanes 0-15 read block 2i and lanes 16-31 block 2i+1, four lanes per
 // 512-bit L2 block; the counts are then gathered so that lane b holds block
 // b's.
+constexpr uint64_t kLost = 1ull << 61;  // of a state word: the counts before it are incomplete
 __global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSelectArgs a) {
   chain_next();
   chain_wait();
@@ -126,10 +129,11 @@ __global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSe
   }
   const uint64_t nreal = (L.nwords + kL1Cover - 1) / kL1Cover, n12 = L.nwords / kL1Cover + 1;
   const uint64_t ctas = nreal ? (nreal + kRsThreads - 1) / kRsThreads : 1;
-  if (blockIdx.y >= ctas) return;
+  const uint32_t withheld = a.withhold && ctas > 1 ? 1 : 0;  // the level's first CTA does not run
+  if (blockIdx.y + withheld >= ctas) return;
   unsigned long long* state = a.state + uint64_t(y) * a.stride;  // a ticket, then a word a CTA
   __shared__ uint32_t s_cta;
-  if (threadIdx.x == 0) s_cta = uint32_t(atomicAdd(state, 1ull));
+  if (threadIdx.x == 0) s_cta = uint32_t(atomicAdd(state, 1ull)) + withheld;
   __syncthreads();
   const uint32_t cta = s_cta;
   const uint64_t first = uint64_t(cta) * kRsThreads;
@@ -177,6 +181,7 @@ __global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSe
   }
   __shared__ uint32_t wsum[kRsThreads / 32];
   __shared__ unsigned long long s_before;
+  __shared__ bool s_lost;
   if (lane == 31) wsum[warp] = x;
   __syncthreads();
   uint32_t before_warp = 0, total = 0;
@@ -188,6 +193,7 @@ __global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSe
   // publish, then look back 32 CTAs a step
   if (warp == 0) {
     unsigned long long before = 0;
+    bool lost = false;
     if (lane == 0) st_volatile(state + 1 + cta, (cta == 0 ? kFlagPrefix : kFlagAggregate) | total);
     for (int64_t at = int64_t(cta) - 1; at >= 0; at -= 32) {
       const int64_t k = at - lane;
@@ -197,7 +203,7 @@ __global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSe
         for (uint32_t spins = 0; (w >> 62) == 0; ++spins) {
           if (spins >= a.spin_limit) {
             atomicOr(a.status, kErrTimeout);
-            w = kFlagPrefix;
+            w = kFlagPrefix | kLost;
             break;
           }
           __nanosleep(32);
@@ -206,15 +212,17 @@ __global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSe
       }
       const uint32_t done = __ballot_sync(0xFFFFFFFFu, (w >> 62) == 2);
       const int stop = done ? __ffs(done) - 1 : 31;  // the nearest CTA with everything before it
-      unsigned long long c = lane <= stop ? (w & kCountMask) : 0ull;
+      unsigned long long c = lane <= stop ? (w & (kLost - 1)) : 0ull;
+      lost |= __any_sync(0xFFFFFFFFu, lane <= stop && (w & kLost));
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, d);
       before += c;
       if (done) break;
     }
     if (lane == 0) {
-      if (cta) st_volatile(state + 1 + cta, kFlagPrefix | (before + total));
+      if (cta) st_volatile(state + 1 + cta, kFlagPrefix | (lost ? kLost : 0) | (before + total));
       s_before = before;
+      s_lost = lost;
     }
   }
   __syncthreads();
@@ -228,7 +236,7 @@ __global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSe
         if (n12 > nreal) R.l12[2 * nreal] = R.l12[2 * nreal + 1] = 0;
       }
     }
-    if (threadIdx.x == 0 && cta + 1 == ctas) R.meta[2] = level_before + total;  // ones of the level
+    if (threadIdx.x == 0 && cta + 1 == ctas) R.meta[2] = s_lost ? ~0ull : level_before + total;  // ones of the level
   };
   finish(L);
   if (twinned) finish(twin);
