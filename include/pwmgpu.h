@@ -446,7 +446,7 @@ PWMGPU_API pwmgpu_status pwmgpu_generate_batch(uint64_t seed, uint32_t count, ui
  * allocate device memory while they run -- plugins whose host framework owns
  * every device buffer and hands them in, serving loops that cannot afford an
  * allocator's implicit synchronisation.  It calls no cudaMalloc/cudaFree and
- * needs no context: its scratch is a fixed 4 MiB array in the library's
+ * needs no context: its scratch is a fixed 16 KiB array in the library's
  * device image, resident on every GPU that loads the library until the
  * process exits.
  *

@@ -779,12 +779,13 @@ void launch_rank_select(const RankSelectArgs& a, uint64_t max_words, cudaStream_
 // ===========================================================================
 namespace {
 
-// 4 MiB: a status word, then the look-back state.  The level limit is the
-// entry point's published one.
-constexpr uint64_t kNoAllocScratchWords = uint64_t(1) << 20;
+// The level limit is the entry point's published one.  The array: a status
+// word (and one to align), then the look-back state of the longest level, a
+// ticket and a word a CTA: 16 KB.
 constexpr uint64_t kNoAllocMaxL1Blocks = (uint64_t(1) << 20) - (uint64_t(1) << 12);
+constexpr uint64_t kNoAllocStateWords = 1 + (kNoAllocMaxL1Blocks + kRsThreads - 1) / kRsThreads;
 
-static __device__ __align__(256) uint32_t g_noalloc_rs_scratch[kNoAllocScratchWords];
+static __device__ __align__(256) uint32_t g_noalloc_rs_scratch[2 + 2 * kNoAllocStateWords];
 
 struct NoAllocSymbols {
   bool ready = false;
@@ -842,6 +843,7 @@ cudaError_t noalloc_rank_select_build(const uint64_t* words, uint64_t nwords, ui
   a.one = RankSelectLevel{words, nwords, l0, l12, s0, s1, counts};
   a.nfirst = 1;
   a.stride = rank_select_state_words(nwords);
+  if (a.stride > kNoAllocStateWords) return cudaErrorInvalidValue;
   a.status = scratch;
   a.state = reinterpret_cast<unsigned long long*>(scratch + 2);
   a.spin_limit = kSpinLimit;

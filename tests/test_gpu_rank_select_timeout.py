@@ -60,3 +60,35 @@ def test_wait_expires_and_context_recovers(pg, ctas):
     assert ones(ds, n) == int(text.sum())
     ds.free()
     ctx.close()
+
+
+def test_longest_level_without_allocation():
+    """pwmgpu_rank_select_build_noalloc at its limit, the whole of its state in
+    use: every block's count of ones before it, against counts by torch."""
+    torch = pytest.importorskip("torch")
+    import pwm_gb300 as pg
+    lib = pg.default_context().lib
+    nwords = 33423360
+    blocks = nwords // 32
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    words = torch.randint(0, 1 << 32, (2 * nwords,), device="cuda", generator=g).to(torch.int32)
+    pop = torch.tensor([bin(i).count("1") for i in range(256)], dtype=torch.uint8, device="cuda")
+    per = torch.empty(blocks, dtype=torch.int64, device="cuda")
+    step = blocks // 16
+    for i in range(0, blocks, step):
+        b = words[64 * i:64 * (i + step)].view(torch.uint8).view(step, 256)
+        per[i:i + step] = pop[b.to(torch.int32)].sum(1, dtype=torch.int64)
+    l0 = torch.full((nwords // 67108863 + 1,), -1, dtype=torch.int64, device="cuda")
+    l12 = torch.full((2 * (blocks + 1),), -1, dtype=torch.int32, device="cuda")
+    s0, s1 = (torch.zeros(nwords * 64 // 8192 + 2, dtype=torch.int32, device="cuda") for _ in range(2))
+    counts = torch.full((3,), -1, dtype=torch.int64, device="cuda")
+    p = [ctypes.c_void_p(t.data_ptr()) for t in (words, l0, l12, s0, s1, counts)]
+    torch.cuda.synchronize()
+    st = lib.pwmgpu_rank_select_build_noalloc(p[0], nwords, *p[1:], ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert st == 0
+    torch.cuda.synchronize()
+    assert int(counts[2]) == int(per.sum())
+    before = torch.cumsum(per, 0) - per
+    assert torch.equal(l12[:2 * blocks:2].to(torch.int64) & 0xFFFFFFFF, before)
+    assert l12[2 * blocks:].tolist() == [0, 0] and l0.tolist() == [0]
