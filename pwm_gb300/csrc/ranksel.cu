@@ -109,12 +109,27 @@ __device__ __forceinline__ bool thread_block_select(const uint64_t* data, uint64
 // threads; 512 threads 254).  Looking back over 64 to 256 CTAs a step changed
 // nothing: the wait is for the slowest loads.
 //
+// With few levels that wait has nothing to hide behind: all resident CTAs load,
+// then all wait.  Up to 3 levels of 2^22 words and more therefore take two
+// kernels: kRsCount leaves every block's ones before it in its CTA in its
+// entry and the CTAs' totals in the state words; kRsFinish adds the totals up
+// and finishes entries and samples from there.  One level alone, one kernel
+// and two: 2^22 words 21.3 and 20.9 us, 2^23 29.9 and 24.2, 2^24 56.6 and
+// 46.5, 33.4 million 98.7 and 80.9 (the three kernels 82.4).  Whole builds of
+// 2^28 symbols: 2 levels of the matrix 200.1 and 197.1 us, 3 of both
+// structures 219.5 and 215.9; 4 levels are even (2^30: 1487 and 1489), 7
+// better in one (1681 and 1699).
+//
 // Counting: warp w reads its 32 blocks (8 KB) with coalesced 16-byte loads: in
 // step i, lanes 0-15 read block 2i and lanes 16-31 block 2i+1, four lanes per
 // 512-bit L2 block; the counts are then gathered so that lane b holds block
 // b's.
 constexpr uint64_t kLost = 1ull << 61;  // of a state word: the counts before it are incomplete
-__global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSelectArgs a) {
+constexpr uint32_t kRsTwoKernelLevels = 3;                 // at most
+constexpr uint64_t kRsTwoKernelWords = uint64_t(1) << 22;  // of the longest, at least
+enum RsPart { kRsAll, kRsCount, kRsFinish };
+template <RsPart PART>
+__global__ void __launch_bounds__(kRsThreads, PART == kRsFinish ? 4 : 2) rank_select_kernel(const RankSelectArgs a) {
   chain_next();
   chain_wait();
   const uint32_t y = blockIdx.x;
@@ -132,14 +147,43 @@ __global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSe
   const uint32_t withheld = a.withhold && ctas > 1 ? 1 : 0;  // the level's first CTA does not run
   if (blockIdx.y + withheld >= ctas) return;
   unsigned long long* state = a.state + uint64_t(y) * a.stride;  // a ticket, then a word a CTA
-  __shared__ uint32_t s_cta;
-  if (threadIdx.x == 0) s_cta = uint32_t(atomicAdd(state, 1ull)) + withheld;
-  __syncthreads();
-  const uint32_t cta = s_cta;
-  const uint64_t first = uint64_t(cta) * kRsThreads;
+  uint32_t cta = blockIdx.y;
+  if constexpr (PART == kRsAll) {
+    __shared__ uint32_t s_cta;
+    if (threadIdx.x == 0) s_cta = uint32_t(atomicAdd(state, 1ull)) + withheld;
+    __syncthreads();
+    cta = s_cta;
+  }
+  const uint64_t first = uint64_t(cta) * kRsThreads, b = first + threadIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t l2[4] = {0, 0, 0, 0};
-  {
+  __shared__ uint32_t wsum[kRsThreads / 32];
+  __shared__ unsigned long long s_before;
+  __shared__ bool s_lost;
+  uint32_t v, fields, total, before_block;  // the block's ones and L2 fields; the CTA's ones, and those before the block
+  if constexpr (PART == kRsFinish) {
+    // as kRsCount left them: the ones before the block in its CTA, and the CTAs' totals
+    __shared__ uint32_t in_cta[kRsThreads + 1];
+    __shared__ unsigned long long wbefore[kRsThreads / 32];
+    total = uint32_t(state[1 + cta]);
+    before_block = b < nreal ? L.l12[2 * b] : total;
+    fields = b < nreal ? L.l12[2 * b + 1] : 0u;
+    in_cta[threadIdx.x] = before_block;
+    if (threadIdx.x == 0) in_cta[kRsThreads] = total;
+    unsigned long long before = 0;
+    for (uint32_t k = threadIdx.x; k < cta; k += kRsThreads) before += state[1 + k];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) before += __shfl_xor_sync(0xFFFFFFFFu, before, d);
+    if (lane == 0) wbefore[warp] = before;
+    __syncthreads();
+    v = in_cta[threadIdx.x + 1] - before_block;
+    if (threadIdx.x == 0) {
+      unsigned long long all = 0;
+      for (int w = 0; w < kRsThreads / 32; ++w) all += wbefore[w];
+      s_before = all;
+      s_lost = false;
+    }
+  } else {
+    uint32_t l2[4] = {0, 0, 0, 0};
     const uint64_t wb = first + 32 * uint64_t(warp);  // first block of this warp
     const uint64_t ww = wb * kL1Cover;                 // first word of this warp
     // 16-byte loads when the warp's words are all in the level and aligned
@@ -170,28 +214,36 @@ __global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSe
         gather(i, (w < L.nwords ? __popcll(L.data[w]) : 0) + (w + 1 < L.nwords ? __popcll(L.data[w + 1]) : 0));
       }
     }
-  }
-  // exclusive scan of the block totals (past the level: 0)
-  const uint32_t v = l2[0] + l2[1] + l2[2] + l2[3];
-  uint32_t x = v;
+    // exclusive scan of the block totals (past the level: 0)
+    v = l2[0] + l2[1] + l2[2] + l2[3];
+    uint32_t x = v;
 #pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t s = __shfl_up_sync(0xFFFFFFFFu, x, d);
-    if (lane >= d) x += s;
-  }
-  __shared__ uint32_t wsum[kRsThreads / 32];
-  __shared__ unsigned long long s_before;
-  __shared__ bool s_lost;
-  if (lane == 31) wsum[warp] = x;
-  __syncthreads();
-  uint32_t before_warp = 0, total = 0;
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t s = __shfl_up_sync(0xFFFFFFFFu, x, d);
+      if (lane >= d) x += s;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    uint32_t before_warp = 0;
+    total = 0;
 #pragma unroll
-  for (int w = 0; w < kRsThreads / 32; ++w) {
-    before_warp += w < warp ? wsum[w] : 0u;
-    total += wsum[w];
+    for (int w = 0; w < kRsThreads / 32; ++w) {
+      before_warp += w < warp ? wsum[w] : 0u;
+      total += wsum[w];
+    }
+    before_block = before_warp + x - v;
+    fields = (l2[0] & 1023u) | ((l2[1] & 1023u) << 10) | ((l2[2] & 1023u) << 20);
+    if constexpr (PART == kRsCount) {
+      if (threadIdx.x == 0) state[1 + cta] = total;
+      if (b < nreal) {
+        L.l12[2 * b] = before_block;
+        L.l12[2 * b + 1] = fields;
+      }
+      return;
+    }
   }
   // publish, then look back 32 CTAs a step
-  if (warp == 0) {
+  if (PART == kRsAll && warp == 0) {
     unsigned long long before = 0;
     bool lost = false;
     if (lane == 0) st_volatile(state + 1 + cta, (cta == 0 ? kFlagPrefix : kFlagAggregate) | total);
@@ -240,10 +292,8 @@ __global__ void __launch_bounds__(kRsThreads, 2) rank_select_kernel(const RankSe
   };
   finish(L);
   if (twinned) finish(twin);
-  const uint64_t b = first + threadIdx.x;
   if (b >= nreal) return;
-  const uint64_t ones_before = level_before + before_warp + x - v, ones_through = ones_before + v;
-  const uint32_t fields = (l2[0] & 1023u) | ((l2[1] & 1023u) << 10) | ((l2[2] & 1023u) << 20);
+  const uint64_t ones_before = level_before + before_block, ones_through = ones_before + v;
   auto entry = [&](const RankSelectLevel& R) {
     R.l12[2 * b] = uint32_t(ones_before);
     R.l12[2 * b + 1] = fields;
@@ -760,7 +810,13 @@ void launch_rank_select(const RankSelectArgs& a, uint64_t max_words, cudaStream_
   const uint32_t levels = a.nfirst + a.nsecond;
   if (levels == 0) return;
   const dim3 grid(levels, unsigned(rank_select_state_words(max_words) - 1));  // at most 8192 CTAs a level (2^32 bits)
-  launch_chained(rank_select_kernel, grid, kRsThreads, 0, s, a);
+  if (levels <= kRsTwoKernelLevels && max_words >= kRsTwoKernelWords && !a.withhold) {
+    launch_chained(rank_select_kernel<kRsCount>, grid, kRsThreads, 0, s, a);
+    launch_chained(rank_select_kernel<kRsFinish>, grid, kRsThreads, 0, s, a);
+    *launches += 2;
+    return;
+  }
+  launch_chained(rank_select_kernel<kRsAll>, grid, kRsThreads, 0, s, a);
   ++*launches;
 }
 
