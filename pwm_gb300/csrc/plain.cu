@@ -214,9 +214,10 @@ namespace {
 // histogram, the tables, the pass, rank/select) and then waits for the zeros
 // and the status word.
 //
-// Measured (GB300), both structures with rank/select and 3 x 10^4 queries:
-// 10^6 bytes, 8 levels 189 -> 94 us a build, 4099 bytes 160 -> 81; 2^26
-// DNA-like bytes, 2 levels, without queries 102 -> 86.
+// Measured (GB300), both structures with rank/select and queries, against a
+// plan made on the host: 10^6 bytes, 8 levels 189 -> 94 us a build, 4099 bytes
+// 160 -> 81; 2^26 DNA-like bytes, 2 levels, without queries 102 -> 86.  (88, 77
+// and 60 with plane histograms, double tiles and chained launches since.)
 //
 // Short texts take half-size tiles and histogram blocks of one tile, so that
 // more SMs work: both structures of 2^20 bytes take 36 us at 8 levels against
@@ -230,11 +231,12 @@ constexpr uint64_t kDoubleTileMin = uint64_t(1) << 24;  // symbols, up to 4 leve
 // 8 levels of bytes in one pass: its tiles cost more than two 4-level passes
 // (127 runs at the deepest level), but a text saves the second pass, the
 // host's plan of it and the regroup.  One pass against two: both structures
-// 48 and 88 us at 2^22 bytes, 116 and 130 at 2^24, 166 either way at 24 2^20,
-// 195 and 189 at 30 2^20, 356 and 302 at 60 2^20; the matrix alone 144 and 156
-// at 24 2^20, 215 and 213 at 40 2^20, 302 and 278 at 60 2^20.
+// 46 and 90 us at 2^22 bytes, 114 and 132 at 2^24, 164 and 167 at 24 2^20, 193
+// and 190 at 30 2^20, 354 and 296 at 60 2^20; the matrix alone 142 and 157 at
+// 24 2^20, 166 and 181 at 30 2^20, and, once the first of two passes takes
+// double tiles (2^25), 199 and 189 at 36 2^20, 212 and 204 at 40 2^20.
 constexpr uint64_t kOnePass8Tree = uint64_t(24) << 20;    // symbols, with a tree
-constexpr uint64_t kOnePass8Matrix = uint64_t(40) << 20;  // a matrix alone
+constexpr uint64_t kOnePass8Matrix = uint64_t(32) << 20;  // a matrix alone
 
 void build_one_pass(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text) {
   cudaStream_t s = ctx->stream;
@@ -389,10 +391,10 @@ void build_plain(pwmgpu_ctx* ctx, pwmgpu_wx* wx, const void* d_text, const HostI
   // Pass width: by default a text of up to kSinglePassMaxLevels levels takes
   // one pass of all its levels (the histogram kernel gives that pass its
   // prefixes), deeper texts passes of kDefaultTileLevels; set_pass_levels(k)
-  // asks for k (<= 4).  At 8 levels one pass would write 127 runs per tile
-  // into each of the deepest levels of both structures, and the two 4-level
-  // passes are faster (measured: 5.9 against 6.2 ms for 2^30 bytes, while
-  // one pass wins at 5..7 levels).
+  // asks for k (<= 4).  One pass of 8 levels writes 127 runs per tile into
+  // each of the deepest levels of both structures: bytes past the lengths
+  // that build_one_pass takes (kOnePass8Tree, kOnePass8Matrix), and wider
+  // symbols, take two of 4.
   const bool auto_k = ctx->tile_levels == 0;
   const int kmax = (auto_k && L > uint32_t(kTileMaxLevels) && L <= kSinglePassMaxLevels)
                        ? int(L)
