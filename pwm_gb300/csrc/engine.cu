@@ -118,7 +118,7 @@ void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint
 }
 
 // Rank/select blocks of every level of the given structures (asynchronous),
-// all levels in one launch.  share_level0: a plain matrix and tree, whose
+// all levels in one launch (a few long ones in two).  share_level0: a plain matrix and tree, whose
 // level 0 is the same bit vector: counted once, written to both.
 //
 // Levels [lo, hi) only, on `stream` (default: the context's) with a scratch

@@ -405,10 +405,11 @@ inline uint64_t rs_ns(uint64_t nwords) { return nwords * 64 / 8192 + 2; }
 void alloc_structure(Structure& s, const std::vector<uint64_t>& level_bits, uint64_t n, bool tree, bool huff,
                      bool rank_select, cudaStream_t stream, cudaStream_t alloc_stream = nullptr);
 // Rank/select blocks of every level of the given structures (asynchronous),
-// all levels in one launch sequence.  share_level0: a plain matrix and tree,
-// whose level 0 is the same bit vector: the tree's blocks of level 0 are a
-// copy of the matrix's.  Levels [lo, hi) only, on `stream` (default: the
-// context's) with scratch buffers named after `tag`.
+// all levels in one launch (a few long ones in two).  share_level0: a plain
+// matrix and tree, whose level 0 is the same bit vector: counted once, written
+// to both.  Levels [lo, hi) only, on `stream` (default: the context's), with
+// the look-back state in a scratch buffer named after `tag`, or in zeroed_state
+// (zeroed on that stream; rank_select_state_words for every level).
 void build_rank_select(pwmgpu_ctx* ctx, Structure* wm, Structure* wt = nullptr, bool share_level0 = false,
                        uint32_t lo = 0, uint32_t hi = ~0u, cudaStream_t stream = nullptr, const char* tag = "",
                        unsigned long long* zeroed_state = nullptr);

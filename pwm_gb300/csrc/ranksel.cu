@@ -347,11 +347,11 @@ __global__ void __launch_bounds__(kRsThreads, PART == kRsFinish ? 4 : 2) rank_se
 // exchanges costing more than the counting they save.  The level descriptors
 // come from shared memory.  Measured (GB300): 3 x 10^4 queries on a tree of
 // 10^6 bytes, 8 levels, 139 -> 52 us; 3 x 2^22 on the 2^28 16-bit matrix (16
-// levels) 8.34 -> 4.23 ms (access 1.18, rank 1.32, select 1.73), bound by L1's
+// levels) 8.34 -> 4.22 ms (access 1.17, rank 1.32, select 1.72), bound by L1's
 // scattered requests (80 % busy; DRAM 45 % of its peak).  128 threads a block
 // spread a small batch over more SMs than 256 (50.7 against 54.5 us); 48
 // registers a thread (10 blocks an SM) answered the large batch faster than 40
-// (4.23 against 4.48 ms).
+// (4.48 ms).
 // ---------------------------------------------------------------------------
 constexpr int kQueryThreads = 128;
 constexpr uint32_t kQueryMaxLevels = 64;
@@ -373,7 +373,7 @@ struct FastLevel {
 // Four words, or four block entries (ones before the block in the low half,
 // its L2 fields in the high one), by one 32-byte load.  The words go round L1
 // and pull in no more than their 64 bytes of L2 (by default a miss fetched up
-// to 128: 2^22 accesses 1.13 -> 1.00 ms, ranks 2.10 -> 1.25 ms).
+// to 128: 2^22 accesses took 13 % longer, ranks 68 %).
 struct Four {
   uint64_t w[4];
 };
